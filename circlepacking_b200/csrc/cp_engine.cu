@@ -212,7 +212,6 @@ struct RefArgs {
     int slab_begin;
     size_t count;  // boxes in this wave
     unsigned long long* cnt;
-    int collect;  // 1: record every failing box (no early exit)
     double* coll;
     uint8_t* coll_handles;
     size_t coll_cap;
@@ -221,7 +220,8 @@ struct RefArgs {
 // The body of the family kernels' loops (e.g. middle_configuration.cu:157-201)
 // over the lattice boxes of lambda slabs [slab_begin, ...), stopping at slabs
 // beyond the first slab that holds a failing box.
-template <int FAM>
+// COLLECT: record every failing box (complete masks, no early exit).
+template <int FAM, bool COLLECT>
 __global__ void __launch_bounds__(kEvalBlock) k_ref_step(RefArgs a) {
     constexpr int D = family_dims(FAM);
     size_t per_slab = 1;
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kEvalBlock) k_ref_step(RefArgs a) {
     volatile unsigned long long* best = a.cnt + C_BEST_SLAB;
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < a.count; t += step) {
         const int slab = a.slab_begin + (int)(t / per_slab);
-        if (!a.collect && (unsigned long long)slab > *best) continue;
+        if (!COLLECT && (unsigned long long)slab > *best) continue;
         size_t rem = t % per_slab;
         int ix[4] = {slab, 0, 0, 0};
         for (int d = D - 1; d >= 1; --d) {
@@ -241,7 +241,8 @@ __global__ void __launch_bounds__(kEvalBlock) k_ref_step(RefArgs a) {
         double lo[4], hi[4];
         if (!lattice_box(a.s, ix, a.slab_single[slab], lo, hi)) continue;
         ++evaluated;
-        Verdict v = a.collect ? eval_box<FAM, FULL>(lo, hi, 0, nullptr) : eval_box<FAM, DECIDE>(lo, hi, 0, nullptr);
+        const Verdict v = COLLECT ? judge_box<FAM, FULL, flt::NEED_FULL>(lo, hi, 0)
+                                  : judge_box<FAM, DECIDE, flt::NEED_VERDICT>(lo, hi, 0);
         if (v.verdict == V_EMPTY) continue;
         const bool nofit = (v.mask & M_FIT) && FAM != F_START && FAM != F_START_END_2D && FAM != F_START_END_3D;
         const bool trap = (v.mask & M_TRAP) != 0;
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(kEvalBlock) k_ref_step(RefArgs a) {
         if (v.mask & M_CRIT) {
             atomicMin(&a.cnt[C_BEST_SLAB], (unsigned long long)slab);
             atomicMin(&a.cnt[C_FIRST_BITS], ordered_bits(lo[0]));
-            if (a.collect) {
+            if (COLLECT) {
                 const unsigned long long k = atomicAdd(&a.cnt[C_COLLECT], 1ull);
                 if (k < a.coll_cap) {
                     // the box as the reference prints it: r2, r1 tightened
@@ -300,9 +301,8 @@ double now_ms() {
 
 // ------------------------------------------------------------------ handle
 struct LevelBuf {
-    BoxList b{nullptr, nullptr, nullptr, 0, nullptr};
+    BoxList b{nullptr, nullptr, nullptr, 0};
     size_t n = 0;
-    double* aux = nullptr;  // kAuxFields x cap, allocated on first use (b.aux points here when in use)
 };
 
 struct cp_prover {
@@ -387,7 +387,6 @@ void free_levels(cp_prover* p) {
         cudaFree(L.b.lo);
         cudaFree(L.b.hi);
         cudaFree(L.b.depth);
-        cudaFree(L.aux);
     }
     p->levels.clear();
 }
@@ -448,9 +447,10 @@ LevelKernel level_kernel(int fam, int prec, int v) {
 }
 
 using RefKernel = void (*)(RefArgs);
+template <bool COLLECT>
 RefKernel ref_kernel(int fam) {
-    static const RefKernel k[6] = {k_ref_step<0>, k_ref_step<1>, k_ref_step<2>,
-                                   k_ref_step<3>, k_ref_step<4>, k_ref_step<5>};
+    static const RefKernel k[6] = {k_ref_step<0, COLLECT>, k_ref_step<1, COLLECT>, k_ref_step<2, COLLECT>,
+                                   k_ref_step<3, COLLECT>, k_ref_step<4, COLLECT>, k_ref_step<5, COLLECT>};
     return k[fam];
 }
 
@@ -802,26 +802,7 @@ cp_status refine_graph(cp_prover* p, const cp_refine_opts& o, cp_refine_report* 
     return CP_OK;
 }
 
-// The lambda-independent terms of the start family travel with the boxes of
-// levels >= 1 (children) when the refinement asks for it (opts.reuse) and its
-// split can leave radii unchanged; every other refinement, and the seed level,
-// sees no aux.  A level whose aux cannot be allocated goes without: its boxes
-// recompute the terms.
-void attach_aux(cp_prover* p, const cp_refine_opts& o) {
-    // a uniform split changes every radius of every child: nothing to carry
-    const bool use = o.reuse != 0 && o.family == F_START && o.policy != CP_SPLIT_UNIFORM;
-    for (size_t l = 0; l < p->levels.size(); ++l) {
-        LevelBuf& L = p->levels[l];
-        if (use && l > 0 && !L.aux && cudaMalloc(&L.aux, sizeof(double) * kAuxFields * L.b.cap) != cudaSuccess) {
-            L.aux = nullptr;
-            cudaGetLastError();  // clear the allocation error
-        }
-        L.b.aux = (use && l > 0) ? L.aux : nullptr;
-    }
-}
-
 cp_status run_refinement(cp_prover* p, const cp_refine_opts& o, cp_refine_report* r, double t0) {
-    attach_aux(p, o);
     if (o.engine == CP_ENGINE_GRAPH && !cp_model_collecting(p)) return refine_graph(p, o, r, t0);
     return refine_levels(p, o, r, t0);
 }
@@ -1415,9 +1396,6 @@ cp_status cp_checkpoint_load(cp_prover* p, const char* path, cp_refine_opts* opt
         for (uint32_t d = 0; d < h.dims; ++d) CP_TRY(load(fc.f, b.lo + d * b.cap, n[l], stage, p->stream));
         for (uint32_t d = 0; d < h.dims; ++d) CP_TRY(load(fc.f, b.hi + d * b.cap, n[l], stage, p->stream));
         CP_TRY(load(fc.f, b.depth, n[l], stage, p->stream));
-        // a checkpoint carries no lambda-independent terms: the loaded boxes recompute them
-        if (p->levels[l].aux)
-            CP_TRY(cuda_ok(cudaMemsetAsync(p->levels[l].aux + 3 * b.cap, 0, sizeof(double) * n[l], p->stream)));
         p->levels[l].n = (size_t)n[l];
     }
     p->pending = true;
@@ -1452,11 +1430,11 @@ cp_status cp_reference_step(cp_prover* p, int family, double la_lb, double la_ub
     for (int d = 1; d < D; ++d) per_slab *= (size_t)s.n[d];
     const size_t wave_boxes = (size_t)1 << 23;
     const int wave_slabs = (int)std::max<size_t>(1, wave_boxes / per_slab);
-    RefKernel k = ref_kernel(family);
+    RefKernel k = ref_kernel<false>(family);
     const unsigned grid = grid_of(k, kEvalBlock);
     for (int s0 = 0; s0 < s.n[0]; s0 += wave_slabs) {
         const int ns = std::min(wave_slabs, s.n[0] - s0);
-        RefArgs a{s, p->slab_single, s0, (size_t)ns * per_slab, p->cnt, 0, nullptr, nullptr, 0};
+        RefArgs a{s, p->slab_single, s0, (size_t)ns * per_slab, p->cnt, nullptr, nullptr, 0};
         k<<<grid, kEvalBlock, 0, p->stream>>>(a);
         CP_TRY(cp_check_launch());
         CP_TRY(read_counters(p));
@@ -1596,8 +1574,8 @@ cp_status cp_reference_criticals(cp_prover* p, int family, double la_lb, double 
     }
     size_t per_slab = 1;
     for (int d = 1; d < D; ++d) per_slab *= (size_t)s.n[d];
-    RefKernel k = ref_kernel(family);
-    RefArgs a{s, p->slab_single, 0, (size_t)s.n[0] * per_slab, p->cnt, 1, dboxes, dh, max_boxes};
+    RefKernel k = ref_kernel<true>(family);
+    RefArgs a{s, p->slab_single, 0, (size_t)s.n[0] * per_slab, p->cnt, dboxes, dh, max_boxes};
     k<<<grid_of(k, kEvalBlock), kEvalBlock, 0, p->stream>>>(a);
     cp_status st = cp_check_launch();
     if (st == CP_OK) st = read_counters(p);

@@ -16,7 +16,11 @@ using namespace cpb;
 namespace {
 
 // ------------------------------------------------------------------ kernels
-template <int FAM, int MODE>
+// What of the mask an evaluation mode reports.
+__host__ __device__ constexpr int need_of(int mode) { return mode == FULL ? flt::NEED_FULL : flt::NEED_MASK; }
+
+// TRACE: the compared values themselves are wanted, so nothing is filtered.
+template <int FAM, int MODE, bool TRACE>
 __global__ void __launch_bounds__(kEvalBlock) k_eval_fp64(const double* __restrict__ lo, const double* __restrict__ hi,
                                                           size_t n, size_t stride, uint8_t* __restrict__ verdict,
                                                           uint8_t* __restrict__ mask, const uint8_t* __restrict__ order,
@@ -31,7 +35,8 @@ __global__ void __launch_bounds__(kEvalBlock) k_eval_fp64(const double* __restri
             h[d] = __ldg(hi + d * stride + i);
         }
         const int ord = order ? order[i] : 0;
-        Verdict v = eval_box<FAM, MODE>(l, h, ord, trace ? trace + 16 * i : nullptr);
+        const Verdict v = TRACE ? eval_box<FAM, MODE>(l, h, ord, trace + 16 * i)
+                                : judge_box<FAM, MODE, need_of(MODE)>(l, h, ord);
         verdict[i] = v.verdict;
         mask[i] = v.mask;
     }
@@ -39,7 +44,7 @@ __global__ void __launch_bounds__(kEvalBlock) k_eval_fp64(const double* __restri
 
 // FP32 enclosure pass; boxes it cannot prove are re-evaluated in FP64 by the
 // same thread (decide mode: the FP64 result; full mode: the full FP64 mask).
-template <int FAM, int MODE>
+template <int FAM, int MODE, bool TRACE>
 __global__ void __launch_bounds__(kEvalBlock) k_eval_prefilter(const double* __restrict__ lo,
                                                                const double* __restrict__ hi, size_t n, size_t stride,
                                                                uint8_t* __restrict__ verdict, uint8_t* __restrict__ mask,
@@ -59,7 +64,7 @@ __global__ void __launch_bounds__(kEvalBlock) k_eval_prefilter(const double* __r
         const int pre = prefilter_box<FAM>(l, h, ord, MODE == FULL, &pmask);
         Verdict v;
         if (pre == PF_UNDECIDED)
-            v = eval_box<FAM, MODE>(l, h, ord, trace ? trace + 16 * i : nullptr);
+            v = TRACE ? eval_box<FAM, MODE>(l, h, ord, trace + 16 * i) : judge_box<FAM, MODE, need_of(MODE)>(l, h, ord);
         else
             v = {pre == PF_PROVED ? V_PROVED : pre == PF_EMPTY ? V_EMPTY : pre == PF_NOFIT ? V_NOFIT : V_CRITICAL,
                  pmask};
@@ -90,6 +95,26 @@ __global__ void k_div_check(const double* __restrict__ a, const double* __restri
         out[4 * i + 2] = __ddiv_rd(a[i], b[i]);
         out[4 * i + 3] = __ddiv_ru(a[i], b[i]);
     }
+}
+
+// Largest errors of the filter's reciprocal and reciprocal-square-root seeds.  The
+// approximations read only the upper word of their operand, so every upper word of
+// the filter's range is tried with the smallest and the largest lower word.
+constexpr int kSeedExpLo = -120, kSeedExpHi = 4;
+__global__ void k_seed_error(unsigned long long* out) {
+    const size_t total = (size_t)(kSeedExpHi - kSeedExpLo) << 20, step = (size_t)gridDim.x * blockDim.x;
+    double er = 0.0, es = 0.0;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += step) {
+        const int hi = (int)(((size_t)(1023 + kSeedExpLo) << 20) + i);
+        for (int low = 0; low < 2; ++low) {
+            const double d = __hiloint2double(hi, low ? -1 : 0);
+            const double y = flt::rcp_seed_(d), z = flt::rsqrt_seed_(d);
+            er = fmax(er, fabs(__fma_rn(-d, y, 1.0)));
+            es = fmax(es, 0.5 * fabs(__fma_rn(-d * z, z, 1.0)));
+        }
+    }
+    atomicMax(out, (unsigned long long)__double_as_longlong(er));
+    atomicMax(out + 1, (unsigned long long)__double_as_longlong(es));
 }
 
 __global__ void k_single_placement(const double* __restrict__ lam, size_t n, double* __restrict__ out) {
@@ -172,14 +197,14 @@ unsigned grid_for(K kernel, size_t n, int block) {
     return (unsigned)(g ? g : 1);
 }
 
-template <int FAM, int MODE>
+template <int FAM, int MODE, bool TRACE>
 cp_status launch_eval(int precision, const double* lo, const double* hi, size_t n, size_t stride, uint8_t* verdict,
                       uint8_t* mask, const uint8_t* order, double* trace, cudaStream_t st) {
     if (precision == CP_FP64) {
-        auto k = k_eval_fp64<FAM, MODE>;
+        auto k = k_eval_fp64<FAM, MODE, TRACE>;
         k<<<grid_for(k, n, kEvalBlock), kEvalBlock, 0, st>>>(lo, hi, n, stride, verdict, mask, order, trace);
     } else {
-        auto k = k_eval_prefilter<FAM, MODE>;
+        auto k = k_eval_prefilter<FAM, MODE, TRACE>;
         k<<<grid_for(k, n, kEvalBlock), kEvalBlock, 0, st>>>(lo, hi, n, stride, verdict, mask, order, trace);
     }
     return cp_check_launch();
@@ -188,8 +213,10 @@ cp_status launch_eval(int precision, const double* lo, const double* hi, size_t 
 template <int FAM>
 cp_status launch_eval_mode(int precision, int mode, const double* lo, const double* hi, size_t n, size_t stride,
                            uint8_t* verdict, uint8_t* mask, const uint8_t* order, double* trace, cudaStream_t st) {
-    if (mode == CP_EVAL_FULL) return launch_eval<FAM, FULL>(precision, lo, hi, n, stride, verdict, mask, order, trace, st);
-    return launch_eval<FAM, DECIDE>(precision, lo, hi, n, stride, verdict, mask, order, nullptr, st);
+    if (mode != CP_EVAL_FULL)
+        return launch_eval<FAM, DECIDE, false>(precision, lo, hi, n, stride, verdict, mask, order, nullptr, st);
+    return trace ? launch_eval<FAM, FULL, true>(precision, lo, hi, n, stride, verdict, mask, order, trace, st)
+                 : launch_eval<FAM, FULL, false>(precision, lo, hi, n, stride, verdict, mask, order, nullptr, st);
 }
 
 std::mutex g_host_mu;
@@ -330,6 +357,14 @@ cp_status cp_div_check(const double* a, const double* b, size_t n, double* out, 
     if (n == 0) return CP_OK;
     if (!a || !b || !out) return CP_ERR_INVALID;
     k_div_check<<<grid_for(k_div_check, n, 128), 128, 0, (cudaStream_t)stream>>>(a, b, n, out);
+    return cp_check_launch();
+}
+
+cp_status cp_seed_error(double* out, void* stream) {
+    if (!out) return CP_ERR_INVALID;
+    cudaError_t e = cudaMemsetAsync(out, 0, 2 * sizeof(double), (cudaStream_t)stream);
+    if (e != cudaSuccess) return cp_record_cuda_error(e, CP_ERR_CUDA);
+    k_seed_error<<<1184, 128, 0, (cudaStream_t)stream>>>(reinterpret_cast<unsigned long long*>(out));
     return cp_check_launch();
 }
 

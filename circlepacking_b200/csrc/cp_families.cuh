@@ -19,6 +19,7 @@
 //           PROVED / EMPTY are exactly as in FULL, a not-proved box reports the
 //           first event met (fit check, trap site or failing handle).
 #pragma once
+#include "cp_filter.cuh"
 #include "cp_fp64.cuh"
 
 namespace cpb {
@@ -26,17 +27,6 @@ namespace cpb {
 struct Verdict {
     uint8_t verdict, mask;
     uint8_t handles;  // guarded criteria (handles) evaluated for this box
-};
-
-// The terms of the start family's criteria that do not depend on lambda
-// (start_configuration.cu:126-162): the collision angle of disks 1 and 3 on the
-// outer border, ca_outer_outer(r1, r3), and the upper semicircle angle of r1.
-// They are functions of the radii alone (r1 tightened by r2 and r3), so a box
-// whose radii equal its parent's bit for bit has its parent's values.
-// flag: 0 = not available, 1 = available, 2 = available and their evaluation
-// reached a trap site.
-struct LaFree {
-    double a13lo, a13hi, so_hi, flag;
 };
 
 enum EvalMode { FULL = 0, DECIDE = 1 };
@@ -233,11 +223,8 @@ __device__ __noinline__ HandleOut end3d_handle_call(Iv la, Iv r1, Iv r2, Iv r3) 
 // order: for the families with two independent handles (middle, end_2d,
 // end_3d) bit 0 set = evaluate the second handle first (DECIDE mode only).
 // tr: FULL mode only, 16 doubles (lhs, rhs per sub-criterion) or nullptr.
-// la_in / la_out (start family, optional): the lambda-independent terms of this
-// box when already known (la_in->flag != 0), and where to report them.
 template <int FAM, int MODE>
-__device__ __forceinline__ Verdict eval_box(const double* lo, const double* hi, int order, double* tr,
-                                            const LaFree* la_in = nullptr, LaFree* la_out = nullptr) {
+__device__ __forceinline__ Verdict eval_box(const double* lo, const double* hi, int order, double* tr) {
     constexpr int D = family_dims(FAM);
     Iv la{lo[0], hi[0]}, r1{lo[1], hi[1]}, r2{lo[2], hi[2]}, r3{0.0, 0.0};
     if (D == 4) {
@@ -261,20 +248,8 @@ __device__ __forceinline__ Verdict eval_box(const double* lo, const double* hi, 
 
     if (FAM == F_START) {
         const Iv a12 = ca_outer_inner(la, r1, r2, trap);
-        Iv a13;
-        double so_hi;
-        if (la_in && la_in->flag != 0.0) {
-            a13 = {la_in->a13lo, la_in->a13hi};
-            so_hi = la_in->so_hi;
-            if (la_in->flag == 2.0) trap = true;
-            if (la_out) *la_out = *la_in;
-        } else {
-            bool t13 = false;
-            a13 = ca_outer_outer(r1, r3, t13);
-            so_hi = semi_outer_hi(r1);
-            if (t13) trap = true;
-            if (la_out) *la_out = {a13.lo, a13.hi, so_hi, t13 ? 2.0 : 1.0};
-        }
+        const Iv a13 = ca_outer_outer(r1, r3, trap);
+        const double so_hi = semi_outer_hi(r1);
         const Iv a23 = ca_inner_outer(la, r2, r3, trap);
         const Iv s = iadd(a12, a23);
         const Ub case1{a13.hi < s.lo, a13.lo < s.hi};  // a12 + a23 > a13
@@ -406,6 +381,47 @@ done:
     else
         v = V_PROVED;
     return {v, mask, handles};
+}
+
+// eval_box for the boxes the filter leaves: one out-of-line copy per family and
+// mode, away from the registers and the instruction footprint of the common path.
+// Verdict in bits 0..7, mask in 8..15, handles in 16..23.
+template <int FAM, int MODE>
+__device__ __noinline__ uint32_t eval_box_call(double l0, double h0, double l1, double h1, double l2, double h2,
+                                               double l3, double h3, int order) {
+    const double lo[4] = {l0, l1, l2, l3}, hi[4] = {h0, h1, h2, h3};
+    const Verdict v = eval_box<FAM, MODE>(lo, hi, order, nullptr);
+    return (uint32_t)v.verdict | ((uint32_t)v.mask << 8) | ((uint32_t)v.handles << 16);
+}
+
+// eval_box without a trace, through the FP64 filter: the same verdict, with the
+// part of mask and handles that NEED asks for (flt::Need).
+template <int FAM, int MODE, int NEED>
+__device__ __forceinline__ Verdict judge_box(const double* lo, const double* hi, int order) {
+    constexpr int D = family_dims(FAM);
+    constexpr bool kFitStops = FAM != F_START && FAM != F_START_END_2D && FAM != F_START_END_3D;
+    flt::FBox b{lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], 0.0, 0.0};
+    bool empty = b.ll > b.lh || b.l2 > b.h2;
+    if (D == 4) {
+        b.l3 = lo[3];
+        b.h3 = hi[3];
+        if (b.l2 < b.l3) b.l2 = b.l3;
+        empty = empty || b.l3 > b.h3 || b.l2 > b.h2;
+    }
+    if (b.l1 < b.l2) b.l1 = b.l2;
+    if (empty || b.l1 > b.h1) return {V_EMPTY, 0, 0};
+    const bool fit_fires = FAM != F_START_END_2D && FAM != F_START_END_3D &&
+                           __dmul_ru(2.0, b.h1) >= __dadd_rd(1.0, -b.lh);
+    const uint8_t fit = fit_fires ? (uint8_t)M_FIT : (uint8_t)0;
+    if (MODE == DECIDE && kFitStops && fit_fires) return {V_NOFIT, fit, 0};
+    flt::FOut o;
+    if (flt::filter_box<FAM, NEED>(b, order, o)) {
+        const uint8_t v = kFitStops && fit_fires ? V_NOFIT : o.mask ? V_CRITICAL : V_PROVED;
+        return {v, (uint8_t)(fit | o.mask), o.handles};
+    }
+    const uint32_t r = eval_box_call<FAM, MODE>(lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], D == 4 ? lo[3] : 0.0,
+                                                D == 4 ? hi[3] : 0.0, order);
+    return {(uint8_t)r, (uint8_t)(r >> 8), (uint8_t)(r >> 16)};
 }
 
 }  // namespace cpb

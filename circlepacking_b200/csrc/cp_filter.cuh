@@ -1,0 +1,564 @@
+// FP64 filter of the lane-packing criteria: the verdict of a box from one
+// round-to-nearest evaluation and an error bound, instead of two directed
+// roundings of every step.
+//
+// filter_box evaluates the quantities that the criteria of a family compare
+// (the same interval ends, combined by the same formulas, cp_families.cuh) in
+// round-to-nearest FP64 and decides each comparison only when its two sides are
+// further apart than the error bound.  Where every comparison on the way to the
+// verdict is decided, the verdict is the one of eval_box; any other box is left
+// to eval_box, bit for bit as before.
+//
+// Error bound.  "Directed" is eval_box's value, "filter" the value here, both
+// against the same formula in exact arithmetic.  The box guard (box_ok) bounds
+// the inputs: lambda in [0.49, 0.996], radii at most 1/3, 0.25 <= L, S < 1.4.
+//   * Directed: L^2 - S^2 and (a + b)^2 are off by at most 2^-49.4 (a few ulps of
+//     values below 2), the quotient q = (L^2 - S^2 +- c^2) / (2 c L) of a
+//     collision angle by 2^-49.4 / c <= 2^-41.4 (c = a + b >= 2^-8), and asin(q) by
+//     2^-41.4 / sqrt(2 (1 - |q|)) <= 2^-33.9 where 1 - |q| >= kEnd = 2^-16.  Its
+//     padding of asin (5 ulps) is far below that.
+//   * Filter: the numerators carry the same roundings; the reciprocal is off by
+//     at most 2^-38 of its value (a 2^-19 seed, checked over all its seeds in
+//     tests/test_filter_gpu.py, and one Newton step); 1 - |q| is formed from the
+//     numerators, not from q, so that its relative error stays small near 1; the
+//     arcsine polynomial is off by 1e-12 of its value (2^-39.9).
+// Every comparison sums at most three collision angles and three semicircle
+// angles: both sides stay within 2^-31 of the exact formula, and kTau = 2^-30
+// separates them.  (Angles enter the area comparisons with a factor of at most
+// 1 - lambda^2, and so does the bound.)
+//
+// Trap sites and clamps.  eval_box's trap sites are domain and emptiness tests of
+// the quotients.  Each corner that eval_box could evaluate is certified here to
+// stay clear of them (the comments at the corners say why); where it is not, the
+// box is left to eval_box.
+//
+// What it gives: the directed evaluation is bound by issue and by the latency of
+// about 24 certified divisions and 12 padded arcsines per box, each a call.  Here
+// a collision angle costs one approximate reciprocal and two short polynomials,
+// inlined, and most boxes are decided from a few of their angles.  About 1 in 5000
+// lattice boxes is left to eval_box.  On B200: middle, 64^4 lattice and two uniform
+// levels, 494 -> 188 ms; 1e6 complete masks (middle) 390 -> 86 us; half of the start
+// proof 74.6 -> 33.8 ms.
+#pragma once
+#include <cstdint>
+
+#ifdef __CUDACC__
+#include "cp_fp64.cuh"
+#define CPF_HD __host__ __device__ __forceinline__
+#else
+#include <cmath>
+#include <cstring>
+#define CPF_HD inline
+#endif
+
+namespace cpb {
+namespace flt {
+
+// What the caller consumes of a decided box.
+enum Need : int {
+    NEED_VERDICT = 0,  // the verdict alone
+    NEED_HANDLES = 1,  // the verdict and the number of guarded criteria evaluated (DECIDE order)
+    NEED_MASK = 2,     // the fail mask of DECIDE order
+    NEED_FULL = 3      // the complete fail mask
+};
+
+constexpr double kTau = 9.313225746154785e-10;   // 2^-30, bound on an angle sum's error
+constexpr double kAbs = 1.4210854715202004e-14;  // 2^-46, bound on the area terms' own roundings
+constexpr double kEnd = 1.52587890625e-05;       // 2^-16, least distance of a quotient from 1
+constexpr double kTie = 1.4210854715202004e-14;  // 2^-46, least distance from the obtuse/acute boundary
+constexpr double kGap = 9.313225746154785e-10;   // 2^-30, least excess of 2 (a + b) over the lane width
+constexpr double kMinB = 0.000244140625;             // 2^-12
+constexpr double kLowSlack = 3.814697265625e-06;     // 2^-18
+constexpr double kMinC = 0.00390625;                // 2^-8, least a + b
+constexpr double kHalfPi = 1.5707963267948966;
+constexpr double kRatio = 0.5642, kPi = 3.141592653589793;  // lane_packing/values.hpp:28-32
+
+// ------------------------------------------------------------------ arithmetic
+CPF_HD double fma_(double a, double b, double c) {
+#ifdef __CUDA_ARCH__
+    return __fma_rn(a, b, c);
+#else
+    return std::fma(a, b, c);
+#endif
+}
+CPF_HD double abs_(double x) { return x < 0.0 ? -x : x; }
+// seeds of 1/d and 1/sqrt(d): the FP64 approximations, within 2^-19 (host: rounded to float)
+CPF_HD double rcp_seed_(double d) {
+#ifdef __CUDA_ARCH__
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    return y;
+#else
+    return (double)(1.0f / (float)d);
+#endif
+}
+CPF_HD double rsqrt_seed_(double d) {
+#ifdef __CUDA_ARCH__
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    return y;
+#else
+    return (double)(1.0f / std::sqrt((float)d));
+#endif
+}
+CPF_HD double rcp_(double d) {
+    const double y = rcp_seed_(d);
+    return fma_(y, fma_(-d, y, 1.0), y);
+}
+CPF_HD double rsqrt_(double d) {
+    const double y = rsqrt_seed_(d);
+    return fma_(0.5 * y, fma_(-d * y, y, 1.0), y);
+}
+// RD(x + y) doubled and RU(x - y): the side-by-side test of the mixed angles is exact
+CPF_HD double add_rd_(double x, double y) {
+#ifdef __CUDA_ARCH__
+    return __dadd_rd(x, y);
+#else
+    const double s = x + y, t = s - x;
+    return (x - (s - t)) + (y - t) < 0.0 ? std::nextafter(s, -4.0) : s;
+#endif
+}
+CPF_HD double add_ru_(double x, double y) { return -add_rd_(-x, -y); }
+
+// asin(x) = x + x z P(z), z = x^2, |x| <= 1/2: minimax polynomial (Remez exchange
+// on z in [0, 1/4], relative error 9.8e-13).
+CPF_HD double asin_core(double x, double z) {
+    double p = 0.03289646763320449;
+    p = fma_(p, z, 0.0019933684297839347);
+    p = fma_(p, z, 0.020640993408479382);
+    p = fma_(p, z, 0.02186676674568419);
+    p = fma_(p, z, 0.030426411564165902);
+    p = fma_(p, z, 0.044640714121541566);
+    p = fma_(p, z, 0.07500004965298718);
+    p = fma_(p, z, 0.16666666627480178);
+    return fma_(x * z, p, x);
+}
+// asin(n / d) for |n| <= d, r = 1/d: beyond 1/2 from 1 - |n|/d = (d - |n|) r.
+// ok: the quotient keeps kEnd away from 1.
+CPF_HD double asin_quot(double n, double d, double r, bool& ok) {
+    const double an = abs_(n);
+    const double x = an * r, y = (d - an) * r;
+    ok = ok && y >= kEnd;
+    double v;
+    if (y < 0.5) {
+        const double z = 0.5 * y;
+        v = fma_(-2.0, asin_core(z * rsqrt_(z), z), kHalfPi);
+    } else {
+        v = asin_core(x, x * x);
+    }
+    return n < 0.0 ? -v : v;
+}
+
+// ------------------------------------------------------------------ collision angles
+// Disks of radii ro (touching the outer border, centre distance P = 1 - ro) and
+// ri (touching the inner one, Q = lambda + ri, an interval through lambda), upper
+// corner.  The longer of P and Q is the side L; where P lies inside Q both orders
+// are taken, each tightened to L >= S (collision_angles.cu:144-158 and 37-57).
+// With c = ro + ri, the wanted bound is asin((Lh^2 - Sl^2 + c^2) / (2 c Ll)) minus
+// asin((Ll^2 - Sh^2 - c^2) / (2 c S)), S = Sh where the angle at S is obtuse, else
+// Sl: the obtuse and acute formulas (collision_angles.cu:59-117) agree at their
+// boundary, so a comparison near it needs no care.
+// Trap sites: the first quotient exceeds 1 only when 2 c <= 1 - lambda.lo (to
+// rounding), where the directed value is clamped if the angle is definitely obtuse
+// and a trap otherwise.  The second exceeds 1 only beyond Sh + c < Ll.
+CPF_HD double mixed_hi_order(double Ll, double Lh, double Sl, double Sh, double c, bool& ok) {
+    const double c2 = c * c, cc = c + c;
+    const double al = fma_(Ll, Ll, -(Sh * Sh)), ah = fma_(Lh, Lh, -(Sl * Sl));
+    const double n1 = ah + c2, n2 = al - c2;
+    const double d1 = cc * Ll, d2 = cc * (n2 > 0.0 ? Sh : Sl);
+    const double r = rcp_(d1 * d2);
+    double v1;
+    if (n1 > d1) {  // clamped to 1: definitely obtuse, clear of 1, lower quotient inside
+        const double d3 = cc * Lh;
+        ok = ok && n2 > kTie && (n1 - d1) >= kEnd * d1 && (d3 - (al + c2)) >= kEnd * d3;
+        v1 = kHalfPi;
+    } else {
+        v1 = asin_quot(n1, d1, r * d2, ok);
+    }
+    return v1 - asin_quot(n2, d2, r * d1, ok);
+}
+CPF_HD double mixed_hi(double ll, double lh, double ro, double ri, bool& ok) {
+    const double P = 1.0 - ro, ql = ll + ri, qh = lh + ri, c = ro + ri;
+    const bool x = ql <= P;
+    double v = mixed_hi_order(x ? P : ql, x ? P : qh, x ? ql : P, x ? (qh < P ? qh : P) : P, c, ok);
+    if (x && qh > P) {
+        const double w = mixed_hi_order(P, qh, P, P, c, ok);
+        if (w > v) v = w;
+    }
+    return v;
+}
+// Lower corner, not side by side: asin((Ll^2 - Sh^2 + c^2) / (2 c Lh)) minus
+// asin((Lh^2 - Sl^2 - c^2) / (2 c S)) (S = Sl where possibly obtuse, else Sh), at
+// least 0; the second quotient is clamped to 1.
+// Trap sites: unless definitely obtuse, (Lh^2 - Sl^2 + c^2) / (2 c Ll) > 1; if
+// obtuse, (Ll^2 - Sh^2 - c^2) / (2 c Sh) > 1.
+CPF_HD double mixed_lo_order(double Ll, double Lh, double Sl, double Sh, double c, bool& ok) {
+    const double c2 = c * c, cc = c + c;
+    double al = fma_(Ll, Ll, -(Sh * Sh));
+    const double ah = fma_(Lh, Lh, -(Sl * Sl));
+    const double n1 = al + c2, n2 = ah - c2;
+    const double d1 = cc * Lh, d2 = cc * (n2 > 0.0 ? Sl : Sh);
+    const double r = rcp_(d1 * d2);
+    if (al <= c2 + kTie) {
+        const double d3 = cc * Ll;
+        ok = ok && d3 - (ah + c2) >= kEnd * d3;
+    } else {
+        const double d3 = cc * Sh;
+        ok = ok && d3 - (al - c2) >= kEnd * d3;
+    }
+    double v2;
+    if (n2 > d2) {
+        ok = ok && n2 - d2 >= kEnd * d2;
+        v2 = kHalfPi;
+    } else {
+        v2 = asin_quot(n2, d2, r * d1, ok);
+    }
+    const double v = asin_quot(n1, d1, r * d2, ok) - v2;
+    return v < 0.0 ? 0.0 : v;
+}
+// the exact test of collision_angles.cu:160-173: disks that possibly fit side by side
+CPF_HD bool side_by_side(double ll, double ro, double ri) { return 2.0 * add_rd_(ro, ri) <= add_ru_(1.0, -ll); }
+CPF_HD double mixed_lo(double ll, double lh, double ro, double ri, bool& ok) {
+    if (side_by_side(ll, ro, ri)) return 0.0;
+    const double P = 1.0 - ro, ql = ll + ri, qh = lh + ri, c = ro + ri;
+    const bool x = ql <= P;
+    double v = mixed_lo_order(x ? P : ql, x ? P : qh, x ? ql : P, x ? (qh < P ? qh : P) : P, c, ok);
+    if (x && qh > P) {
+        const double w = mixed_lo_order(P, qh, P, P, c, ok);
+        if (w < v) v = w;
+    }
+    return v;
+}
+// Certificates for corners whose value is not needed.  With D = 2 (a + b) - (1 -
+// lambda.lo) > 0 no quotient of a mixed corner exceeds 1: in the order L = P the
+// excess is -D (P - c + ql), in the order L = Q it is bounded by the box guard.
+CPF_HD bool clear_mixed_hi(double ll, double lh, double ro, double ri) {
+    const double c = ro + ri;
+    bool clear = 2.0 * c - (1.0 - ll) >= kGap;
+    if (!clear) {  // definitely obtuse: the first quotient is clamped, its lower end below 1
+        const double P = 1.0 - ro, qh = lh + ri;
+        clear = 2.0 * c - (1.0 - lh) >= kGap && qh < P && fma_(P, P, -(qh * qh)) - c * c > kTie;
+    }
+    return clear;
+}
+CPF_HD bool clear_mixed_lo(double ll, double ro, double ri) {
+    return side_by_side(ll, ro, ri) || 2.0 * (ro + ri) - (1.0 - ll) >= kGap;
+}
+
+// The directed evaluation's own trap test of the upper corner of disks 2 and 3 (no
+// arcsine), for end_3d: its radii ranges end at r2 = r3 = (1 - lambda.hi) / 4, where the lower
+// quotient is 1 to the last bit, so no margin can certify that corner.  Host builds
+// leave those boxes undecided.
+CPF_HD bool exact_clear_23_hi(double ll, double lh, double h2, double h3, bool inner) {
+#ifdef __CUDA_ARCH__
+    bool trap = false;
+    if (inner)
+        ca_mixed_hi<true, true>(Iv{ll, lh}, pt(h2), pt(h3), trap);
+    else
+        ca_mixed_hi<false, true>(Iv{ll, lh}, pt(h2), pt(h3), trap);
+    return !trap;
+#else
+    return false;
+#endif
+}
+
+// Two disks on the same border, a >= b: near-point sides L = x + a, S = x + b
+// (inner, x = lambda) or 1 - b, 1 - a (outer), twox + c = L + S, so the angle is
+// the point formula cos = 1 - 2 a b / (L S): 2 asin(sqrt(a b / (L S))).  1 - q >=
+// b / c keeps the directed evaluation clear of 1 for b >= kMinB, and |L^2 - S^2 -
+// c^2| > kTie clear of an empty partial result at the obtuse/acute boundary.
+CPF_HD double excess(double a, double b, double sides) {
+    const double c = a + b;
+    return fma_(a - b, sides, -(c * c));  // L^2 - S^2 - c^2
+}
+CPF_HD bool clear_same(double a, double b, double sides) {
+    return a >= b && b >= kMinB && abs_(excess(a, b, sides)) > kTie;
+}
+// Lower corner of a radius b below kMinB (end_3d: down to 0): definitely obtuse, both
+// quotients at most 1 before their rounding, which is downward, so no trap site is
+// reached; the directed value lies within kLowSlack below the angle.
+CPF_HD bool clear_same_low(double a, double b, double sides) {
+    return a >= b && (b >= kMinB ? abs_(excess(a, b, sides)) > kTie : excess(a, b, sides) > kTie);
+}
+CPF_HD double sides_inner(double x, double a, double b) { return 2.0 * x + (a + b); }
+CPF_HD double sides_outer(double a, double b) { return 2.0 - (a + b); }
+CPF_HD double same_angle(double a, double b, double L, double S) {
+    double ab = a * b;
+    if (ab < 1e-30) ab = 1e-30;  // b = 0: an angle of 2e-15
+    const double s = ab * rsqrt_(ab * (L * S));
+    return 2.0 * asin_core(s, s * s);
+}
+CPF_HD double inner_angle(double x, double a, double b) { return same_angle(a, b, x + a, x + b); }
+CPF_HD double outer_angle(double a, double b) { return same_angle(a, b, 1.0 - a, 1.0 - b); }
+
+// collision_angles.cu:233-246, quotients at most 1/2
+CPF_HD double semi_angle(double r, double d) {
+    const double x = r * rcp_(d);
+    return asin_core(x, x * x);
+}
+CPF_HD double semi_outer(double r) { return semi_angle(r, 1.0 - r); }
+CPF_HD double semi_inner(double x, double r) { return semi_angle(r, x + r); }
+
+// x < y, decided only when they are more than tol apart
+CPF_HD bool less_(double x, double y, double tol, bool& ok) {
+    const double d = y - x;
+    ok = ok && abs_(d) > tol;
+    return d > 0.0;
+}
+
+// ------------------------------------------------------------------ boxes
+struct FBox {
+    double ll, lh;             // lambda
+    double l1, h1, l2, h2, l3, h3;  // radii (lower ends tightened)
+};
+// The guard of the error bound (negated comparisons, so NaN fails): see the file
+// comment.  lh - ll >= 2^-40 keeps the two ends of a mixed corner's L^2 - S^2 apart,
+// so that they do not both fall on the obtuse/acute boundary; the last test bounds
+// the first quotient of the order L = Q: (1 - lh)(P + qh - c) > 2 c (lh - ll).
+template <bool THREE>
+CPF_HD bool box_ok(const FBox& b) {
+    const double w = b.lh - b.ll;
+    double m = b.h1 > b.h2 ? b.h1 : b.h2;
+    bool ok = b.ll >= 0.49 && b.lh <= 0.992 && w >= 9.094947017729282e-13;
+    ok = ok && b.l1 > 0.0 && b.l2 >= 0.0 && b.l1 <= b.h1 && b.l2 <= b.h2 && b.h1 + b.h2 >= kMinC;
+    if (THREE) {
+        ok = ok && b.l3 >= 0.0 && b.l3 <= b.h3 && b.h2 + b.h3 >= kMinC && b.l1 + b.l3 >= 0.5 * kMinC;
+        if (b.h3 > m) m = b.h3;
+    }
+    ok = ok && m <= 0.3333;
+    return ok && (1.0 - b.lh) * (1.0 + b.lh - 2.0 * m) >= fma_(4.0 * m, w, kGap);
+}
+
+struct FOut {
+    uint8_t mask;     // NEED_MASK / NEED_FULL: failing sub-criteria; else nonzero when a criterion fails
+    uint8_t handles;  // NEED_HANDLES
+};
+
+// middle_configuration.cu:86-154.  The handle fails when (g1 and A) or (g2 and B):
+// g1, g2 its two guards, A, B its two area tests.  c13.hi <= (c12 + c23).lo rules
+// out c13.lo > (c12 + c23).hi (directed bounds of angles that grow with the
+// radii), so g1 or g2 always holds: a handle whose tests both fail (both hold)
+// fails (holds) whatever its guards say, and they are evaluated only in between.
+template <int NEED>
+CPF_HD uint8_t middle_handle(const FBox& b, bool inner, double ratio, double tol, double ar1, double ar2, double ar3,
+                             bool& ok) {
+    const double ro12h = inner ? b.h2 : b.h1, ri12h = inner ? b.h1 : b.h2;
+    const double ro12l = inner ? b.l2 : b.l1, ri12l = inner ? b.l1 : b.l2;
+    const double ro23h = inner ? b.h2 : b.h3, ri23h = inner ? b.h3 : b.h2;
+    const double ro23l = inner ? b.l2 : b.l3, ri23l = inner ? b.l3 : b.l2;
+    const double c12_hi = mixed_hi(b.ll, b.lh, ro12h, ri12h, ok);
+    double c13_hi;
+    if (inner) {
+        ok = ok && clear_same(b.h1, b.h3, sides_inner(b.ll, b.h1, b.h3)) && clear_same(b.l1, b.l3, sides_inner(b.lh, b.l1, b.l3));
+        c13_hi = inner_angle(b.ll, b.h1, b.h3);
+    } else {
+        ok = ok && clear_same(b.h1, b.h3, sides_outer(b.h1, b.h3)) && clear_same(b.l1, b.l3, sides_outer(b.l1, b.l3));
+        c13_hi = outer_angle(b.h1, b.h3);
+    }
+    ok = ok && clear_mixed_hi(b.ll, b.lh, ro23h, ri23h) && clear_mixed_lo(b.ll, ro12l, ri12l) &&
+         clear_mixed_lo(b.ll, ro23l, ri23l);
+    const double k = 0.5 * kRatio * ratio;
+    const bool fa = less_(0.5 * (ar1 + ar2), k * c12_hi, tol, ok);
+    const bool fb = less_(fma_(0.5, ar1 + ar3, ar2), k * c13_hi, tol, ok);
+    if (!ok) return 0;
+    if (!fa && !fb) return 0;
+    if (NEED < NEED_MASK && fa && fb) return 3;
+    uint8_t m = 0;
+    if (fa) {
+        const double c13_lo = inner ? inner_angle(b.lh, b.l1, b.l3) : outer_angle(b.l1, b.l3);
+        const double c23_hi = mixed_hi(b.ll, b.lh, ro23h, ri23h, ok);
+        if (less_(c13_lo, c12_hi + c23_hi, kTau, ok)) m |= 1;
+        if (NEED != NEED_FULL && m) return m;
+    }
+    if (fb) {
+        const double c12_lo = mixed_lo(b.ll, b.lh, ro12l, ri12l, ok);
+        const double c23_lo = mixed_lo(b.ll, b.lh, ro23l, ri23l, ok);
+        if (!less_(c13_hi, c12_lo + c23_lo, kTau, ok)) m |= 2;
+    }
+    return m;
+}
+
+// end_configuration.cu:71-101
+CPF_HD bool end2d_fails(const FBox& b, bool inner, double ratio, double tol, double ar1, double ar2, bool& ok) {
+    const double roh = inner ? b.h2 : b.h1, rih = inner ? b.h1 : b.h2;
+    const double rol = inner ? b.l2 : b.l1, ril = inner ? b.l1 : b.l2;
+    ok = ok && clear_mixed_lo(b.ll, rol, ril);
+    const double ca_hi = mixed_hi(b.ll, b.lh, roh, rih, ok);
+    const double sa_hi = inner ? semi_outer(b.h2) : semi_inner(b.ll, b.h2);
+    const double other = inner ? semi_inner(b.ll, b.h1) : semi_outer(b.h1);
+    const double t = inner ? 1.0 - 2.0 * b.h2 : fma_(2.0, b.h2, b.lh);
+    double rho = inner ? t * t - b.lh * b.lh : 1.0 - t * t;
+    if (rho < 0.0) rho = 0.0;
+    const double a_hi = ca_hi + sa_hi, used = 0.5 * ratio * a_hi;
+    const double lhs = fma_(0.5, ar1, ar2);
+    // reusable = 0.5 rho (a.lo - other), a.lo in [0, a.hi]
+    if (!ok) return false;
+    if (lhs - kRatio * fma_(0.5 * rho, other, used) > tol) return false;
+    if (lhs - kRatio * fma_(0.5 * rho, other - a_hi, used) < -tol) return true;
+    const double a_lo = mixed_lo(b.ll, b.lh, rol, ril, ok) + (inner ? semi_outer(b.l2) : semi_inner(b.lh, b.l2));
+    return less_(lhs, kRatio * fma_(0.5 * rho, other - a_lo, used), tol, ok);
+}
+
+// end_configuration.cu:154-210
+CPF_HD bool end3d_fails(const FBox& b, bool inner, double ratio, double tol, double ar1, double ar2, double ar3,
+                        bool& ok) {
+    const double ro12h = inner ? b.h2 : b.h1, ri12h = inner ? b.h1 : b.h2;
+    const double ro12l = inner ? b.l2 : b.l1, ri12l = inner ? b.l1 : b.l2;
+    const double ro23h = inner ? b.h2 : b.h3, ri23h = inner ? b.h3 : b.h2;
+    const double ro23l = inner ? b.l2 : b.l3, ri23l = inner ? b.l3 : b.l2;
+    double a13_hi;
+    if (inner) {
+        ok = ok && clear_same(b.h1, b.h3, sides_inner(b.ll, b.h1, b.h3)) && clear_same_low(b.l1, b.l3, sides_inner(b.lh, b.l1, b.l3));
+        a13_hi = inner_angle(b.ll, b.h1, b.h3);
+    } else {
+        ok = ok && clear_same(b.h1, b.h3, sides_outer(b.h1, b.h3)) && clear_same_low(b.l1, b.l3, sides_outer(b.l1, b.l3));
+        a13_hi = outer_angle(b.h1, b.h3);
+    }
+    ok = ok && clear_mixed_hi(b.ll, b.lh, ro12h, ri12h) && clear_mixed_lo(b.ll, ro12l, ri12l) &&
+         clear_mixed_lo(b.ll, ro23l, ri23l) &&
+         (clear_mixed_hi(b.ll, b.lh, ro23h, ri23h) || exact_clear_23_hi(b.ll, b.lh, b.h2, b.h3, inner));
+    if (!ok) return false;
+    const double s_lo = mixed_lo(b.ll, b.lh, ro12l, ri12l, ok) + mixed_lo(b.ll, b.lh, ro23l, ri23l, ok);
+    if (less_(a13_hi, s_lo, kTau, ok)) return false;
+    const double a13_lo = inner ? inner_angle(b.lh, b.l1, b.l3) : outer_angle(b.l1, b.l3);
+    const double a12_hi = mixed_hi(b.ll, b.lh, ro12h, ri12h, ok);
+    const double a3_lo = inner ? semi_inner(b.lh, b.l3) : semi_outer(b.l3);
+    const double a3_hi = inner ? semi_inner(b.ll, b.h3) : semi_outer(b.h3);
+    const double a2_hi = inner ? semi_outer(b.h2) : semi_inner(b.ll, b.h2);
+    const double t = inner ? fma_(2.0, b.h3, b.lh) : 1.0 - 2.0 * b.h3;
+    double rho = inner ? 1.0 - t * t : t * t - b.lh * b.lh;
+    if (rho < 0.0) rho = 0.0;
+    const double alpha = (a13_lo + a3_lo) - (a12_hi + a2_hi);
+    const double used = 0.5 * ratio * (a13_hi + a3_hi);
+    if (b.l3 < kMinB) tol = fma_(0.5 * kLowSlack, rho, tol);
+    return less_(fma_(0.5, ar1, ar2 + ar3), kRatio * fma_(-0.5 * rho, alpha, used), tol, ok);
+}
+
+// The verdict of a box that is neither empty nor stopped by the fit check.  order:
+// bit 0 = second handle first (DECIDE).  Returns false when the box is left to
+// eval_box; else o holds what NEED asks for.
+template <int FAM, int NEED>
+CPF_HD bool filter_box(const FBox& b, int order, FOut& o) {
+    constexpr bool kThree = FAM != 1 && FAM != 4;
+    bool ok = box_ok<kThree>(b);
+    if (!ok) return false;
+    o.mask = 0;
+    o.handles = 1;
+    const double ratio = fma_(-b.ll, b.ll, 1.0);
+    const double tol = fma_(kTau, ratio, kAbs);
+    const double ar1 = kPi * (b.l1 * b.l1), ar2 = kPi * (b.l2 * b.l2), ar3 = kPi * (b.l3 * b.l3);
+    if (FAM == 0) {  // start_configuration.cu:126-162
+        ok = clear_same(b.h1, b.h3, sides_outer(b.h1, b.h3)) && clear_same(b.l1, b.l3, sides_outer(b.l1, b.l3)) && clear_mixed_hi(b.ll, b.lh, b.h3, b.h2) &&
+             clear_mixed_lo(b.ll, b.l1, b.l2) && clear_mixed_lo(b.ll, b.l3, b.l2);
+        if (!ok) return false;
+        const double so = semi_outer(b.h1);
+        const double a12_hi = mixed_hi(b.ll, b.lh, b.h1, b.h2, ok);
+        const double a13_hi = outer_angle(b.h1, b.h3);
+        const double k = 0.5 * kRatio * ratio;
+        const bool f1 = less_(fma_(0.5, ar2, ar1), k * (so + a12_hi), tol, ok);
+        const bool f2 = less_(fma_(0.5, ar3, ar1 + ar2), k * (so + a13_hi), tol, ok);
+        if (!ok) return false;
+        // criterion 1 is evaluated when a12 + a23 > a13 possibly holds, criterion 2
+        // unless it definitely holds; "definitely" implies "possibly"
+        if (NEED < NEED_MASK && f1 && f2) {
+            o.mask = 1;
+            return true;
+        }
+        if (NEED != NEED_HANDLES && !f1 && !f2) return true;
+        bool pos = true, def = false;
+        if (f2 || NEED == NEED_HANDLES) {
+            def = less_(a13_hi, mixed_lo(b.ll, b.lh, b.l1, b.l2, ok) + mixed_lo(b.ll, b.lh, b.l3, b.l2, ok), kTau, ok);
+            if (!ok) return false;
+        }
+        if ((f1 || NEED == NEED_HANDLES) && !def)
+            pos = less_(outer_angle(b.l1, b.l3), a12_hi + mixed_hi(b.ll, b.lh, b.h3, b.h2, ok), kTau, ok);
+        if (pos && f1) o.mask |= 1;
+        if (NEED != NEED_FULL && o.mask) return ok;
+        if (!def && f2) o.mask |= 2;
+        o.handles = (pos ? 1 : 0) + (def ? 0 : 1);
+        return ok;
+    } else if (FAM == 1) {  // start_configuration.cu:169-188
+        ok = clear_mixed_lo(b.ll, b.l1, b.l2);
+        const double a1 = semi_outer(b.h1), a2_hi = semi_inner(b.ll, b.h2);
+        const double a12_hi = mixed_hi(b.ll, b.lh, b.h1, b.h2, ok);
+        const double t = fma_(2.0, b.h2, b.lh);
+        double rho = 1.0 - t * t;
+        if (rho < 0.0) rho = 0.0;
+        const double used = 0.5 * ratio * (a1 + a2_hi + a12_hi), lhs = ar1 + ar2;
+        if (!ok) return false;
+        // the reused angle lies between 0 and a12.hi + a2.hi - a1
+        if (lhs - kRatio * used > tol) return true;
+        double top = a12_hi + a2_hi - a1;
+        if (top < 0.0) top = 0.0;
+        if (lhs - kRatio * fma_(-0.5 * rho, top, used) < -tol) {
+            o.mask = 1;
+            return true;
+        }
+        double reuse = mixed_lo(b.ll, b.lh, b.l1, b.l2, ok) + semi_inner(b.lh, b.l2) - a1;
+        if (reuse < 0.0) reuse = 0.0;
+        if (less_(lhs, kRatio * fma_(-0.5 * rho, reuse, used), tol, ok)) o.mask = 1;
+        return ok;
+    } else if (FAM == 2) {  // start_configuration.cu:227-265 (a13 of r1 and r2, as there)
+        ok = clear_same(b.h1, b.h2, sides_outer(b.h1, b.h2)) && clear_same(b.l1, b.l2, sides_outer(b.l1, b.l2)) && clear_mixed_lo(b.ll, b.l1, b.l2) &&
+             clear_mixed_lo(b.ll, b.l3, b.l2);
+        if (!ok) return false;
+        const double a1_hi = semi_outer(b.h1), a2_hi = semi_inner(b.ll, b.h2), a3_hi = semi_outer(b.h3);
+        const double a12_hi = mixed_hi(b.ll, b.lh, b.h1, b.h2, ok), a13_hi = outer_angle(b.h1, b.h2);
+        const double a23_hi = mixed_hi(b.ll, b.lh, b.h3, b.h2, ok);
+        const double b123_hi = a12_hi + a23_hi, b13_hi = a13_hi < b123_hi ? b123_hi : a13_hi;
+        const double a123_hi = a1_hi + b13_hi + a3_hi, a122_hi = a1_hi + a12_hi + a2_hi;
+        const double a_hi = a123_hi < a122_hi ? a122_hi : a123_hi;
+        const double outer = fma_(-2.0, b.h3, 1.0);
+        double lane = 0.5 * (outer * outer - b.lh * b.lh);
+        if (lane < 0.0) lane = 0.0;
+        const double used = 0.5 * ratio * a_hi, lhs = ar1 + (ar2 + ar3);
+        if (!ok) return false;
+        // the reused angle a.lo - a122.hi lies between 0 and a.hi - a122.hi
+        if (lhs - kRatio * used > tol) return true;
+        if (lhs - kRatio * fma_(-lane, a_hi - a122_hi, used) < -tol) {
+            o.mask = 1;
+            return true;
+        }
+        const double a1_lo = semi_outer(b.l1), a2_lo = semi_inner(b.lh, b.l2), a3_lo = semi_outer(b.l3);
+        const double a12_lo = mixed_lo(b.ll, b.lh, b.l1, b.l2, ok), a13_lo = outer_angle(b.l1, b.l2);
+        const double b123_lo = a12_lo + mixed_lo(b.ll, b.lh, b.l3, b.l2, ok);
+        const double b13_lo = a13_lo < b123_lo ? b123_lo : a13_lo;
+        const double a123_lo = a1_lo + b13_lo + a3_lo, a122_lo = a1_lo + a12_lo + a2_lo;
+        double reuse = (a123_lo < a122_lo ? a122_lo : a123_lo) - a122_hi;
+        if (reuse < 0.0) reuse = 0.0;
+        if (less_(lhs, kRatio * fma_(-lane, reuse, used), tol, ok)) o.mask = 1;
+        return ok;
+    } else if (FAM == 3) {
+        const bool second = NEED != NEED_FULL && (order & 1);
+        uint8_t h = 0;
+        for (int i = 0; i < 2; ++i) {
+            const bool inner = (i == 0) != second;
+            ++h;
+            const uint8_t m = middle_handle<NEED>(b, inner, ratio, tol, ar1, ar2, ar3, ok);
+            if (!ok) return false;
+            o.mask |= inner ? m : (uint8_t)(m << 2);
+            if (NEED != NEED_FULL && m) break;
+        }
+        o.handles = h;
+        return true;
+    } else {
+        const bool second = NEED != NEED_FULL && (order & 1);
+        uint8_t h = 0;
+        for (int i = 0; i < 2; ++i) {
+            const bool inner = (i == 0) != second;
+            ++h;
+            const bool f = FAM == 4 ? end2d_fails(b, inner, ratio, tol, ar1, ar2, ok)
+                                    : end3d_fails(b, inner, ratio, tol, ar1, ar2, ar3, ok);
+            if (!ok) return false;
+            if (f) {
+                o.mask |= inner ? 1 : 2;
+                if (NEED != NEED_FULL) break;
+            }
+        }
+        o.handles = h;
+        return true;
+    }
+}
+
+}  // namespace flt
+}  // namespace cpb

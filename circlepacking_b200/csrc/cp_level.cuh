@@ -97,7 +97,7 @@ __device__ __forceinline__ void level_smem_init(LevelSmem<WARPS>& sm) {
 template <int FAM, int WARPS>
 __device__ __forceinline__ void level_emit(const LevelArgs& a, LevelSmem<WARPS>& sm, int v, bool clipped,
                                            bool fp32_decided, const double* lo, const double* hi, int depth,
-                                           int given, const LaFree& lf);
+                                           int given);
 
 // One lane's box j of the chunk (j >= a.count: the lane only takes part in the
 // warp's collective child write).  All 32 lanes of the warp must call it.
@@ -111,7 +111,6 @@ __device__ __forceinline__ void level_step(const LevelArgs& a, size_t j, LevelSm
     double lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
     int depth = 0, given = 0;
     int v = -1;                 // this lane's verdict (-1: no box evaluated)
-    LaFree lf{0.0, 0.0, 0.0, 0.0};  // start family: the box's lambda-independent terms, when known
     bool clipped = false, fp32_decided = false;
     if (j < a.count) {
         depth = a.in.depth[i];
@@ -124,21 +123,11 @@ __device__ __forceinline__ void level_step(const LevelArgs& a, size_t j, LevelSm
                 hi[d] = a.in.hi[d * a.in.cap + i];
             }
             const int ord = ord_in >= 0 ? ord_in : (a.order_hint ? a.order_hint[j] : 0);
-            LaFree lin{0.0, 0.0, 0.0, 0.0};
-            if (FAM == F_START && a.in.aux) {
-                lin.flag = a.in.aux[3 * a.in.cap + i];
-                if (lin.flag != 0.0) {
-                    lin.a13lo = a.in.aux[i];
-                    lin.a13hi = a.in.aux[a.in.cap + i];
-                    lin.so_hi = a.in.aux[2 * a.in.cap + i];
-                }
-                lf = lin;
-            }
             if (PREC == CP_FP32_PREFILTER) {
                 uint8_t pmask;
                 const int pre = prefilter_box<FAM>(lo, hi, ord, false, &pmask);
                 if (pre == PF_UNDECIDED) {
-                    const Verdict r = eval_box<FAM, DECIDE>(lo, hi, ord, nullptr, &lin, &lf);
+                    const Verdict r = judge_box<FAM, DECIDE, flt::NEED_HANDLES>(lo, hi, ord);
                     v = r.verdict;
                     handles += r.handles;
                 } else {
@@ -146,25 +135,25 @@ __device__ __forceinline__ void level_step(const LevelArgs& a, size_t j, LevelSm
                     fp32_decided = pre != PF_EMPTY;
                 }
             } else {
-                const Verdict r = eval_box<FAM, DECIDE>(lo, hi, ord, nullptr, &lin, &lf);
+                const Verdict r = judge_box<FAM, DECIDE, flt::NEED_HANDLES>(lo, hi, ord);
                 v = r.verdict;
                 handles += r.handles;
             }
             if (a.policy == SPLIT_GIVEN) given = axis_in >= 0 ? axis_in % D : (a.axis_hint ? (a.axis_hint[j] % D) : 0);
         }
     }
-    level_emit<FAM>(a, sm, v, clipped, fp32_decided, lo, hi, depth, given, lf);
+    level_emit<FAM>(a, sm, v, clipped, fp32_decided, lo, hi, depth, given);
 }
 
 // The end of a level step, for every lane of a warp (all 32 must call it):
 // v = the lane's verdict (-1: no box evaluated), its box lo/hi and depth,
-// given = its split axis for SPLIT_GIVEN, lf = its lambda-independent terms.
+// given = its split axis for SPLIT_GIVEN.
 // Counts the verdicts, folds the digest and writes the children of every box
 // that is neither proved nor empty (unresolved at the depth limit).
 template <int FAM, int WARPS>
 __device__ __forceinline__ void level_emit(const LevelArgs& a, LevelSmem<WARPS>& sm, int v, bool clipped,
                                            bool fp32_decided, const double* lo, const double* hi, int depth,
-                                           int given, const LaFree& lf) {
+                                           int given) {
     constexpr int D = family_dims(FAM);
     unsigned nchild = 0;
     int axis = 0;
@@ -246,13 +235,6 @@ __device__ __forceinline__ void level_emit(const LevelArgs& a, LevelSmem<WARPS>&
                 const int c = (int)k - (int)__shfl_sync(0xffffffffu, excl, own);
                 const int pax = __shfl_sync(0xffffffffu, axis, own);
                 const int pdep = __shfl_sync(0xffffffffu, depth, own);
-                LaFree plf{0.0, 0.0, 0.0, 0.0};
-                if (FAM == F_START && a.out.aux) {
-                    plf.a13lo = __shfl_sync(0xffffffffu, lf.a13lo, own);
-                    plf.a13hi = __shfl_sync(0xffffffffu, lf.a13hi, own);
-                    plf.so_hi = __shfl_sync(0xffffffffu, lf.so_hi, own);
-                    plf.flag = __shfl_sync(0xffffffffu, lf.flag, own);
-                }
                 if (valid) {
                     make_child<D>(plo, phi, a.policy, pax, c, clo, chi);
                     const bool alive = clip_child<FAM>(clo, chi, a.tab);
@@ -263,20 +245,6 @@ __device__ __forceinline__ void level_emit(const LevelArgs& a, LevelSmem<WARPS>&
                         a.out.hi[d * a.out.cap + o] = chi[d];
                     }
                     a.out.depth[o] = alive ? (uint8_t)(pdep + 1) : (uint8_t)0xFF;
-                    if (FAM == F_START && a.out.aux) {
-                        // the parent's terms hold for the child when its radii are the parent's, bit for bit
-                        bool same = plf.flag != 0.0;
-#pragma unroll
-                        for (int d = 1; d < D; ++d)
-                            same = same && __double_as_longlong(clo[d]) == __double_as_longlong(plo[d]) &&
-                                   __double_as_longlong(chi[d]) == __double_as_longlong(phi[d]);
-                        a.out.aux[3 * a.out.cap + o] = same ? plf.flag : 0.0;
-                        if (same) {
-                            a.out.aux[o] = plf.a13lo;
-                            a.out.aux[a.out.cap + o] = plf.a13hi;
-                            a.out.aux[2 * a.out.cap + o] = plf.so_hi;
-                        }
-                    }
                 }
             }
             __syncwarp();

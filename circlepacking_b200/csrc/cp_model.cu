@@ -1065,7 +1065,7 @@ __global__ void __launch_bounds__(128) k_label(LabelArgs a) {
             lo[d] = a.in.lo[d * a.in.cap + i];
             hi[d] = a.in.hi[d * a.in.cap + i];
         }
-        const Verdict v = eval_box<FAM, FULL>(lo, hi, 0, nullptr);
+        const Verdict v = judge_box<FAM, FULL, flt::NEED_FULL>(lo, hi, 0);
         if (v.verdict == V_EMPTY) continue;
         int label = -1;
         if (v.verdict == V_CRITICAL) {

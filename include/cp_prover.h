@@ -76,7 +76,9 @@ typedef enum cp_verdict {
 #define CP_MASK_TRAP 0x80u
 
 typedef enum cp_precision {
-    CP_FP64 = 0,           /* FP64 directed rounding, bit-identical to the reference */
+    CP_FP64 = 0,           /* FP64: verdicts of the reference's directed rounding, decided by a round-to-nearest
+                              FP64 evaluation where every comparison clears its error bound, else by directed
+                              rounding, bit-identical to the reference */
     CP_FP32_PREFILTER = 1  /* FP32 enclosure pass issues PROVED; every other box is re-evaluated in FP64 */
 } cp_precision;
 
@@ -203,11 +205,8 @@ typedef struct cp_refine_opts {
     int32_t seed_part;      /* ... and refines piece seed_part only: lattice boxes seed_part + k * seed_parts
                                (one rank's share of the same proof; the pieces' reports add up to the
                                whole seed's, digests included) */
-    int32_t reuse;          /* start family: 1 = a child whose radii equal its parent's (every child of a
-                               lambda-only split that clipping leaves alone) takes the parent's
-                               lambda-independent criterion terms instead of recomputing them (same
-                               values bit for bit; 32 B more per box in the levels above the seed);
-                               0 = every box computes every term */
+    int32_t reuse;          /* accepted, without effect: every box computes every term it needs (the
+                               filter needs too few of them for carrying a parent's to pay) */
 } cp_refine_opts;
 
 /* Refinement engines.  CP_ENGINE_LEVELS: the host picks each chunk, launches
@@ -390,6 +389,12 @@ cp_status cp_div_check(const double* a, const double* b, size_t n, double* out, 
  * __fdiv_rd / __fdiv_ru it replaces.  a, b: n device floats; out: 4n device
  * floats per element (library RD, library RU, __fdiv_rd, __fdiv_ru). */
 cp_status cp_fdiv_check(const float* a, const float* b, size_t n, float* out, void* stream);
+
+/* Diagnostics: the largest relative errors of the FP64 reciprocal (out[0]) and
+ * reciprocal square root (out[1]) approximations that the FP64 filter starts
+ * from, over every upper word of operands in [2^-120, 2^4).  out: 2 device
+ * doubles.  Asynchronous. */
+cp_status cp_seed_error(double* out, void* stream);
 
 /* Diagnostics: measured peak throughput (operations per second, whole device)
  * of the FP64 primitives the criteria use, each run alone with full occupancy
