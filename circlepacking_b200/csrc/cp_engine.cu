@@ -15,6 +15,7 @@
 #include "cp_engine.h"
 #include "cp_graph_kernels.cuh"
 #include "cp_level.cuh"
+#include "cp_refine.cuh"
 
 using namespace cpb;
 
@@ -39,7 +40,22 @@ __host__ __device__ __forceinline__ double ordered_value(unsigned long long u) {
 // MINB: minimum resident blocks per SM requested from the compiler (register cap
 // 65536 / (128 * MINB)); the autotuner picks the variant per family and precision.
 template <int FAM, int PREC, int MINB>
-__global__ void __launch_bounds__(kEvalBlock, MINB) k_level(LevelArgs a) {
+__global__ void __launch_bounds__(kEvalBlock, MINB) k_level(RefineArgs r) {
+    constexpr unsigned kWarps = kEvalBlock / 32;
+    __shared__ LevelSmem<kWarps> sm;
+    __shared__ WarpBoxes<family_dims(FAM)> wb[kWarps];
+    level_smem_init(sm);
+    __syncthreads();
+    unsigned handles = 0;
+    const unsigned w = threadIdx.x >> 5;
+    refine_warp<FAM, PREC, false>(r, sm, wb[w], gridDim.x * kWarps, blockIdx.x * kWarps + w, handles);
+    level_flush(r.level, sm, handles);
+}
+
+// The level kernel for refinements in which every box passes through a level:
+// per-box proposals of the learned model, and the collection of its records.
+template <int FAM, int PREC>
+__global__ void __launch_bounds__(kEvalBlock) k_level_each(LevelArgs a) {
     __shared__ LevelSmem<kEvalBlock / 32> sm;
     level_smem_init(sm);
     __syncthreads();
@@ -86,7 +102,20 @@ __global__ void k_copy_seed(int dims, const double* __restrict__ lo, const doubl
     }
 }
 
-__global__ void k_set_u64(unsigned long long* p, unsigned long long v) { *p = v; }
+// A chunk of the host-driven loop starts: its children append at `base`, none of
+// its boxes is handed out yet.
+__global__ void k_begin_chunk(unsigned long long* cnt, unsigned long long base) {
+    cnt[C_OUT] = base;
+    cnt[C_CLAIM] = 0;
+}
+// A depth-first refinement of `count` seed boxes starts.
+__global__ void k_begin_deep(DeepSched* s, unsigned long long count) {
+    if (threadIdx.x != 0) return;
+    const unsigned long long epoch = s->epoch + 2;  // no flag of an earlier refinement carries this or the one before
+    *s = DeepSched{};
+    s->epoch = epoch;
+    s->count = count;
+}
 __global__ void k_zero_u64(unsigned long long* p, int n) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) p[i] = 0;
 }
@@ -144,12 +173,9 @@ __global__ void k_random_boxes(int fam, unsigned long long seed, int max_label, 
     }
 }
 
-__global__ void k_single_table(double lo, double h, int n, double* t, double* v) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double x = __fma_rn((double)i, h, lo);
-        t[i] = x;
-        v[i] = single_placement(x);
-    }
+__global__ void k_single_table(double lo, double h, int n, double* v) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        v[i] = single_placement(__fma_rn((double)i, h, lo));
 }
 
 // The device-side scheduler of the graph-driven loop (one thread): commits the
@@ -241,8 +267,8 @@ __global__ void __launch_bounds__(kEvalBlock) k_ref_step(RefArgs a) {
         double lo[4], hi[4];
         if (!lattice_box(a.s, ix, a.slab_single[slab], lo, hi)) continue;
         ++evaluated;
-        const Verdict v = COLLECT ? judge_box<FAM, FULL, flt::NEED_FULL>(lo, hi, 0)
-                                  : judge_box<FAM, DECIDE, flt::NEED_VERDICT>(lo, hi, 0);
+        const Verdict v = COLLECT ? judge_box<FAM, FULL, flt::NEED_FULL>(val_ref<D>(lo, hi), 0)
+                                  : judge_box<FAM, DECIDE, flt::NEED_VERDICT>(val_ref<D>(lo, hi), 0);
         if (v.verdict == V_EMPTY) continue;
         const bool nofit = (v.mask & M_FIT) && FAM != F_START && FAM != F_START_END_2D && FAM != F_START_END_3D;
         const bool trap = (v.mask & M_TRAP) != 0;
@@ -313,7 +339,6 @@ struct cp_prover {
     unsigned long long* cnt = nullptr;  // C_COUNT counters
     unsigned long long* per_depth = nullptr;
     unsigned long long* h_cnt = nullptr;  // pinned mirror
-    double* tab_t = nullptr;
     double* tab_v = nullptr;
     int tab_n = 0;
     double tab_h = 0;
@@ -330,13 +355,20 @@ struct cp_prover {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
     unsigned long long graph_key[12] = {0};
-    int graph_variant[6][2] = {{1, 1}, {1, 1}, {1, 1}, {1, 1}, {1, 1}, {1, 1}};  // block-size variant
-    int graph_bpt[6][2] = {{2, 2}, {2, 2}, {2, 2}, {2, 2}, {2, 2}, {2, 2}};      // boxes per thread
+    // depth-first refinement (cp_refine.cuh)
+    DeepSched* deep_sched = nullptr;
+    DeepSched* h_deep = nullptr;  // pinned mirror
+    MetaList deep_list[2] = {};
+    unsigned long long* deep_flags = nullptr;  // two arrays of kParcels
+    MetaList deep_spill{};
+    int deep_dims = 0;
+    int graph_variant[6][2] = {{3, 3}, {3, 3}, {3, 3}, {3, 3}, {3, 3}, {3, 3}};  // block-size variant
+    int graph_bpt[6][2] = {{1, 1}, {1, 1}, {1, 1}, {1, 1}, {1, 1}, {1, 1}};      // boxes per thread
     // an interrupted host-driven refinement: the level stack and counters hold
     // its remaining boxes and partial counts (cp_refine_resume, checkpoints)
     bool pending = false;
     cp_refine_opts pending_opts{};
-    int variant[6][2] = {{1, 1}, {0, 0}, {1, 1}, {1, 1}, {0, 0}, {1, 1}};  // level-kernel variant per family/precision
+    int variant[6][2] = {{2, 1}, {2, 0}, {2, 1}, {2, 1}, {2, 0}, {2, 1}};  // level-kernel variant per family/precision
     // called before every lattice launch of cp_prove_family_reference
     cp_step_callback step_cb = nullptr;
     void* step_user = nullptr;
@@ -417,9 +449,10 @@ cp_status ensure_slab(cp_prover* p, int n) {
     return CP_OK;
 }
 
-SingleTable table_of(const cp_prover* p) { return SingleTable{p->tab_t, p->tab_v, p->tab_n, p->tab_h}; }
+SingleTable table_of(const cp_prover* p) { return SingleTable{p->tab_v, p->tab_n, p->tab_h, 1.0 / p->tab_h}; }
 
-using LevelKernel = void (*)(LevelArgs);
+using LevelKernel = void (*)(RefineArgs);
+using LevelEachKernel = void (*)(LevelArgs);
 // register variants of the level kernel: minimum resident blocks 1, 4, 5, 6
 constexpr int kVariants = 4;
 template <int FAM, int PREC>
@@ -446,6 +479,38 @@ LevelKernel level_kernel(int fam, int prec, int v) {
     }
 }
 
+template <int FAM>
+LevelEachKernel level_each_p(int prec) {
+    return prec ? k_level_each<FAM, 1> : k_level_each<FAM, 0>;
+}
+LevelEachKernel level_each_kernel(int fam, int prec) {
+    switch (fam) {
+    case 0: return level_each_p<0>(prec);
+    case 1: return level_each_p<1>(prec);
+    case 2: return level_each_p<2>(prec);
+    case 3: return level_each_p<3>(prec);
+    case 4: return level_each_p<4>(prec);
+    default: return level_each_p<5>(prec);
+    }
+}
+
+// Input boxes a warp takes per claim of a chunk.
+constexpr unsigned kClaim = 32;
+// Launches the level kernel over a chunk.  A warp per input box at most: the
+// boxes of a small chunk are spread over the device.
+cp_status launch_level(LevelKernel k, const LevelArgs& a, unsigned long long out_base, cudaStream_t st) {
+    k_begin_chunk<<<1, 1, 0, st>>>(a.cnt, out_base);
+    CP_TRY(cp_check_launch());
+    RefineArgs r{};
+    r.level = a;
+    r.claim = a.cnt + C_CLAIM;
+    r.per = kClaim;
+    const size_t warps = kEvalBlock / 32, need = (a.count + warps - 1) / warps;
+    const unsigned grid = (unsigned)std::min<size_t>(grid_of(k, kEvalBlock), std::max<size_t>(need, 1));
+    k<<<grid, kEvalBlock, 0, st>>>(r);
+    return cp_check_launch();
+}
+
 using RefKernel = void (*)(RefArgs);
 template <bool COLLECT>
 RefKernel ref_kernel(int fam) {
@@ -467,14 +532,14 @@ void reference_sizes(int fam, int* n) {
 // ------------------------------------------------------------------ engine pieces
 size_t cp_engine_counter_words() { return (size_t)(C_COUNT + kDepthBins); }
 
-cp_status cp_engine_launch_table(double lambda_lo, double h, int n, double* t, double* v, cudaStream_t st) {
-    k_single_table<<<64, 128, 0, st>>>(lambda_lo, h, n, t, v);
+cp_status cp_engine_launch_table(double lambda_lo, double h, int n, double* v, cudaStream_t st) {
+    k_single_table<<<64, 128, 0, st>>>(lambda_lo, h, n, v);
     return cp_check_launch();
 }
 
 cp_status cp_engine_launch_level(int fam, int prec, int variant, const BoxList& in, size_t begin, size_t count,
                                  const BoxList* out, unsigned long long out_base, unsigned long long* counters,
-                                 const double* tab_t, const double* tab_v, int tab_n, double tab_h, int policy,
+                                 const double* tab_v, int tab_n, double tab_h, int policy,
                                  int max_depth, cudaStream_t st) {
     LevelArgs a;
     a.in = in;
@@ -483,22 +548,14 @@ cp_status cp_engine_launch_level(int fam, int prec, int variant, const BoxList& 
     a.out = out ? *out : BoxList{nullptr, nullptr, nullptr, 0};
     a.cnt = counters;
     a.per_depth = counters + C_COUNT;
-    a.tab = SingleTable{tab_t, tab_v, tab_n, tab_h};
+    a.tab = SingleTable{tab_v, tab_n, tab_h, 1.0 / tab_h};
     a.policy = policy == CP_SPLIT_LEARNED ? SPLIT_GIVEN : policy;
     a.lambda_scale = kDefaultLambdaScale;
     a.max_depth = out ? max_depth : 0;
     a.axis_hint = nullptr;
     a.order_hint = nullptr;
     a.digest = 0;
-    cudaError_t e = cudaMemcpyAsync(counters + C_OUT, &out_base, sizeof(out_base), cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return cp_record_cuda_error(e, CP_ERR_CUDA);
-    LevelKernel k = level_kernel(fam, prec, variant);
-    const int block = kEvalBlock;
-    unsigned grid = grid_of(k, block);
-    const size_t need = (count + block - 1) / block;
-    if (need < grid) grid = (unsigned)std::max<size_t>(need, 1);
-    k<<<grid, block, 0, st>>>(a);
-    return cp_check_launch();
+    return launch_level(level_kernel(fam, prec, variant), a, out_base, st);
 }
 
 bool cp_engine_overflowed(const unsigned long long* h) { return (h[C_ERR] & E_OVERFLOW) != 0; }
@@ -540,18 +597,21 @@ cp_status cp_engine_eval_chunk(cp_prover* p, int fam, const cp_refine_opts& o, L
     a.order_hint = order_hint;
     a.digest = o.digest ? 1 : 0;
     // children append after the boxes already in `out`
-    unsigned long long base = out ? out->n : 0;
-    k_set_u64<<<1, 1, 0, p->stream>>>(p->cnt + C_OUT, base);
-    CP_TRY(cp_check_launch());
-    LevelKernel k = level_kernel(fam, o.precision, p->variant[fam][o.precision ? 1 : 0]);
-    const int block = kEvalBlock;
-    unsigned grid = grid_of(k, block);
-    size_t need = (count + block - 1) / block;
-    if (need < grid) grid = (unsigned)std::max<size_t>(need, 1);
+    const unsigned long long base = out ? out->n : 0;
+    const int pr = o.precision ? 1 : 0;
     cudaEventRecord(p->ev0, p->stream);
-    k<<<grid, block, 0, p->stream>>>(a);
+    if (axis_hint || order_hint || cp_model_collecting(p)) {
+        k_begin_chunk<<<1, 1, 0, p->stream>>>(p->cnt, base);
+        CP_TRY(cp_check_launch());
+        LevelEachKernel k = level_each_kernel(fam, pr);
+        const size_t need = (count + kEvalBlock - 1) / kEvalBlock;
+        const unsigned grid = (unsigned)std::min<size_t>(grid_of(k, kEvalBlock), std::max<size_t>(need, 1));
+        k<<<grid, kEvalBlock, 0, p->stream>>>(a);
+        CP_TRY(cp_check_launch());
+    } else {
+        CP_TRY(launch_level(level_kernel(fam, pr, p->variant[fam][pr]), a, base, p->stream));
+    }
     cudaEventRecord(p->ev1, p->stream);
-    CP_TRY(cp_check_launch());
     CP_TRY(read_counters(p));
     float t = 0;
     cudaEventElapsedTime(&t, p->ev0, p->ev1);
@@ -591,7 +651,7 @@ cp_status refine_levels(cp_prover* p, const cp_refine_opts& o, cp_refine_report*
         const size_t begin = in.n - c;
         uint8_t *axis = nullptr, *order = nullptr;
         if (cp_model_collecting(p))
-            CP_TRY(cp_model_collect_chunk(p, fam, in.b, begin, c, p->tab_t, p->tab_v, p->tab_n, p->tab_h));
+            CP_TRY(cp_model_collect_chunk(p, fam, in.b, begin, c, p->tab_v, p->tab_n, p->tab_h));
         if (o.policy == CP_SPLIT_LEARNED || o.learned_order) {
             // the inference launch is part of the refinement's device time
             CP_TRY(cuda_ok(cudaEventRecord(p->ev0, p->stream)));
@@ -641,13 +701,11 @@ int graph_variant_of_block(int block) {
     return -1;
 }
 
-// Builds the graph of the device-driven loop: a WHILE node whose body is
-// scheduler -> (model hints) -> persistent level kernel.
-cp_status build_graph(cp_prover* p, const cp_refine_opts& o, int variant, int bpt, bool learned_axis,
-                      bool learned_order) {
+// Builds a graph whose only node is a WHILE loop over the launches `body` makes on
+// the handle's stream (body(handle of the loop condition)).
+template <class Body>
+cp_status build_loop(cp_prover* p, Body body) {
     free_graph(p);
-    const int fam = o.family;
-    const int prec = o.precision ? 1 : 0;
     CP_TRY(cuda_ok(cudaGraphCreate(&p->graph, 0)));
     cudaGraphConditionalHandle h;
     CP_TRY(cuda_ok(cudaGraphConditionalHandleCreate(&h, p->graph, 1, cudaGraphCondAssignDefault)));
@@ -658,71 +716,9 @@ cp_status build_graph(cp_prover* p, const cp_refine_opts& o, int variant, int bp
     cp.conditional.size = 1;
     cudaGraphNode_t node;
     CP_TRY(cuda_ok(cudaGraphAddNode(&node, p->graph, nullptr, 0, &cp)));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    CP_TRY(cuda_ok(cudaStreamBeginCaptureToGraph(p->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed)));
-    cp_status st = CP_OK;
-    do {
-        k_sched<<<1, 32, 0, p->stream>>>(p->d_sched, p->cnt, h);
-        if ((st = cp_check_launch()) != CP_OK) break;
-        // with a learned policy the level kernel runs the network inline (tcgen05)
-        const bool net = learned_axis || learned_order;
-        NetArgs na{};
-        if (net) {
-            const void* views = nullptr;
-            const float* master = nullptr;
-            int limit = 0;
-            if ((st = cp_model_net_params(p, fam, &views, &master, &limit)) != CP_OK) break;
-            na.views = static_cast<const tc::bf16*>(views);
-            na.master = master;
-            na.wait_limit = limit;
-            na.want_order = learned_order ? 1 : 0;
-            na.want_axis = learned_axis ? 1 : 0;
-        }
-        PersistArgs pa;
-        pa.levels = p->d_levels;
-        pa.sched = p->d_sched;
-        pa.cnt = p->cnt;
-        pa.per_depth = p->per_depth;
-        pa.tab = table_of(p);
-        pa.policy = o.policy == CP_SPLIT_LEARNED ? SPLIT_GIVEN : o.policy;
-        pa.lambda_scale = lambda_scale_of(o);
-        pa.max_depth = o.max_depth;
-        pa.bpt = bpt;
-        pa.axis_hint = nullptr;
-        pa.order_hint = nullptr;
-        pa.digest = o.digest ? 1 : 0;
-        void* kern = net ? (prec ? cp_graph_kernel_net_fp32(fam) : cp_graph_kernel_net_fp64(fam))
-                         : (prec ? cp_graph_kernel_fp32(fam, variant) : cp_graph_kernel_fp64(fam, variant));
-        const int block = net ? kNetBlock : kGraphBlock[variant];
-        int per_sm = 0, sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
-        if (net) {
-            // The occupancy calculator reports one CTA per SM for the kernel that
-            // uses tensor memory, while the SM keeps as many resident as its
-            // registers, shared memory (about 32 KB per CTA, largest carveout)
-            // and tensor memory (tc::kNetCols columns per CTA) allow; the grid is
-            // sized from those limits.  A CTA beyond the resident ones starts when
-            // one ends (the kernel claims work dynamically), so an overestimate
-            // costs a few idle CTAs, never a wait on one another.
-            cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-            cudaFuncAttributes fa{};
-            int regs_sm = 65536, smem_sm = 0;
-            cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, p->device);
-            cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, p->device);
-            if (cudaFuncGetAttributes(&fa, kern) == cudaSuccess && fa.numRegs > 0) {
-                const int by_regs = regs_sm / (((fa.numRegs + 7) / 8 * 8) * block);
-                const int by_smem = smem_sm / ((int)fa.sharedSizeBytes + 1024);  // 1 KB reserved per CTA
-                per_sm = std::min(std::min(by_regs, by_smem), kNetMaxCtasPerSm);
-            }
-            if (per_sm < 1) per_sm = 1;
-        } else if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0) != cudaSuccess || per_sm < 1) {
-            per_sm = 1;
-        }
-        void* args[] = {&pa};
-        void* net_args[] = {&pa, &na};
-        st = cuda_ok(cudaLaunchKernel(kern, dim3((unsigned)(sms * per_sm)), dim3((unsigned)block), net ? net_args : args,
-                                      0, p->stream));
-    } while (0);
+    cudaGraph_t inner = cp.conditional.phGraph_out[0];
+    CP_TRY(cuda_ok(cudaStreamBeginCaptureToGraph(p->stream, inner, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed)));
+    const cp_status st = body(h);
     cudaGraph_t captured = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(p->stream, &captured);
     if (st != CP_OK) return st;
@@ -730,56 +726,106 @@ cp_status build_graph(cp_prover* p, const cp_refine_opts& o, int variant, int bp
     return cuda_ok(cudaGraphInstantiate(&p->graph_exec, p->graph, 0));
 }
 
-// The level-stack loop of refine_levels, run on the device by one CUDA graph
-// launch: no host round trip between chunks.
-cp_status refine_graph(cp_prover* p, const cp_refine_opts& o, cp_refine_report* r, double t_wall0) {
+int sm_count(int device) {
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    return sms;
+}
+
+// The level-stack loop with a learned policy: scheduler, then the persistent level
+// kernel with the network inline (tcgen05).
+cp_status build_net_graph(cp_prover* p, const cp_refine_opts& o, bool learned_axis, bool learned_order) {
+    const int fam = o.family;
+    const int prec = o.precision ? 1 : 0;
+    NetArgs na{};
+    const void* views = nullptr;
+    const float* master = nullptr;
+    int limit = 0;
+    CP_TRY(cp_model_net_params(p, fam, &views, &master, &limit));
+    na.views = static_cast<const tc::bf16*>(views);
+    na.master = master;
+    na.wait_limit = limit;
+    na.want_order = learned_order ? 1 : 0;
+    na.want_axis = learned_axis ? 1 : 0;
+    PersistArgs pa;
+    pa.levels = p->d_levels;
+    pa.sched = p->d_sched;
+    pa.cnt = p->cnt;
+    pa.per_depth = p->per_depth;
+    pa.tab = table_of(p);
+    pa.policy = o.policy == CP_SPLIT_LEARNED ? SPLIT_GIVEN : o.policy;
+    pa.lambda_scale = lambda_scale_of(o);
+    pa.max_depth = o.max_depth;
+    pa.digest = o.digest ? 1 : 0;
+    void* kern = prec ? cp_graph_kernel_net_fp32(fam) : cp_graph_kernel_net_fp64(fam);
+    // The occupancy calculator reports one CTA per SM for the kernel that
+    // uses tensor memory, while the SM keeps as many resident as its
+    // registers, shared memory (about 32 KB per CTA, largest carveout)
+    // and tensor memory (tc::kNetCols columns per CTA) allow; the grid is
+    // sized from those limits.  A CTA beyond the resident ones starts when
+    // one ends (the kernel claims work dynamically), so an overestimate
+    // costs a few idle CTAs, never a wait on one another.
+    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaFuncAttributes fa{};
+    int per_sm = 0, regs_sm = 65536, smem_sm = 0;
+    cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, p->device);
+    cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, p->device);
+    if (cudaFuncGetAttributes(&fa, kern) == cudaSuccess && fa.numRegs > 0) {
+        const int by_regs = regs_sm / (((fa.numRegs + 7) / 8 * 8) * kNetBlock);
+        const int by_smem = smem_sm / ((int)fa.sharedSizeBytes + 1024);  // 1 KB reserved per CTA
+        per_sm = std::min(std::min(by_regs, by_smem), kNetMaxCtasPerSm);
+    }
+    if (per_sm < 1) per_sm = 1;
+    return build_loop(p, [&](cudaGraphConditionalHandle h) -> cp_status {
+        k_sched<<<1, 32, 0, p->stream>>>(p->d_sched, p->cnt, h);
+        CP_TRY(cp_check_launch());
+        void* args[] = {&pa, &na};
+        return cuda_ok(cudaLaunchKernel(kern, dim3((unsigned)(sm_count(p->device) * per_sm)), dim3(kNetBlock), args, 0,
+                                        p->stream));
+    });
+}
+
+// The level-stack loop of refine_levels with the network inline, run on the
+// device by one CUDA graph launch: no host round trip between chunks.
+cp_status refine_net_graph(cp_prover* p, const cp_refine_opts& o, cp_refine_report* r, double t_wall0) {
     const int fam = o.family;
     const int D = family_dims(fam);
-    const int prec = o.precision ? 1 : 0;
     const int nlevels = (int)p->levels.size();
     if (nlevels > kMaxLevels) return cp_fail(CP_ERR_INVALID, "graph engine: max_depth must be < %d", kMaxLevels);
-    int variant = o.block > 0 ? graph_variant_of_block(o.block) : p->graph_variant[fam][prec];
-    if (variant < 0) return cp_fail(CP_ERR_INVALID, "graph engine: block must be 64, 128, 256, 512 or 1024");
-    const int bpt = o.boxes_per_thread > 0 ? o.boxes_per_thread : p->graph_bpt[fam][prec];
-    if (bpt > 8) return cp_fail(CP_ERR_INVALID, "graph engine: boxes_per_thread must be 1..8");
     const bool learned_axis = o.policy == CP_SPLIT_LEARNED, learned_order = o.learned_order != 0;
     if (!p->d_levels) {
         CP_TRY(cuda_ok(cudaMalloc(&p->d_levels, sizeof(BoxList) * kMaxLevels)));
         CP_TRY(cuda_ok(cudaMalloc(&p->d_sched, sizeof(DevSched))));
         CP_TRY(cuda_ok(cudaMallocHost(&p->h_sched, sizeof(DevSched))));
     }
-    BoxList hl[kMaxLevels];
-    for (int l = 0; l < nlevels; ++l) hl[l] = p->levels[l].b;
-    DevSched& hs = *p->h_sched;
-    std::memset(&hs, 0, sizeof(hs));
-    for (int l = 0; l < nlevels; ++l) hs.n[l] = p->levels[l].n;
-    hs.cap = p->level_cap;
-    hs.nlevels = nlevels;
-    hs.max_depth = o.max_depth;
-    hs.fanout = fanout(o.policy == CP_SPLIT_LEARNED ? SPLIT_GIVEN : o.policy, D);
     {
         // the level table and the schedule travel as kernel parameters: a copy
         // would queue behind a large host-to-device copy of staged seeds on the
         // copy engine and delay the refinement
         GraphUpload u;
-        for (int l = 0; l < nlevels; ++l) u.levels[l] = hl[l];
-        u.sched = hs;
+        std::memset(&u.sched, 0, sizeof(u.sched));
+        for (int l = 0; l < nlevels; ++l) {
+            u.levels[l] = p->levels[l].b;
+            u.sched.n[l] = p->levels[l].n;
+        }
+        u.sched.cap = p->level_cap;
+        u.sched.nlevels = nlevels;
+        u.sched.max_depth = o.max_depth;
+        u.sched.fanout = fanout(o.policy == CP_SPLIT_LEARNED ? SPLIT_GIVEN : o.policy, D);
         u.nlevels = nlevels;
         k_graph_upload<<<1, 64, 0, p->stream>>>(u, p->d_levels, p->d_sched);
         CP_TRY(cp_check_launch());
     }
-    double ls = lambda_scale_of(o);
+    const double scale = lambda_scale_of(o);
     unsigned long long ls_bits;
-    std::memcpy(&ls_bits, &ls, 8);
-    const unsigned long long key[12] = {ls_bits, (unsigned long long)fam + 1, (unsigned long long)prec, (unsigned long long)variant,
-                                        (unsigned long long)bpt, (unsigned long long)o.policy,
-                                        (unsigned long long)o.max_depth,
+    std::memcpy(&ls_bits, &scale, 8);
+    const unsigned long long key[12] = {ls_bits, (unsigned long long)fam + 1, (unsigned long long)(o.precision ? 1 : 0),
+                                        1ull, (unsigned long long)o.policy, (unsigned long long)o.max_depth,
                                         (unsigned long long)(learned_axis | (learned_order << 1) | (o.digest ? 4 : 0)),
                                         (unsigned long long)(uintptr_t)p->levels[0].b.lo, (unsigned long long)p->level_cap,
-                                        (unsigned long long)nlevels,
-                                        (unsigned long long)(uintptr_t)p->model};
+                                        (unsigned long long)nlevels, (unsigned long long)(uintptr_t)p->model, 0ull};
     if (!p->graph_exec || std::memcmp(key, p->graph_key, sizeof(key)) != 0) {
-        CP_TRY(build_graph(p, o, variant, bpt, learned_axis, learned_order));
+        CP_TRY(build_net_graph(p, o, learned_axis, learned_order));
         std::memcpy(p->graph_key, key, sizeof(key));
     }
     CP_TRY(cuda_ok(cudaEventRecord(p->ev0, p->stream)));
@@ -800,6 +846,123 @@ cp_status refine_graph(cp_prover* p, const cp_refine_opts& o, cp_refine_report* 
     r->device_ms = t;
     r->wall_ms = now_ms() - t_wall0;
     return CP_OK;
+}
+
+void free_meta(MetaList* l) {
+    cudaFree(l->lo);
+    cudaFree(l->hi);
+    cudaFree(l->meta);
+    *l = MetaList{};
+}
+void free_deep(cp_prover* p) {
+    free_meta(&p->deep_list[0]);
+    free_meta(&p->deep_list[1]);
+    free_meta(&p->deep_spill);
+    cudaFree(p->deep_flags);
+    p->deep_flags = nullptr;
+    p->deep_dims = 0;
+}
+
+cp_status alloc_meta(MetaList* l, int dims, size_t cap) {
+    CP_TRY(cuda_ok(cudaMalloc(&l->lo, sizeof(double) * dims * cap)));
+    CP_TRY(cuda_ok(cudaMalloc(&l->hi, sizeof(double) * dims * cap)));
+    CP_TRY(cuda_ok(cudaMalloc(&l->meta, sizeof(uint32_t) * cap)));
+    l->cap = cap;
+    return CP_OK;
+}
+
+// Lists of a depth-first refinement: the parcels, and what every warp spills.
+cp_status ensure_deep(cp_prover* p, int dims, size_t spill_cap) {
+    if (!p->deep_sched) {
+        CP_TRY(cuda_ok(cudaMalloc(&p->deep_sched, sizeof(DeepSched))));
+        CP_TRY(cuda_ok(cudaMallocHost(&p->h_deep, sizeof(DeepSched))));
+        CP_TRY(cuda_ok(cudaMemsetAsync(p->deep_sched, 0, sizeof(DeepSched), p->stream)));
+    }
+    if (p->deep_dims >= dims && p->deep_spill.cap >= spill_cap) return CP_OK;
+    dims = std::max(dims, p->deep_dims);
+    spill_cap = std::max(spill_cap, p->deep_spill.cap);
+    free_deep(p);
+    CP_TRY(alloc_meta(&p->deep_spill, dims, spill_cap));
+    CP_TRY(alloc_meta(&p->deep_list[0], dims, (size_t)kParcels * 32));
+    CP_TRY(alloc_meta(&p->deep_list[1], dims, (size_t)kParcels * 32));
+    CP_TRY(cuda_ok(cudaMalloc(&p->deep_flags, 2 * sizeof(unsigned long long) * kParcels)));
+    CP_TRY(cuda_ok(cudaMemsetAsync(p->deep_flags, 0, 2 * sizeof(unsigned long long) * kParcels, p->stream)));
+    p->deep_dims = dims;
+    return CP_OK;
+}
+
+// The whole refinement as one launch of the depth-first kernel.
+cp_status refine_graph(cp_prover* p, const cp_refine_opts& o, cp_refine_report* r, double t_wall0) {
+    const int fam = o.family;
+    const int D = family_dims(fam);
+    const int prec = o.precision ? 1 : 0;
+    if (o.max_depth + 1 > kMaxLevels)
+        return cp_fail(CP_ERR_INVALID, "graph engine: max_depth must be < %d", kMaxLevels);
+    const int variant = o.block > 0 ? graph_variant_of_block(o.block) : p->graph_variant[fam][prec];
+    if (variant < 0) return cp_fail(CP_ERR_INVALID, "graph engine: block must be 64, 128, 256, 512 or 1024");
+    const int bpt = o.boxes_per_thread > 0 ? o.boxes_per_thread : p->graph_bpt[fam][prec];
+    if (bpt > 8) return cp_fail(CP_ERR_INVALID, "graph engine: boxes_per_thread must be 1..8");
+    if (o.policy == CP_SPLIT_LEARNED || o.learned_order) return refine_net_graph(p, o, r, t_wall0);
+    const size_t n = p->levels[0].n;
+    // (the contract of level_capacity: a level holds at least one box's children)
+    if (n && o.max_depth > 0 && p->level_cap < (size_t)fanout(o.policy, D))
+        return cp_fail(CP_ERR_CAPACITY, "graph engine: worklist level capacity exceeded");
+    const DeepKernel k = prec ? cp_deep_kernel_fp32(fam, variant) : cp_deep_kernel_fp64(fam, variant);
+    CP_TRY(cuda_ok(cudaFuncSetAttribute(k.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem)));
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.kernel, k.threads, k.smem) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
+    const unsigned grid = (unsigned)(sm_count(p->device) * per_sm);
+    const size_t warps = (size_t)grid * (k.threads / 32);
+    RefineArgs a{};
+    // a warp works strictly from 512 spilled parents on; then the stack's bound, and what
+    // the buffers on chip add (cp_refine.cuh)
+    a.strict = 512;
+    a.seg = a.strict + 32 * (size_t)(o.max_depth + 1) + 2 * (kParents + kReady);
+    a.per = 32u * (unsigned)bpt;
+    CP_TRY(ensure_deep(p, D, warps * a.seg));
+    a.level.in = p->levels[0].b;
+    a.level.cnt = p->cnt;
+    a.level.per_depth = p->per_depth;
+    a.level.tab = table_of(p);
+    a.level.policy = o.policy;
+    a.level.max_depth = o.max_depth;
+    a.level.lambda_scale = lambda_scale_of(o);
+    a.level.digest = o.digest ? 1 : 0;
+    a.sched = p->deep_sched;
+    a.lists[0] = p->deep_list[0];
+    a.lists[1] = p->deep_list[1];
+    a.flags[0] = p->deep_flags;
+    a.flags[1] = p->deep_flags + kParcels;
+    a.spill = p->deep_spill;
+    k_begin_deep<<<1, 1, 0, p->stream>>>(p->deep_sched, (unsigned long long)n);
+    CP_TRY(cp_check_launch());
+    CP_TRY(cuda_ok(cudaEventRecord(p->ev0, p->stream)));
+    do {  // (hardly ever more than one round)
+        void* args[] = {&a};
+        CP_TRY(cuda_ok(cudaLaunchKernel(k.kernel, dim3(grid), dim3((unsigned)k.threads), args, (size_t)k.smem,
+                                        p->stream)));
+        CP_TRY(cuda_ok(cudaEventRecord(p->ev1, p->stream)));
+        CP_TRY(cuda_ok(cudaMemcpyAsync(p->h_deep, p->deep_sched, sizeof(DeepSched), cudaMemcpyDeviceToHost, p->stream)));
+        CP_TRY(read_counters(p));
+    } while (p->h_deep->left != 0 && p->h_deep->status == 0);
+    float t = 0;
+    cudaEventElapsedTime(&t, p->ev0, p->ev1);
+    p->levels[0].n = 0;
+    if (p->h_deep->status != 0)
+        return cp_fail(CP_ERR_DEVICE, "graph engine: depth-first kernel stopped (status %d)", p->h_deep->status);
+    cp_engine_fill_report(p->h_cnt, r);
+    r->launches = (int32_t)p->h_deep->rounds;
+    r->device_ms = t;
+    r->wall_ms = now_ms() - t_wall0;
+    return CP_OK;
+}
+
+// Levels a refinement keeps in memory: the depth-first kernel only its seeds.
+int levels_of(cp_prover* p, const cp_refine_opts& o) {
+    const bool deep = o.engine == CP_ENGINE_GRAPH && o.policy != CP_SPLIT_LEARNED && !o.learned_order &&
+                      !cp_model_collecting(p);
+    return deep ? 1 : o.max_depth + 1;
 }
 
 cp_status run_refinement(cp_prover* p, const cp_refine_opts& o, cp_refine_report* r, double t0) {
@@ -862,9 +1025,8 @@ cp_status cp_create(int device, cp_prover** out) {
         // single-placement table on 2^16 lambda points over [0.5, 0.99]
         p->tab_n = 1 << 16;
         p->tab_h = (kLambdaMax - kLambdaMin) / (p->tab_n - 1);
-        if ((s = cuda_ok(cudaMalloc(&p->tab_t, sizeof(double) * p->tab_n))) != CP_OK) break;
         if ((s = cuda_ok(cudaMalloc(&p->tab_v, sizeof(double) * p->tab_n))) != CP_OK) break;
-        k_single_table<<<256, 128, 0, p->stream>>>(kLambdaMin, p->tab_h, p->tab_n, p->tab_t, p->tab_v);
+        k_single_table<<<256, 128, 0, p->stream>>>(kLambdaMin, p->tab_h, p->tab_n, p->tab_v);
         if ((s = cp_check_launch()) != CP_OK) break;
         if ((s = cuda_ok(cudaStreamSynchronize(p->stream))) != CP_OK) break;
     } while (0);
@@ -885,10 +1047,12 @@ void cp_destroy(cp_prover* p) {
     cudaFree(p->d_levels);
     cudaFree(p->d_sched);
     cudaFreeHost(p->h_sched);
+    free_deep(p);
+    cudaFree(p->deep_sched);
+    cudaFreeHost(p->h_deep);
     free_levels(p);
     cudaFree(p->cnt);
     cudaFreeHost(p->h_cnt);
-    cudaFree(p->tab_t);
     cudaFree(p->tab_v);
     cudaFree(p->slab_single);
     if (p->ev0) cudaEventDestroy(p->ev0);
@@ -953,7 +1117,7 @@ __attribute__((visibility("hidden"))) cp_status cp_refine_keep_interrupt(cp_prov
     total = lattice_total > part ? (lattice_total - part + parts - 1) / parts : 0;
     const size_t cap = o->level_capacity > 0 ? (size_t)o->level_capacity : ((size_t)1 << 25);
     if (total > cap) return CP_ERR_CAPACITY;
-    CP_TRY(ensure_levels(p, o->max_depth + 1, D, cap));
+    CP_TRY(ensure_levels(p, levels_of(p, *o), D, cap));
     for (auto& L : p->levels) L.n = 0;
     CP_TRY(ensure_slab(p, s.n[0]));
     CP_TRY(cp_launch_slab_single(s, p->slab_single, p->stream));
@@ -1164,7 +1328,7 @@ cp_status cp_refine_boxes(cp_prover* p, const cp_refine_opts* o, const double* l
     const int D = family_dims(o->family);
     const size_t cap = o->level_capacity > 0 ? (size_t)o->level_capacity : ((size_t)1 << 25);
     if (n > cap) return CP_ERR_CAPACITY;
-    CP_TRY(ensure_levels(p, o->max_depth + 1, D, cap));
+    CP_TRY(ensure_levels(p, levels_of(p, *o), D, cap));
     for (auto& L : p->levels) L.n = 0;
     if (n) {
         k_copy_seed<<<grid_of(k_copy_seed, 128), 128, 0, p->stream>>>(D, lo, hi, depth, n, p->levels[0].b);
@@ -1189,7 +1353,7 @@ cp_status cp_refine_boxes_host(cp_prover* p, const cp_refine_opts* o, const doub
     const int D = family_dims(o->family);
     const size_t cap = o->level_capacity > 0 ? (size_t)o->level_capacity : ((size_t)1 << 25);
     if (n > cap) return CP_ERR_CAPACITY;
-    CP_TRY(ensure_levels(p, o->max_depth + 1, D, cap));
+    CP_TRY(ensure_levels(p, levels_of(p, *o), D, cap));
     for (auto& L : p->levels) L.n = 0;
     BoxList& b = p->levels[0].b;
     for (int d = 0; d < D && n; ++d) {
@@ -1254,7 +1418,7 @@ cp_status cp_refine_staged(cp_prover* p, const cp_refine_opts* o, int slot, cp_r
     const size_t n = st.n;
     const size_t cap = o->level_capacity > 0 ? (size_t)o->level_capacity : ((size_t)1 << 25);
     if (n > cap) return CP_ERR_CAPACITY;
-    CP_TRY(ensure_levels(p, o->max_depth + 1, D, cap));
+    CP_TRY(ensure_levels(p, levels_of(p, *o), D, cap));
     for (auto& L : p->levels) L.n = 0;
     // the refinement's stream waits for the slot's copy, then moves the boxes
     // into the level stack (device to device)

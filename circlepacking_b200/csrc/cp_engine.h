@@ -22,11 +22,15 @@ void cp_model_free(cp_prover* p);
 // before the engine evaluates it; a no-op unless a collection is running.
 bool cp_model_collecting(cp_prover* p);
 cp_status cp_model_collect_chunk(cp_prover* p, int fam, const cpb::BoxList& in, size_t begin, size_t count,
-                                 const double* tab_t, const double* tab_v, int tab_n, double tab_h);
+                                 const double* tab_v, int tab_n, double tab_h);
 
-// Persistent level kernels of the graph engine (cp_graph_fp64.cu / cp_graph_fp32.cu).
-void* cp_graph_kernel_fp64(int fam, int variant);
-void* cp_graph_kernel_fp32(int fam, int variant);
+// Depth-first kernels of the graph engine (cp_graph_fp64.cu / cp_graph_fp32.cu).
+struct DeepKernel {
+    void* kernel;
+    int threads, smem;  // threads per block, dynamic shared memory
+};
+DeepKernel cp_deep_kernel_fp64(int fam, int variant);
+DeepKernel cp_deep_kernel_fp32(int fam, int variant);
 // Persistent level kernels that run the proposal network inline (128 threads).
 void* cp_graph_kernel_net_fp64(int fam);
 void* cp_graph_kernel_net_fp32(int fam);
@@ -38,10 +42,10 @@ cp_status cp_model_net_params(cp_prover* p, int fam, const void** views, const f
 // Pieces of the refinement engine reused by the static-scratch entry point
 // (cp_noalloc.cu).  Counters: cp_engine_counter_words() 64-bit words.
 size_t cp_engine_counter_words();
-cp_status cp_engine_launch_table(double lambda_lo, double h, int n, double* t, double* v, cudaStream_t st);
+cp_status cp_engine_launch_table(double lambda_lo, double h, int n, double* v, cudaStream_t st);
 cp_status cp_engine_launch_level(int fam, int prec, int variant, const cpb::BoxList& in, size_t begin, size_t count,
                                  const cpb::BoxList* out, unsigned long long out_base, unsigned long long* counters,
-                                 const double* tab_t, const double* tab_v, int tab_n, double tab_h, int policy,
+                                 const double* tab_v, int tab_n, double tab_h, int policy,
                                  int max_depth, cudaStream_t st);
 // Reads the overflow flag and children count of a counter block copied to the host.
 bool cp_engine_overflowed(const unsigned long long* h_counters);

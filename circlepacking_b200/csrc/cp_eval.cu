@@ -28,15 +28,17 @@ __global__ void __launch_bounds__(kEvalBlock) k_eval_fp64(const double* __restri
     constexpr int D = family_dims(FAM);
     const size_t step = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
-        double l[4], h[4];
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-            l[d] = __ldg(lo + d * stride + i);
-            h[d] = __ldg(hi + d * stride + i);
-        }
         const int ord = order ? order[i] : 0;
+        double l[4], h[4];
+        if (TRACE) {
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                l[d] = __ldg(lo + d * stride + i);
+                h[d] = __ldg(hi + d * stride + i);
+            }
+        }
         const Verdict v = TRACE ? eval_box<FAM, MODE>(l, h, ord, trace + 16 * i)
-                                : judge_box<FAM, MODE, need_of(MODE)>(l, h, ord);
+                                : judge_box<FAM, MODE, need_of(MODE)>(BoxRef<D>{lo + i, hi + i, stride}, ord);
         verdict[i] = v.verdict;
         mask[i] = v.mask;
     }
@@ -64,7 +66,7 @@ __global__ void __launch_bounds__(kEvalBlock) k_eval_prefilter(const double* __r
         const int pre = prefilter_box<FAM>(l, h, ord, MODE == FULL, &pmask);
         Verdict v;
         if (pre == PF_UNDECIDED)
-            v = TRACE ? eval_box<FAM, MODE>(l, h, ord, trace + 16 * i) : judge_box<FAM, MODE, need_of(MODE)>(l, h, ord);
+            v = TRACE ? eval_box<FAM, MODE>(l, h, ord, trace + 16 * i) : judge_box<FAM, MODE, need_of(MODE)>(BoxRef<D>{lo + i, hi + i, stride}, ord);
         else
             v = {pre == PF_PROVED ? V_PROVED : pre == PF_EMPTY ? V_EMPTY : pre == PF_NOFIT ? V_NOFIT : V_CRITICAL,
                  pmask};

@@ -394,34 +394,71 @@ __device__ __noinline__ uint32_t eval_box_call(double l0, double h0, double l1, 
     return (uint32_t)v.verdict | ((uint32_t)v.mask << 8) | ((uint32_t)v.handles << 16);
 }
 
+// A box in memory, lo axis d at lo[d * stride] and hi likewise (flt::ValRef).
+template <int D>
+struct BoxRef {
+    const double* lo;
+    const double* hi;
+    size_t stride;
+    __device__ __forceinline__ flt::FBox load() const {
+        asm volatile("" ::: "memory");
+        flt::FBox b{lo[0], hi[0], lo[stride], hi[stride], lo[2 * stride], hi[2 * stride], 0.0, 0.0};
+        if (D == 4) {
+            b.l3 = lo[3 * stride];
+            b.h3 = hi[3 * stride];
+        }
+        flt::tighten(b, D == 4);
+        return b;
+    }
+};
+
 // eval_box without a trace, through the FP64 filter: the same verdict, with the
-// part of mask and handles that NEED asks for (flt::Need).
-template <int FAM, int MODE, int NEED>
-__device__ __forceinline__ Verdict judge_box(const double* lo, const double* hi, int order) {
+// part of mask and handles that NEED asks for (flt::Need).  In two steps, so that a
+// warp can come together in between: judge_fast returns false for the boxes the
+// filter leaves, judge_slow evaluates those.
+template <int FAM, int MODE, int NEED, class Ref>
+__device__ __forceinline__ bool judge_fast(const Ref& ref, int order, Verdict& v) {
     constexpr int D = family_dims(FAM);
     constexpr bool kFitStops = FAM != F_START && FAM != F_START_END_2D && FAM != F_START_END_3D;
-    flt::FBox b{lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], 0.0, 0.0};
-    bool empty = b.ll > b.lh || b.l2 > b.h2;
-    if (D == 4) {
-        b.l3 = lo[3];
-        b.h3 = hi[3];
-        if (b.l2 < b.l3) b.l2 = b.l3;
-        empty = empty || b.l3 > b.h3 || b.l2 > b.h2;
-    }
-    if (b.l1 < b.l2) b.l1 = b.l2;
-    if (empty || b.l1 > b.h1) return {V_EMPTY, 0, 0};
-    const bool fit_fires = FAM != F_START_END_2D && FAM != F_START_END_3D &&
+    uint8_t fit = 0;
+    {
+        const flt::FBox b = ref.load();
+        if (b.ll > b.lh || b.l1 > b.h1 || b.l2 > b.h2 || (D == 4 && b.l3 > b.h3)) {
+            v = {V_EMPTY, 0, 0};
+            return true;
+        }
+        const bool fires = FAM != F_START_END_2D && FAM != F_START_END_3D &&
                            __dmul_ru(2.0, b.h1) >= __dadd_rd(1.0, -b.lh);
-    const uint8_t fit = fit_fires ? (uint8_t)M_FIT : (uint8_t)0;
-    if (MODE == DECIDE && kFitStops && fit_fires) return {V_NOFIT, fit, 0};
-    flt::FOut o;
-    if (flt::filter_box<FAM, NEED>(b, order, o)) {
-        const uint8_t v = kFitStops && fit_fires ? V_NOFIT : o.mask ? V_CRITICAL : V_PROVED;
-        return {v, (uint8_t)(fit | o.mask), o.handles};
+        if (fires) fit = (uint8_t)M_FIT;
+        if (MODE == DECIDE && kFitStops && fires) {
+            v = {V_NOFIT, fit, 0};
+            return true;
+        }
     }
-    const uint32_t r = eval_box_call<FAM, MODE>(lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], D == 4 ? lo[3] : 0.0,
-                                                D == 4 ? hi[3] : 0.0, order);
+    flt::FOut o{0, 0};
+    const bool decided = flt::filter_box<FAM, NEED>(ref, order, o);
+    v = {(uint8_t)(kFitStops && fit ? V_NOFIT : o.mask ? V_CRITICAL : V_PROVED), (uint8_t)(fit | o.mask), o.handles};
+    return decided;
+}
+template <int FAM, int MODE, class Ref>
+__device__ __forceinline__ Verdict judge_slow(const Ref& ref, int order) {
+    const flt::FBox b = ref.load();  // (tightened: eval_box's own tightening changes nothing)
+    const uint32_t r = eval_box_call<FAM, MODE>(b.ll, b.lh, b.l1, b.h1, b.l2, b.h2, b.l3, b.h3, order);
     return {(uint8_t)r, (uint8_t)(r >> 8), (uint8_t)(r >> 16)};
+}
+template <int FAM, int MODE, int NEED, class Ref>
+__device__ __forceinline__ Verdict judge_box(const Ref& ref, int order) {
+    Verdict v;
+    if (!judge_fast<FAM, MODE, NEED>(ref, order, v)) v = judge_slow<FAM, MODE>(ref, order);
+    return v;
+}
+
+// A box in registers, for judge_box.
+template <int D>
+__device__ __forceinline__ flt::ValRef val_ref(const double* lo, const double* hi) {
+    flt::FBox b{lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], D == 4 ? lo[3] : 0.0, D == 4 ? hi[3] : 0.0};
+    flt::tighten(b, D == 4);
+    return {b};
 }
 
 }  // namespace cpb

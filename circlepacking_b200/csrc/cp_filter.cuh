@@ -43,13 +43,11 @@
 #include <cstdint>
 
 #ifdef __CUDACC__
-#include "cp_fp64.cuh"
 #define CPF_HD __host__ __device__ __forceinline__
 #else
-#include <cmath>
-#include <cstring>
 #define CPF_HD inline
 #endif
+#include <cmath>
 
 namespace cpb {
 namespace flt {
@@ -81,7 +79,7 @@ CPF_HD double fma_(double a, double b, double c) {
     return std::fma(a, b, c);
 #endif
 }
-CPF_HD double abs_(double x) { return x < 0.0 ? -x : x; }
+CPF_HD double abs_(double x) { return fabs(x); }
 // seeds of 1/d and 1/sqrt(d): the FP64 approximations, within 2^-19 (host: rounded to float)
 CPF_HD double rcp_seed_(double d) {
 #ifdef __CUDA_ARCH__
@@ -109,7 +107,7 @@ CPF_HD double rsqrt_(double d) {
     const double y = rsqrt_seed_(d);
     return fma_(0.5 * y, fma_(-d * y, y, 1.0), y);
 }
-// RD(x + y) doubled and RU(x - y): the side-by-side test of the mixed angles is exact
+// RD(x + y) and RU(x + y), for the comparisons that are exact
 CPF_HD double add_rd_(double x, double y) {
 #ifdef __CUDA_ARCH__
     return __dadd_rd(x, y);
@@ -119,6 +117,23 @@ CPF_HD double add_rd_(double x, double y) {
 #endif
 }
 CPF_HD double add_ru_(double x, double y) { return -add_rd_(-x, -y); }
+CPF_HD double mul_rd_(double x, double y) {
+#ifdef __CUDA_ARCH__
+    return __dmul_rd(x, y);
+#else
+    const double p = x * y;
+    return fma_(x, y, -p) < 0.0 ? std::nextafter(p, -4.0) : p;
+#endif
+}
+CPF_HD double mul_ru_(double x, double y) { return -mul_rd_(-x, y); }
+// the next double above a positive x
+CPF_HD double above_(double x) {
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double(__double_as_longlong(x) + 1);
+#else
+    return std::nextafter(x, 1e300);
+#endif
+}
 
 // asin(x) = x + x z P(z), z = x^2, |x| <= 1/2: minimax polynomial (Remez exchange
 // on z in [0, 1/4], relative error 9.8e-13).
@@ -134,77 +149,74 @@ CPF_HD double asin_core(double x, double z) {
     return fma_(x * z, p, x);
 }
 // asin(n / d) for |n| <= d, r = 1/d: beyond 1/2 from 1 - |n|/d = (d - |n|) r.
-// ok: the quotient keeps kEnd away from 1.
-CPF_HD double asin_quot(double n, double d, double r, bool& ok) {
-    const double an = abs_(n);
-    const double x = an * r, y = (d - an) * r;
-    ok = ok && y >= kEnd;
-    double v;
-    if (y < 0.5) {
-        const double z = 0.5 * y;
-        v = fma_(-2.0, asin_core(z * rsqrt_(z), z), kHalfPi);
-    } else {
-        v = asin_core(x, x * x);
+// ok: the quotient keeps kEnd away from 1.  One polynomial for both ranges, so that
+// lanes on either side of 1/2 share it.
+CPF_HD double asin_pos(double n, double d, double r, bool& ok) {
+    const double x = n * r;
+    const bool far = n + n > d;
+    double s = x, z = x * x;
+    if (far) {
+        z = (0.5 * r) * (d - n);
+        ok = ok && z >= 0.5 * kEnd;
+        s = z * rsqrt_(z);
     }
-    return n < 0.0 ? -v : v;
+    const double p = asin_core(s, z);
+    return far ? fma_(-2.0, p, kHalfPi) : p;
+}
+CPF_HD double asin_quot(double n, double d, double r, bool& ok) {
+    return copysign(asin_pos(abs_(n), d, r, ok), n);
 }
 
 // ------------------------------------------------------------------ collision angles
 // Disks of radii ro (touching the outer border, centre distance P = 1 - ro) and
-// ri (touching the inner one, Q = lambda + ri, an interval through lambda), upper
-// corner.  The longer of P and Q is the side L; where P lies inside Q both orders
-// are taken, each tightened to L >= S (collision_angles.cu:144-158 and 37-57).
-// With c = ro + ri, the wanted bound is asin((Lh^2 - Sl^2 + c^2) / (2 c Ll)) minus
-// asin((Ll^2 - Sh^2 - c^2) / (2 c S)), S = Sh where the angle at S is obtuse, else
-// Sl: the obtuse and acute formulas (collision_angles.cu:59-117) agree at their
-// boundary, so a comparison near it needs no care.
+// ri (touching the inner one, Q = lambda + ri, an interval [ql, qh] through lambda),
+// upper corner, c = ro + ri.  The longer side is L = P, the shorter S = Q; where P
+// lies below qh the reference takes the other order too (collision_angles.cu:144-158),
+// the radii then nearly add up to the lane width: about 1 in 500 boxes of a coarse
+// lattice, fewer of a finer one, left to eval_box.
+// The wanted bound is asin((P^2 - ql^2 + c^2) / (2 c P)) minus asin((P^2 - qh^2 - c^2)
+// / (2 c S)), S = qh where the angle at S is obtuse, else ql: the obtuse and acute
+// formulas (collision_angles.cu:59-117) agree at their boundary, so a comparison near
+// it needs no care.
 // Trap sites: the first quotient exceeds 1 only when 2 c <= 1 - lambda.lo (to
 // rounding), where the directed value is clamped if the angle is definitely obtuse
-// and a trap otherwise.  The second exceeds 1 only beyond Sh + c < Ll.
-CPF_HD double mixed_hi_order(double Ll, double Lh, double Sl, double Sh, double c, bool& ok) {
-    const double c2 = c * c, cc = c + c;
-    const double al = fma_(Ll, Ll, -(Sh * Sh)), ah = fma_(Lh, Lh, -(Sl * Sl));
-    const double n1 = ah + c2, n2 = al - c2;
-    const double d1 = cc * Ll, d2 = cc * (n2 > 0.0 ? Sh : Sl);
+// and a trap otherwise.  The second exceeds 1 only beyond qh + c < P.
+CPF_HD double mixed_hi(double ll, double lh, double ro, double ri, bool& ok) {
+    const double P = 1.0 - ro, ql = ll + ri, qh = lh + ri, c = ro + ri;
+    const double c2 = c * c, cc = c + c, P2 = P * P;
+    const double n1 = fma_(-ql, ql, P2 + c2), n2 = fma_(-qh, qh, P2 - c2);
+    const double d1 = cc * P, d2 = cc * (n2 > 0.0 ? qh : ql);
     const double r = rcp_(d1 * d2);
+    ok = ok && qh <= P;
     double v1;
     if (n1 > d1) {  // clamped to 1: definitely obtuse, clear of 1, lower quotient inside
-        const double d3 = cc * Lh;
-        ok = ok && n2 > kTie && (n1 - d1) >= kEnd * d1 && (d3 - (al + c2)) >= kEnd * d3;
+        ok = ok && n2 > kTie && n1 - d1 >= kEnd * d1 && d1 - (n2 + 2.0 * c2) >= kEnd * d1;
         v1 = kHalfPi;
     } else {
-        v1 = asin_quot(n1, d1, r * d2, ok);
+        v1 = asin_pos(n1, d1, r * d2, ok);
     }
     return v1 - asin_quot(n2, d2, r * d1, ok);
 }
-CPF_HD double mixed_hi(double ll, double lh, double ro, double ri, bool& ok) {
-    const double P = 1.0 - ro, ql = ll + ri, qh = lh + ri, c = ro + ri;
-    const bool x = ql <= P;
-    double v = mixed_hi_order(x ? P : ql, x ? P : qh, x ? ql : P, x ? (qh < P ? qh : P) : P, c, ok);
-    if (x && qh > P) {
-        const double w = mixed_hi_order(P, qh, P, P, c, ok);
-        if (w > v) v = w;
-    }
-    return v;
-}
-// Lower corner, not side by side: asin((Ll^2 - Sh^2 + c^2) / (2 c Lh)) minus
-// asin((Lh^2 - Sl^2 - c^2) / (2 c S)) (S = Sl where possibly obtuse, else Sh), at
+// the exact test of collision_angles.cu:160-173: disks that possibly fit side by side
+CPF_HD bool side_by_side(double ll, double ro, double ri) { return 2.0 * add_rd_(ro, ri) <= add_ru_(1.0, -ll); }
+// Lower corner: 0 side by side, else asin((P^2 - qh^2 + c^2) / (2 c P)) minus
+// asin((P^2 - ql^2 - c^2) / (2 c S)) (S = ql where possibly obtuse, else qh), at
 // least 0; the second quotient is clamped to 1.
-// Trap sites: unless definitely obtuse, (Lh^2 - Sl^2 + c^2) / (2 c Ll) > 1; if
-// obtuse, (Ll^2 - Sh^2 - c^2) / (2 c Sh) > 1.
-CPF_HD double mixed_lo_order(double Ll, double Lh, double Sl, double Sh, double c, bool& ok) {
-    const double c2 = c * c, cc = c + c;
-    double al = fma_(Ll, Ll, -(Sh * Sh));
-    const double ah = fma_(Lh, Lh, -(Sl * Sl));
-    const double n1 = al + c2, n2 = ah - c2;
-    const double d1 = cc * Lh, d2 = cc * (n2 > 0.0 ? Sl : Sh);
+// Trap sites: unless definitely obtuse, (P^2 - ql^2 + c^2) / (2 c P) > 1; if obtuse,
+// (P^2 - qh^2 - c^2) / (2 c qh) > 1.
+CPF_HD double mixed_lo(double ll, double lh, double ro, double ri, bool& ok) {
+    if (side_by_side(ll, ro, ri)) return 0.0;
+    const double P = 1.0 - ro, ql = ll + ri, qh = lh + ri, c = ro + ri;
+    const double c2 = c * c, cc = c + c, P2 = P * P;
+    const double n1 = fma_(-qh, qh, P2 + c2), n2 = fma_(-ql, ql, P2 - c2);
+    const double d1 = cc * P, d2 = cc * (n2 > 0.0 ? ql : qh);
     const double r = rcp_(d1 * d2);
+    const double al = n1 - c2;  // P^2 - qh^2
     if (al <= c2 + kTie) {
-        const double d3 = cc * Ll;
-        ok = ok && d3 - (ah + c2) >= kEnd * d3;
+        ok = ok && qh <= P && d1 - (n2 + 2.0 * c2) >= kEnd * d1;
     } else {
-        const double d3 = cc * Sh;
-        ok = ok && d3 - (al - c2) >= kEnd * d3;
+        const double d3 = cc * qh;
+        ok = ok && qh <= P && d3 - (al - c2) >= kEnd * d3;
     }
     double v2;
     if (n2 > d2) {
@@ -213,53 +225,35 @@ CPF_HD double mixed_lo_order(double Ll, double Lh, double Sl, double Sh, double 
     } else {
         v2 = asin_quot(n2, d2, r * d1, ok);
     }
-    const double v = asin_quot(n1, d1, r * d2, ok) - v2;
+    const double v = asin_pos(n1, d1, r * d2, ok) - v2;
     return v < 0.0 ? 0.0 : v;
 }
-// the exact test of collision_angles.cu:160-173: disks that possibly fit side by side
-CPF_HD bool side_by_side(double ll, double ro, double ri) { return 2.0 * add_rd_(ro, ri) <= add_ru_(1.0, -ll); }
-CPF_HD double mixed_lo(double ll, double lh, double ro, double ri, bool& ok) {
-    if (side_by_side(ll, ro, ri)) return 0.0;
-    const double P = 1.0 - ro, ql = ll + ri, qh = lh + ri, c = ro + ri;
-    const bool x = ql <= P;
-    double v = mixed_lo_order(x ? P : ql, x ? P : qh, x ? ql : P, x ? (qh < P ? qh : P) : P, c, ok);
-    if (x && qh > P) {
-        const double w = mixed_lo_order(P, qh, P, P, c, ok);
-        if (w < v) v = w;
-    }
-    return v;
-}
-// Certificates for corners whose value is not needed.  With D = 2 (a + b) - (1 -
-// lambda.lo) > 0 no quotient of a mixed corner exceeds 1: in the order L = P the
-// excess is -D (P - c + ql), in the order L = Q it is bounded by the box guard.
+// Certificates for corners whose value is not needed.  They hold for either order of
+// P and Q: with D = 2 (a + b) - (1 - lambda.lo) > 0 no quotient of a mixed corner
+// exceeds 1, in the order L = P the excess is -D (P - c + ql), in the order L = Q it
+// is bounded by the box guard.
+// Below that, a definitely obtuse corner tests the lower ends of its quotients only.
+// end_3d's radius ranges end where those are 1 to the last bit, so no margin can
+// decide it: the directed chain itself is followed, the quotient add.lo = RD(num / ch)
+// compared by multiplication.  RD(add.lo + cl) / 2 exceeds L.hi, by the reference's
+// test RD(. / L.hi) > 1 as well as by emptiness, when add.lo + cl >= the double above
+// 2 L.hi; RD(add.lo - ch) / 2 exceeds S.hi likewise.
 CPF_HD bool clear_mixed_hi(double ll, double lh, double ro, double ri) {
     const double c = ro + ri;
     bool clear = 2.0 * c - (1.0 - ll) >= kGap;
-    if (!clear) {  // definitely obtuse: the first quotient is clamped, its lower end below 1
+    if (!clear) {
         const double P = 1.0 - ro, qh = lh + ri;
-        clear = 2.0 * c - (1.0 - lh) >= kGap && qh < P && fma_(P, P, -(qh * qh)) - c * c > kTie;
+        const double cl = add_rd_(ro, ri), ch = add_ru_(ro, ri);
+        const double l_lo = add_rd_(1.0, -ro), l_hi = add_ru_(1.0, -ro), s_hi = add_ru_(lh, ri);
+        const double num = add_rd_(mul_rd_(l_lo, l_lo), -mul_ru_(s_hi, s_hi));
+        clear = qh < P && fma_(P, P, -(qh * qh)) - c * c > kTie &&
+                num < mul_rd_(add_rd_(above_(2.0 * l_hi), -cl), ch) &&
+                num < mul_rd_(add_rd_(above_(2.0 * s_hi), ch), ch);
     }
     return clear;
 }
 CPF_HD bool clear_mixed_lo(double ll, double ro, double ri) {
     return side_by_side(ll, ro, ri) || 2.0 * (ro + ri) - (1.0 - ll) >= kGap;
-}
-
-// The directed evaluation's own trap test of the upper corner of disks 2 and 3 (no
-// arcsine), for end_3d: its radii ranges end at r2 = r3 = (1 - lambda.hi) / 4, where the lower
-// quotient is 1 to the last bit, so no margin can certify that corner.  Host builds
-// leave those boxes undecided.
-CPF_HD bool exact_clear_23_hi(double ll, double lh, double h2, double h3, bool inner) {
-#ifdef __CUDA_ARCH__
-    bool trap = false;
-    if (inner)
-        ca_mixed_hi<true, true>(Iv{ll, lh}, pt(h2), pt(h3), trap);
-    else
-        ca_mixed_hi<false, true>(Iv{ll, lh}, pt(h2), pt(h3), trap);
-    return !trap;
-#else
-    return false;
-#endif
 }
 
 // Two disks on the same border, a >= b: near-point sides L = x + a, S = x + b
@@ -329,6 +323,25 @@ CPF_HD bool box_ok(const FBox& b) {
     return ok && (1.0 - b.lh) * (1.0 + b.lh - 2.0 * m) >= fma_(4.0 * m, w, kGap);
 }
 
+// Where a box comes from: load() gives it with its radii tightened.  On the device it
+// reads memory again each time (ref.load() is opaque to the compiler), so that no
+// stage of an evaluation holds the box, or terms it shares with another stage, in
+// registers: with all stages inlined and sharing, the kernels spilled 600 B a thread.
+struct ValRef {  // a box in registers
+    FBox b;
+    CPF_HD FBox load() const { return b; }
+};
+CPF_HD void tighten(FBox& b, bool three) {
+    if (three && b.l2 < b.l3) b.l2 = b.l3;
+    if (b.l1 < b.l2) b.l1 = b.l2;
+}
+
+struct Terms {
+    double ratio, tol;
+    CPF_HD explicit Terms(const FBox& b) : ratio(fma_(-b.ll, b.ll, 1.0)), tol(fma_(kTau, ratio, kAbs)) {}
+};
+CPF_HD double disk_area(double l) { return kPi * (l * l); }
+
 struct FOut {
     uint8_t mask;     // NEED_MASK / NEED_FULL: failing sub-criteria; else nonzero when a criterion fails
     uint8_t handles;  // NEED_HANDLES
@@ -339,154 +352,185 @@ struct FOut {
 // out c13.lo > (c12 + c23).hi (directed bounds of angles that grow with the
 // radii), so g1 or g2 always holds: a handle whose tests both fail (both hold)
 // fails (holds) whatever its guards say, and they are evaluated only in between.
-template <int NEED>
-CPF_HD uint8_t middle_handle(const FBox& b, bool inner, double ratio, double tol, double ar1, double ar2, double ar3,
-                             bool& ok) {
-    const double ro12h = inner ? b.h2 : b.h1, ri12h = inner ? b.h1 : b.h2;
-    const double ro12l = inner ? b.l2 : b.l1, ri12l = inner ? b.l1 : b.l2;
-    const double ro23h = inner ? b.h2 : b.h3, ri23h = inner ? b.h3 : b.h2;
-    const double ro23l = inner ? b.l2 : b.l3, ri23l = inner ? b.l3 : b.l2;
-    const double c12_hi = mixed_hi(b.ll, b.lh, ro12h, ri12h, ok);
-    double c13_hi;
-    if (inner) {
-        ok = ok && clear_same(b.h1, b.h3, sides_inner(b.ll, b.h1, b.h3)) && clear_same(b.l1, b.l3, sides_inner(b.lh, b.l1, b.l3));
-        c13_hi = inner_angle(b.ll, b.h1, b.h3);
-    } else {
-        ok = ok && clear_same(b.h1, b.h3, sides_outer(b.h1, b.h3)) && clear_same(b.l1, b.l3, sides_outer(b.l1, b.l3));
-        c13_hi = outer_angle(b.h1, b.h3);
+template <int NEED, bool INNER, class Ref>
+CPF_HD uint8_t middle_handle(const Ref& ref, bool& ok) {
+    bool fa, fb;
+    double c12_hi, c13_hi;
+    {
+        const FBox b = ref.load();
+        const Terms t(b);
+        const double k = 0.5 * kRatio * t.ratio;
+        const double ar1 = disk_area(b.l1), ar2 = disk_area(b.l2), ar3 = disk_area(b.l3);
+        if (INNER) {
+            ok = ok && clear_same(b.h1, b.h3, sides_inner(b.ll, b.h1, b.h3)) &&
+                 clear_same(b.l1, b.l3, sides_inner(b.lh, b.l1, b.l3)) && clear_mixed_hi(b.ll, b.lh, b.h2, b.h3) &&
+                 clear_mixed_lo(b.ll, b.l2, b.l1) && clear_mixed_lo(b.ll, b.l2, b.l3);
+            c12_hi = mixed_hi(b.ll, b.lh, b.h2, b.h1, ok);
+            c13_hi = inner_angle(b.ll, b.h1, b.h3);
+        } else {
+            ok = ok && clear_same(b.h1, b.h3, sides_outer(b.h1, b.h3)) &&
+                 clear_same(b.l1, b.l3, sides_outer(b.l1, b.l3)) && clear_mixed_hi(b.ll, b.lh, b.h3, b.h2) &&
+                 clear_mixed_lo(b.ll, b.l1, b.l2) && clear_mixed_lo(b.ll, b.l3, b.l2);
+            c12_hi = mixed_hi(b.ll, b.lh, b.h1, b.h2, ok);
+            c13_hi = outer_angle(b.h1, b.h3);
+        }
+        fa = less_(0.5 * (ar1 + ar2), k * c12_hi, t.tol, ok);
+        fb = less_(fma_(0.5, ar1 + ar3, ar2), k * c13_hi, t.tol, ok);
     }
-    ok = ok && clear_mixed_hi(b.ll, b.lh, ro23h, ri23h) && clear_mixed_lo(b.ll, ro12l, ri12l) &&
-         clear_mixed_lo(b.ll, ro23l, ri23l);
-    const double k = 0.5 * kRatio * ratio;
-    const bool fa = less_(0.5 * (ar1 + ar2), k * c12_hi, tol, ok);
-    const bool fb = less_(fma_(0.5, ar1 + ar3, ar2), k * c13_hi, tol, ok);
     if (!ok) return 0;
     if (!fa && !fb) return 0;
     if (NEED < NEED_MASK && fa && fb) return 3;
+    const FBox b = ref.load();
     uint8_t m = 0;
     if (fa) {
-        const double c13_lo = inner ? inner_angle(b.lh, b.l1, b.l3) : outer_angle(b.l1, b.l3);
-        const double c23_hi = mixed_hi(b.ll, b.lh, ro23h, ri23h, ok);
+        const double c13_lo = INNER ? inner_angle(b.lh, b.l1, b.l3) : outer_angle(b.l1, b.l3);
+        const double c23_hi =
+            INNER ? mixed_hi(b.ll, b.lh, b.h2, b.h3, ok) : mixed_hi(b.ll, b.lh, b.h3, b.h2, ok);
         if (less_(c13_lo, c12_hi + c23_hi, kTau, ok)) m |= 1;
         if (NEED != NEED_FULL && m) return m;
     }
     if (fb) {
-        const double c12_lo = mixed_lo(b.ll, b.lh, ro12l, ri12l, ok);
-        const double c23_lo = mixed_lo(b.ll, b.lh, ro23l, ri23l, ok);
+        const double c12_lo = INNER ? mixed_lo(b.ll, b.lh, b.l2, b.l1, ok) : mixed_lo(b.ll, b.lh, b.l1, b.l2, ok);
+        const double c23_lo = INNER ? mixed_lo(b.ll, b.lh, b.l2, b.l3, ok) : mixed_lo(b.ll, b.lh, b.l3, b.l2, ok);
         if (!less_(c13_hi, c12_lo + c23_lo, kTau, ok)) m |= 2;
     }
     return m;
 }
 
 // end_configuration.cu:71-101
-CPF_HD bool end2d_fails(const FBox& b, bool inner, double ratio, double tol, double ar1, double ar2, bool& ok) {
-    const double roh = inner ? b.h2 : b.h1, rih = inner ? b.h1 : b.h2;
-    const double rol = inner ? b.l2 : b.l1, ril = inner ? b.l1 : b.l2;
-    ok = ok && clear_mixed_lo(b.ll, rol, ril);
-    const double ca_hi = mixed_hi(b.ll, b.lh, roh, rih, ok);
-    const double sa_hi = inner ? semi_outer(b.h2) : semi_inner(b.ll, b.h2);
-    const double other = inner ? semi_inner(b.ll, b.h1) : semi_outer(b.h1);
-    const double t = inner ? 1.0 - 2.0 * b.h2 : fma_(2.0, b.h2, b.lh);
-    double rho = inner ? t * t - b.lh * b.lh : 1.0 - t * t;
-    if (rho < 0.0) rho = 0.0;
-    const double a_hi = ca_hi + sa_hi, used = 0.5 * ratio * a_hi;
-    const double lhs = fma_(0.5, ar1, ar2);
-    // reusable = 0.5 rho (a.lo - other), a.lo in [0, a.hi]
-    if (!ok) return false;
-    if (lhs - kRatio * fma_(0.5 * rho, other, used) > tol) return false;
-    if (lhs - kRatio * fma_(0.5 * rho, other - a_hi, used) < -tol) return true;
-    const double a_lo = mixed_lo(b.ll, b.lh, rol, ril, ok) + (inner ? semi_outer(b.l2) : semi_inner(b.lh, b.l2));
+template <bool INNER, class Ref>
+CPF_HD bool end2d_fails(const Ref& ref, bool& ok) {
+    double lhs, rho, used, other, tol;
+    {
+        const FBox b = ref.load();
+        const Terms t(b);
+        tol = t.tol;
+        ok = ok && (INNER ? clear_mixed_lo(b.ll, b.l2, b.l1) : clear_mixed_lo(b.ll, b.l1, b.l2));
+        const double ca_hi =
+            INNER ? mixed_hi(b.ll, b.lh, b.h2, b.h1, ok) : mixed_hi(b.ll, b.lh, b.h1, b.h2, ok);
+        const double sa_hi = INNER ? semi_outer(b.h2) : semi_inner(b.ll, b.h2);
+        other = INNER ? semi_inner(b.ll, b.h1) : semi_outer(b.h1);
+        const double q = INNER ? 1.0 - 2.0 * b.h2 : fma_(2.0, b.h2, b.lh);
+        rho = INNER ? q * q - b.lh * b.lh : 1.0 - q * q;
+        if (rho < 0.0) rho = 0.0;
+        const double a_hi = ca_hi + sa_hi;
+        used = 0.5 * t.ratio * a_hi;
+        lhs = fma_(0.5, disk_area(b.l1), disk_area(b.l2));
+        // reusable = 0.5 rho (a.lo - other), a.lo in [0, a.hi]
+        if (!ok) return false;
+        if (lhs - kRatio * fma_(0.5 * rho, other, used) > tol) return false;
+        if (lhs - kRatio * fma_(0.5 * rho, other - a_hi, used) < -tol) return true;
+    }
+    const FBox b = ref.load();
+    const double a_lo = INNER ? mixed_lo(b.ll, b.lh, b.l2, b.l1, ok) + semi_outer(b.l2)
+                              : mixed_lo(b.ll, b.lh, b.l1, b.l2, ok) + semi_inner(b.lh, b.l2);
     return less_(lhs, kRatio * fma_(0.5 * rho, other - a_lo, used), tol, ok);
 }
 
 // end_configuration.cu:154-210
-CPF_HD bool end3d_fails(const FBox& b, bool inner, double ratio, double tol, double ar1, double ar2, double ar3,
-                        bool& ok) {
-    const double ro12h = inner ? b.h2 : b.h1, ri12h = inner ? b.h1 : b.h2;
-    const double ro12l = inner ? b.l2 : b.l1, ri12l = inner ? b.l1 : b.l2;
-    const double ro23h = inner ? b.h2 : b.h3, ri23h = inner ? b.h3 : b.h2;
-    const double ro23l = inner ? b.l2 : b.l3, ri23l = inner ? b.l3 : b.l2;
+template <bool INNER, class Ref>
+CPF_HD bool end3d_fails(const Ref& ref, bool& ok) {
     double a13_hi;
-    if (inner) {
-        ok = ok && clear_same(b.h1, b.h3, sides_inner(b.ll, b.h1, b.h3)) && clear_same_low(b.l1, b.l3, sides_inner(b.lh, b.l1, b.l3));
-        a13_hi = inner_angle(b.ll, b.h1, b.h3);
-    } else {
-        ok = ok && clear_same(b.h1, b.h3, sides_outer(b.h1, b.h3)) && clear_same_low(b.l1, b.l3, sides_outer(b.l1, b.l3));
-        a13_hi = outer_angle(b.h1, b.h3);
+    {
+        const FBox b = ref.load();
+        double s_lo;
+        if (INNER) {
+            ok = ok && clear_same(b.h1, b.h3, sides_inner(b.ll, b.h1, b.h3)) &&
+                 clear_same_low(b.l1, b.l3, sides_inner(b.lh, b.l1, b.l3)) && clear_mixed_hi(b.ll, b.lh, b.h2, b.h1) &&
+                 clear_mixed_hi(b.ll, b.lh, b.h2, b.h3) && clear_mixed_lo(b.ll, b.l2, b.l1) &&
+                 clear_mixed_lo(b.ll, b.l2, b.l3);
+            if (!ok) return false;
+            a13_hi = inner_angle(b.ll, b.h1, b.h3);
+            s_lo = mixed_lo(b.ll, b.lh, b.l2, b.l1, ok) + mixed_lo(b.ll, b.lh, b.l2, b.l3, ok);
+        } else {
+            ok = ok && clear_same(b.h1, b.h3, sides_outer(b.h1, b.h3)) &&
+                 clear_same_low(b.l1, b.l3, sides_outer(b.l1, b.l3)) && clear_mixed_hi(b.ll, b.lh, b.h1, b.h2) &&
+                 clear_mixed_hi(b.ll, b.lh, b.h3, b.h2) && clear_mixed_lo(b.ll, b.l1, b.l2) &&
+                 clear_mixed_lo(b.ll, b.l3, b.l2);
+            if (!ok) return false;
+            a13_hi = outer_angle(b.h1, b.h3);
+            s_lo = mixed_lo(b.ll, b.lh, b.l1, b.l2, ok) + mixed_lo(b.ll, b.lh, b.l3, b.l2, ok);
+        }
+        if (less_(a13_hi, s_lo, kTau, ok)) return false;
     }
-    ok = ok && clear_mixed_hi(b.ll, b.lh, ro12h, ri12h) && clear_mixed_lo(b.ll, ro12l, ri12l) &&
-         clear_mixed_lo(b.ll, ro23l, ri23l) &&
-         (clear_mixed_hi(b.ll, b.lh, ro23h, ri23h) || exact_clear_23_hi(b.ll, b.lh, b.h2, b.h3, inner));
-    if (!ok) return false;
-    const double s_lo = mixed_lo(b.ll, b.lh, ro12l, ri12l, ok) + mixed_lo(b.ll, b.lh, ro23l, ri23l, ok);
-    if (less_(a13_hi, s_lo, kTau, ok)) return false;
-    const double a13_lo = inner ? inner_angle(b.lh, b.l1, b.l3) : outer_angle(b.l1, b.l3);
-    const double a12_hi = mixed_hi(b.ll, b.lh, ro12h, ri12h, ok);
-    const double a3_lo = inner ? semi_inner(b.lh, b.l3) : semi_outer(b.l3);
-    const double a3_hi = inner ? semi_inner(b.ll, b.h3) : semi_outer(b.h3);
-    const double a2_hi = inner ? semi_outer(b.h2) : semi_inner(b.ll, b.h2);
-    const double t = inner ? fma_(2.0, b.h3, b.lh) : 1.0 - 2.0 * b.h3;
-    double rho = inner ? 1.0 - t * t : t * t - b.lh * b.lh;
+    const FBox b = ref.load();
+    const Terms t(b);
+    const double a13_lo = INNER ? inner_angle(b.lh, b.l1, b.l3) : outer_angle(b.l1, b.l3);
+    const double a12_hi = INNER ? mixed_hi(b.ll, b.lh, b.h2, b.h1, ok) : mixed_hi(b.ll, b.lh, b.h1, b.h2, ok);
+    const double a3_lo = INNER ? semi_inner(b.lh, b.l3) : semi_outer(b.l3);
+    const double a3_hi = INNER ? semi_inner(b.ll, b.h3) : semi_outer(b.h3);
+    const double a2_hi = INNER ? semi_outer(b.h2) : semi_inner(b.ll, b.h2);
+    const double q = INNER ? fma_(2.0, b.h3, b.lh) : 1.0 - 2.0 * b.h3;
+    double rho = INNER ? 1.0 - q * q : q * q - b.lh * b.lh;
     if (rho < 0.0) rho = 0.0;
     const double alpha = (a13_lo + a3_lo) - (a12_hi + a2_hi);
-    const double used = 0.5 * ratio * (a13_hi + a3_hi);
+    const double used = 0.5 * t.ratio * (a13_hi + a3_hi);
+    double tol = t.tol;
     if (b.l3 < kMinB) tol = fma_(0.5 * kLowSlack, rho, tol);
-    return less_(fma_(0.5, ar1, ar2 + ar3), kRatio * fma_(-0.5 * rho, alpha, used), tol, ok);
+    const double lhs = fma_(0.5, disk_area(b.l1), disk_area(b.l2) + disk_area(b.l3));
+    return less_(lhs, kRatio * fma_(-0.5 * rho, alpha, used), tol, ok);
 }
 
-// The verdict of a box that is neither empty nor stopped by the fit check.  order:
-// bit 0 = second handle first (DECIDE).  Returns false when the box is left to
-// eval_box; else o holds what NEED asks for.
-template <int FAM, int NEED>
-CPF_HD bool filter_box(const FBox& b, int order, FOut& o) {
-    constexpr bool kThree = FAM != 1 && FAM != 4;
-    bool ok = box_ok<kThree>(b);
+// start_configuration.cu:126-162.  Criterion 1 is evaluated when a12 + a23 > a13
+// possibly holds, criterion 2 unless it definitely holds; "definitely" implies
+// "possibly".
+template <int NEED, class Ref>
+CPF_HD bool start_box(const Ref& ref, FOut& o) {
+    bool ok, f1, f2;
+    double a12_hi, a13_hi;
+    {
+        const FBox b = ref.load();
+        ok = clear_same(b.h1, b.h3, sides_outer(b.h1, b.h3)) && clear_same(b.l1, b.l3, sides_outer(b.l1, b.l3)) &&
+             clear_mixed_hi(b.ll, b.lh, b.h3, b.h2) && clear_mixed_lo(b.ll, b.l1, b.l2) &&
+             clear_mixed_lo(b.ll, b.l3, b.l2);
+        if (!ok) return false;
+        const Terms t(b);
+        const double so = semi_outer(b.h1), k = 0.5 * kRatio * t.ratio;
+        a12_hi = mixed_hi(b.ll, b.lh, b.h1, b.h2, ok);
+        a13_hi = outer_angle(b.h1, b.h3);
+        const double ar1 = disk_area(b.l1), ar2 = disk_area(b.l2), ar3 = disk_area(b.l3);
+        f1 = less_(fma_(0.5, ar2, ar1), k * (so + a12_hi), t.tol, ok);
+        f2 = less_(fma_(0.5, ar3, ar1 + ar2), k * (so + a13_hi), t.tol, ok);
+    }
     if (!ok) return false;
-    o.mask = 0;
-    o.handles = 1;
-    const double ratio = fma_(-b.ll, b.ll, 1.0);
-    const double tol = fma_(kTau, ratio, kAbs);
-    const double ar1 = kPi * (b.l1 * b.l1), ar2 = kPi * (b.l2 * b.l2), ar3 = kPi * (b.l3 * b.l3);
-    if (FAM == 0) {  // start_configuration.cu:126-162
-        ok = clear_same(b.h1, b.h3, sides_outer(b.h1, b.h3)) && clear_same(b.l1, b.l3, sides_outer(b.l1, b.l3)) && clear_mixed_hi(b.ll, b.lh, b.h3, b.h2) &&
-             clear_mixed_lo(b.ll, b.l1, b.l2) && clear_mixed_lo(b.ll, b.l3, b.l2);
+    if (NEED < NEED_MASK && f1 && f2) {
+        o.mask = 1;
+        return true;
+    }
+    if (NEED != NEED_HANDLES && !f1 && !f2) return true;
+    const FBox b = ref.load();
+    bool pos = true, def = false;
+    if (f2 || NEED == NEED_HANDLES) {
+        def = less_(a13_hi, mixed_lo(b.ll, b.lh, b.l1, b.l2, ok) + mixed_lo(b.ll, b.lh, b.l3, b.l2, ok), kTau, ok);
         if (!ok) return false;
-        const double so = semi_outer(b.h1);
-        const double a12_hi = mixed_hi(b.ll, b.lh, b.h1, b.h2, ok);
-        const double a13_hi = outer_angle(b.h1, b.h3);
-        const double k = 0.5 * kRatio * ratio;
-        const bool f1 = less_(fma_(0.5, ar2, ar1), k * (so + a12_hi), tol, ok);
-        const bool f2 = less_(fma_(0.5, ar3, ar1 + ar2), k * (so + a13_hi), tol, ok);
-        if (!ok) return false;
-        // criterion 1 is evaluated when a12 + a23 > a13 possibly holds, criterion 2
-        // unless it definitely holds; "definitely" implies "possibly"
-        if (NEED < NEED_MASK && f1 && f2) {
-            o.mask = 1;
-            return true;
-        }
-        if (NEED != NEED_HANDLES && !f1 && !f2) return true;
-        bool pos = true, def = false;
-        if (f2 || NEED == NEED_HANDLES) {
-            def = less_(a13_hi, mixed_lo(b.ll, b.lh, b.l1, b.l2, ok) + mixed_lo(b.ll, b.lh, b.l3, b.l2, ok), kTau, ok);
-            if (!ok) return false;
-        }
-        if ((f1 || NEED == NEED_HANDLES) && !def)
-            pos = less_(outer_angle(b.l1, b.l3), a12_hi + mixed_hi(b.ll, b.lh, b.h3, b.h2, ok), kTau, ok);
-        if (pos && f1) o.mask |= 1;
-        if (NEED != NEED_FULL && o.mask) return ok;
-        if (!def && f2) o.mask |= 2;
-        o.handles = (pos ? 1 : 0) + (def ? 0 : 1);
-        return ok;
-    } else if (FAM == 1) {  // start_configuration.cu:169-188
+    }
+    if ((f1 || NEED == NEED_HANDLES) && !def)
+        pos = less_(outer_angle(b.l1, b.l3), a12_hi + mixed_hi(b.ll, b.lh, b.h3, b.h2, ok), kTau, ok);
+    if (pos && f1) o.mask |= 1;
+    if (NEED != NEED_FULL && o.mask) return ok;
+    if (!def && f2) o.mask |= 2;
+    o.handles = (pos ? 1 : 0) + (def ? 0 : 1);
+    return ok;
+}
+
+// start_configuration.cu:169-188.  The reused angle lies between 0 and a12.hi + a2.hi - a1.
+template <class Ref>
+CPF_HD bool start_end_2d_box(const Ref& ref, FOut& o) {
+    bool ok;
+    double a1, rho, used, lhs, tol;
+    {
+        const FBox b = ref.load();
+        const Terms t(b);
+        tol = t.tol;
         ok = clear_mixed_lo(b.ll, b.l1, b.l2);
-        const double a1 = semi_outer(b.h1), a2_hi = semi_inner(b.ll, b.h2);
-        const double a12_hi = mixed_hi(b.ll, b.lh, b.h1, b.h2, ok);
-        const double t = fma_(2.0, b.h2, b.lh);
-        double rho = 1.0 - t * t;
+        a1 = semi_outer(b.h1);
+        const double a2_hi = semi_inner(b.ll, b.h2), a12_hi = mixed_hi(b.ll, b.lh, b.h1, b.h2, ok);
+        const double q = fma_(2.0, b.h2, b.lh);
+        rho = 1.0 - q * q;
         if (rho < 0.0) rho = 0.0;
-        const double used = 0.5 * ratio * (a1 + a2_hi + a12_hi), lhs = ar1 + ar2;
+        used = 0.5 * t.ratio * (a1 + a2_hi + a12_hi);
+        lhs = disk_area(b.l1) + disk_area(b.l2);
         if (!ok) return false;
-        // the reused angle lies between 0 and a12.hi + a2.hi - a1
         if (lhs - kRatio * used > tol) return true;
         double top = a12_hi + a2_hi - a1;
         if (top < 0.0) top = 0.0;
@@ -494,70 +538,89 @@ CPF_HD bool filter_box(const FBox& b, int order, FOut& o) {
             o.mask = 1;
             return true;
         }
-        double reuse = mixed_lo(b.ll, b.lh, b.l1, b.l2, ok) + semi_inner(b.lh, b.l2) - a1;
-        if (reuse < 0.0) reuse = 0.0;
-        if (less_(lhs, kRatio * fma_(-0.5 * rho, reuse, used), tol, ok)) o.mask = 1;
-        return ok;
-    } else if (FAM == 2) {  // start_configuration.cu:227-265 (a13 of r1 and r2, as there)
-        ok = clear_same(b.h1, b.h2, sides_outer(b.h1, b.h2)) && clear_same(b.l1, b.l2, sides_outer(b.l1, b.l2)) && clear_mixed_lo(b.ll, b.l1, b.l2) &&
-             clear_mixed_lo(b.ll, b.l3, b.l2);
+    }
+    const FBox b = ref.load();
+    double reuse = mixed_lo(b.ll, b.lh, b.l1, b.l2, ok) + semi_inner(b.lh, b.l2) - a1;
+    if (reuse < 0.0) reuse = 0.0;
+    if (less_(lhs, kRatio * fma_(-0.5 * rho, reuse, used), tol, ok)) o.mask = 1;
+    return ok;
+}
+
+// start_configuration.cu:227-265 (a13 of r1 and r2, as there).  The reused angle
+// a.lo - a122.hi lies between 0 and a.hi - a122.hi.
+template <class Ref>
+CPF_HD bool start_end_3d_box(const Ref& ref, FOut& o) {
+    bool ok;
+    double a122_hi, lane, used, lhs, tol;
+    {
+        const FBox b = ref.load();
+        ok = clear_same(b.h1, b.h2, sides_outer(b.h1, b.h2)) && clear_same(b.l1, b.l2, sides_outer(b.l1, b.l2)) &&
+             clear_mixed_lo(b.ll, b.l1, b.l2) && clear_mixed_lo(b.ll, b.l3, b.l2);
         if (!ok) return false;
+        const Terms t(b);
+        tol = t.tol;
         const double a1_hi = semi_outer(b.h1), a2_hi = semi_inner(b.ll, b.h2), a3_hi = semi_outer(b.h3);
         const double a12_hi = mixed_hi(b.ll, b.lh, b.h1, b.h2, ok), a13_hi = outer_angle(b.h1, b.h2);
         const double a23_hi = mixed_hi(b.ll, b.lh, b.h3, b.h2, ok);
         const double b123_hi = a12_hi + a23_hi, b13_hi = a13_hi < b123_hi ? b123_hi : a13_hi;
-        const double a123_hi = a1_hi + b13_hi + a3_hi, a122_hi = a1_hi + a12_hi + a2_hi;
+        const double a123_hi = a1_hi + b13_hi + a3_hi;
+        a122_hi = a1_hi + a12_hi + a2_hi;
         const double a_hi = a123_hi < a122_hi ? a122_hi : a123_hi;
         const double outer = fma_(-2.0, b.h3, 1.0);
-        double lane = 0.5 * (outer * outer - b.lh * b.lh);
+        lane = 0.5 * (outer * outer - b.lh * b.lh);
         if (lane < 0.0) lane = 0.0;
-        const double used = 0.5 * ratio * a_hi, lhs = ar1 + (ar2 + ar3);
+        used = 0.5 * t.ratio * a_hi;
+        lhs = disk_area(b.l1) + (disk_area(b.l2) + disk_area(b.l3));
         if (!ok) return false;
-        // the reused angle a.lo - a122.hi lies between 0 and a.hi - a122.hi
         if (lhs - kRatio * used > tol) return true;
         if (lhs - kRatio * fma_(-lane, a_hi - a122_hi, used) < -tol) {
             o.mask = 1;
             return true;
         }
-        const double a1_lo = semi_outer(b.l1), a2_lo = semi_inner(b.lh, b.l2), a3_lo = semi_outer(b.l3);
-        const double a12_lo = mixed_lo(b.ll, b.lh, b.l1, b.l2, ok), a13_lo = outer_angle(b.l1, b.l2);
-        const double b123_lo = a12_lo + mixed_lo(b.ll, b.lh, b.l3, b.l2, ok);
-        const double b13_lo = a13_lo < b123_lo ? b123_lo : a13_lo;
-        const double a123_lo = a1_lo + b13_lo + a3_lo, a122_lo = a1_lo + a12_lo + a2_lo;
-        double reuse = (a123_lo < a122_lo ? a122_lo : a123_lo) - a122_hi;
-        if (reuse < 0.0) reuse = 0.0;
-        if (less_(lhs, kRatio * fma_(-lane, reuse, used), tol, ok)) o.mask = 1;
-        return ok;
-    } else if (FAM == 3) {
-        const bool second = NEED != NEED_FULL && (order & 1);
-        uint8_t h = 0;
-        for (int i = 0; i < 2; ++i) {
-            const bool inner = (i == 0) != second;
-            ++h;
-            const uint8_t m = middle_handle<NEED>(b, inner, ratio, tol, ar1, ar2, ar3, ok);
-            if (!ok) return false;
-            o.mask |= inner ? m : (uint8_t)(m << 2);
-            if (NEED != NEED_FULL && m) break;
-        }
-        o.handles = h;
-        return true;
-    } else {
-        const bool second = NEED != NEED_FULL && (order & 1);
-        uint8_t h = 0;
-        for (int i = 0; i < 2; ++i) {
-            const bool inner = (i == 0) != second;
-            ++h;
-            const bool f = FAM == 4 ? end2d_fails(b, inner, ratio, tol, ar1, ar2, ok)
-                                    : end3d_fails(b, inner, ratio, tol, ar1, ar2, ar3, ok);
-            if (!ok) return false;
-            if (f) {
-                o.mask |= inner ? 1 : 2;
-                if (NEED != NEED_FULL) break;
-            }
-        }
-        o.handles = h;
-        return true;
     }
+    const FBox b = ref.load();
+    const double a1_lo = semi_outer(b.l1), a2_lo = semi_inner(b.lh, b.l2), a3_lo = semi_outer(b.l3);
+    const double a12_lo = mixed_lo(b.ll, b.lh, b.l1, b.l2, ok), a13_lo = outer_angle(b.l1, b.l2);
+    const double b123_lo = a12_lo + mixed_lo(b.ll, b.lh, b.l3, b.l2, ok);
+    const double b13_lo = a13_lo < b123_lo ? b123_lo : a13_lo;
+    const double a123_lo = a1_lo + b13_lo + a3_lo, a122_lo = a1_lo + a12_lo + a2_lo;
+    double reuse = (a123_lo < a122_lo ? a122_lo : a123_lo) - a122_hi;
+    if (reuse < 0.0) reuse = 0.0;
+    if (less_(lhs, kRatio * fma_(-lane, reuse, used), tol, ok)) o.mask = 1;
+    return ok;
+}
+
+// The verdict of a box that is neither empty nor stopped by the fit check.  order:
+// bit 0 = second handle first (DECIDE).  Returns false when the box is left to
+// eval_box; else o holds what NEED asks for.
+template <int FAM, int NEED, class Ref>
+CPF_HD bool filter_box(const Ref& ref, int order, FOut& o) {
+    constexpr bool kThree = FAM != 1 && FAM != 4;
+    if (!box_ok<kThree>(ref.load())) return false;
+    o.mask = 0;
+    o.handles = 1;
+    if (FAM == 0) return start_box<NEED>(ref, o);
+    if (FAM == 1) return start_end_2d_box(ref, o);
+    if (FAM == 2) return start_end_3d_box(ref, o);
+    const bool second = NEED != NEED_FULL && (order & 1);
+    bool ok = true;
+    uint8_t h = 0;
+    for (int i = 0; i < 2; ++i) {
+        const bool inner = (i == 0) != second;
+        ++h;
+        uint8_t m;
+        if (FAM == 3)
+            m = inner ? middle_handle<NEED, true>(ref, ok) : (uint8_t)(middle_handle<NEED, false>(ref, ok) << 2);
+        else if (FAM == 4)
+            m = inner ? (end2d_fails<true>(ref, ok) ? 1 : 0) : (end2d_fails<false>(ref, ok) ? 2 : 0);
+        else
+            m = inner ? (end3d_fails<true>(ref, ok) ? 1 : 0) : (end3d_fails<false>(ref, ok) ? 2 : 0);
+        if (!ok) return false;
+        o.mask |= m;
+        if (NEED != NEED_FULL && m) break;
+    }
+    o.handles = h;
+    return true;
 }
 
 }  // namespace flt

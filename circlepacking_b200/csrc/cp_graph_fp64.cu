@@ -1,23 +1,28 @@
-// Persistent level kernels of the device-driven loop, precision fp64
+// Depth-first kernels of the graph engine, precision fp64
 // (cp_graph_kernels.cuh), by family and block-size variant.
+#include "cp_engine.h"
 #include "cp_graph_kernels.cuh"
 
 using namespace cpb;
 
 namespace {
+template <int FAM, int BLOCK>
+DeepKernel deep() {
+    return {(void*)k_refine_deep<FAM, 0, BLOCK>, deep_threads(BLOCK), (int)sizeof(DeepSmem<FAM, BLOCK>)};
+}
 template <int FAM>
-void* pick(int v) {
+DeepKernel pick(int v) {
     switch (v) {
-    case 0: return (void*)k_level_persist<FAM, 0, 64>;
-    case 1: return (void*)k_level_persist<FAM, 0, 128>;
-    case 2: return (void*)k_level_persist<FAM, 0, 256>;
-    case 3: return (void*)k_level_persist<FAM, 0, 512>;
-    default: return (void*)k_level_persist<FAM, 0, 1024>;
+    case 0: return deep<FAM, 64>();
+    case 1: return deep<FAM, 128>();
+    case 2: return deep<FAM, 256>();
+    case 3: return deep<FAM, 512>();
+    default: return deep<FAM, 1024>();
     }
 }
 }  // namespace
 
-void* cp_graph_kernel_fp64(int fam, int variant) {
+DeepKernel cp_deep_kernel_fp64(int fam, int variant) {
     switch (fam) {
     case 0: return pick<0>(variant);
     case 1: return pick<1>(variant);

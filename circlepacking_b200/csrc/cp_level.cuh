@@ -21,6 +21,7 @@ enum : int {
     C_OUT = 8,      // children appended
     C_ERR = 9,      // error flags
     C_BEST_SLAB = 10,
+    C_CLAIM = C_BEST_SLAB,  // in a refinement: boxes of the chunk handed to warps
     C_EVALUATED = 11,
     C_FIRST_BITS = 12,  // ordered encoding of the smallest failing lambda.lb
     C_ERRBOX_CLAIM = 13,
@@ -71,19 +72,20 @@ __device__ __forceinline__ unsigned long long box_hash(const double* lo, const d
     return h;
 }
 
-// Per-block shared state of the level step; WARPS = warps per block.
-template <int WARPS>
-struct LevelSmem {
+// Per-block shared state of the level step: counts, and for kernels that append
+// children to a level (WARPS > 0) the lane owning each slot of a warp's children.
+struct LevelCounts {
     unsigned long long hist[8];
     unsigned long long depth[kDepthBins];
     unsigned long long handles;
     unsigned long long dig_sum, dig_xor;
-    // per warp: the lane owning each slot of one iteration's children
+};
+template <int WARPS>
+struct LevelSmem : LevelCounts {
     uint8_t own[WARPS][32 * 16];
 };
 
-template <int WARPS>
-__device__ __forceinline__ void level_smem_init(LevelSmem<WARPS>& sm) {
+__device__ __forceinline__ void level_smem_init(LevelCounts& sm) {
     for (int t = threadIdx.x; t < kDepthBins; t += blockDim.x) sm.depth[t] = 0;
     if (threadIdx.x < 8) sm.hist[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
@@ -93,11 +95,123 @@ __device__ __forceinline__ void level_smem_init(LevelSmem<WARPS>& sm) {
     }
 }
 
-// (defined below)
+// Folds a warp's evaluated boxes (v >= 0) into the block's digest words.
+template <int D>
+__device__ __forceinline__ void digest_step(LevelCounts& sm, int v, const double* lo, const double* hi) {
+    const unsigned long long h = v >= 0 ? box_hash<D>(lo, hi, v) : 0ull;
+    unsigned long long hs = h;
+    unsigned long long hx = v >= 0 ? mix64(h ^ 0x5851f42d4c957f2dull) : 0ull;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        hs += __shfl_xor_sync(0xffffffffu, hs, off);
+        hx ^= __shfl_xor_sync(0xffffffffu, hx, off);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&sm.dig_sum, hs);
+        atomicXor(&sm.dig_xor, hx);
+    }
+}
+
+// Counts one warp step: v = the lane's verdict (-1: no box evaluated).  One
+// shared-memory atomic per verdict, depth and flag present in the warp.
+template <int D>
+__device__ __forceinline__ void tally(LevelCounts& sm, int digest, int v, bool unresolved, bool fp32_decided,
+                                      const double* lo, const double* hi, int depth) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const unsigned b = __ballot_sync(0xffffffffu, v == k);
+        if (b && lane == 0) atomicAdd(&sm.hist[k], (unsigned long long)__popc(b));
+    }
+    const unsigned bu = __ballot_sync(0xffffffffu, unresolved);
+    const unsigned bf = __ballot_sync(0xffffffffu, fp32_decided);
+    if (lane == 0) {
+        if (bu) atomicAdd(&sm.hist[C_UNRESOLVED], (unsigned long long)__popc(bu));
+        if (bf) atomicAdd(&sm.hist[C_FP32], (unsigned long long)__popc(bf));
+    }
+    // (a step holds boxes of one or two depths: peel them off instead of matching)
+    const int dbin = depth < kDepthBins ? depth : kDepthBins - 1;
+    unsigned left = __ballot_sync(0xffffffffu, v >= 0);
+    while (left) {
+        const int d0 = __shfl_sync(0xffffffffu, dbin, __ffs(left) - 1);
+        const unsigned same = __ballot_sync(0xffffffffu, v >= 0 && dbin == d0);
+        if (lane == 0) atomicAdd(&sm.depth[d0], (unsigned long long)__popc(same));
+        left &= ~same;
+    }
+    if (digest) digest_step<D>(sm, v, lo, hi);
+}
+
+// The axis a not-proved box is split on (0 where the policy splits every axis).
+template <int D>
+__device__ __forceinline__ int split_axis(int policy, double lambda_scale, const double* lo, const double* hi) {
+    if (policy == SPLIT_WIDEST) return widest_axis<D>(lo, hi);
+    if (policy == SPLIT_HYBRID) return hybrid_axis<D>(lo, hi, lambda_scale);
+    return 0;
+}
+
+// Appends the children of the warp's boxes (nchild per lane, 0 = none) to the
+// next level: the warp reserves one contiguous range and writes it
+// cooperatively, lane k of an iteration writing slot k, so every store of an
+// axis array is one coalesced 256-byte segment per warp.
+template <int FAM, int WARPS>
+__device__ __forceinline__ void emit_children(const LevelArgs& a, LevelSmem<WARPS>& sm, const double* lo,
+                                              const double* hi, int depth, int axis, unsigned nchild) {
+    constexpr int D = family_dims(FAM);
+    unsigned excl, total;
+    const unsigned long long wbase = warp_reserve_range(&a.cnt[C_OUT], nchild, &excl, &total);
+    if (!total) return;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (wbase + total > a.out.cap) {
+        if (lane == 0) atomicOr(&a.cnt[C_ERR], E_OVERFLOW);
+        return;
+    }
+    // slot -> owning lane; the parent box itself comes from the owner by shuffles
+    for (unsigned c = 0; c < nchild; ++c) sm.own[w][excl + c] = (uint8_t)lane;
+    __syncwarp();
+    for (unsigned base = 0; base < total; base += 32) {
+        const unsigned k = base + lane;
+        const bool valid = k < total;
+        const int own = valid ? sm.own[w][k] : 0;
+        double plo[4], phi[4], clo[4], chi[4];
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            plo[d] = __shfl_sync(0xffffffffu, lo[d], own);
+            phi[d] = __shfl_sync(0xffffffffu, hi[d], own);
+        }
+        const int c = (int)k - (int)__shfl_sync(0xffffffffu, excl, own);
+        const int pax = __shfl_sync(0xffffffffu, axis, own);
+        const int pdep = __shfl_sync(0xffffffffu, depth, own);
+        if (valid) {
+            make_child<D>(plo, phi, a.policy, pax, c, clo, chi);
+            const bool alive = clip_child<FAM>(clo, chi, a.tab);
+            const size_t o = (size_t)(wbase + k);
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                a.out.lo[d * a.out.cap + o] = clo[d];
+                a.out.hi[d * a.out.cap + o] = chi[d];
+            }
+            a.out.depth[o] = alive ? (uint8_t)(pdep + 1) : (uint8_t)0xFF;
+        }
+    }
+    __syncwarp();
+}
+
+// The end of a level step whose children all go to the next level, for every
+// lane of a warp (all 32 must call it): v = the lane's verdict (-1: no box
+// evaluated), its box lo/hi and depth, given = its split axis for SPLIT_GIVEN.
 template <int FAM, int WARPS>
 __device__ __forceinline__ void level_emit(const LevelArgs& a, LevelSmem<WARPS>& sm, int v, bool clipped,
                                            bool fp32_decided, const double* lo, const double* hi, int depth,
-                                           int given);
+                                           int given) {
+    constexpr int D = family_dims(FAM);
+    const bool open = v >= 0 && v != V_PROVED && v != V_EMPTY;
+    const bool split = open && depth < a.max_depth;
+    const unsigned bc = __ballot_sync(0xffffffffu, clipped);
+    if (bc && (threadIdx.x & 31) == 0) atomicAdd(&sm.hist[C_CLIPPED], (unsigned long long)__popc(bc));
+    tally<D>(sm, a.digest, v, open && !split, fp32_decided, lo, hi, depth);
+    const int axis = !split ? 0 : a.policy == SPLIT_GIVEN ? given : split_axis<D>(a.policy, a.lambda_scale, lo, hi);
+    emit_children<FAM>(a, sm, lo, hi, depth, axis, split ? (unsigned)fanout(a.policy, D) : 0u);
+}
 
 // One lane's box j of the chunk (j >= a.count: the lane only takes part in the
 // warp's collective child write).  All 32 lanes of the warp must call it.
@@ -127,7 +241,7 @@ __device__ __forceinline__ void level_step(const LevelArgs& a, size_t j, LevelSm
                 uint8_t pmask;
                 const int pre = prefilter_box<FAM>(lo, hi, ord, false, &pmask);
                 if (pre == PF_UNDECIDED) {
-                    const Verdict r = judge_box<FAM, DECIDE, flt::NEED_HANDLES>(lo, hi, ord);
+                    const Verdict r = judge_box<FAM, DECIDE, flt::NEED_HANDLES>(BoxRef<D>{a.in.lo + i, a.in.hi + i, a.in.cap}, ord);
                     v = r.verdict;
                     handles += r.handles;
                 } else {
@@ -135,7 +249,7 @@ __device__ __forceinline__ void level_step(const LevelArgs& a, size_t j, LevelSm
                     fp32_decided = pre != PF_EMPTY;
                 }
             } else {
-                const Verdict r = judge_box<FAM, DECIDE, flt::NEED_HANDLES>(lo, hi, ord);
+                const Verdict r = judge_box<FAM, DECIDE, flt::NEED_HANDLES>(BoxRef<D>{a.in.lo + i, a.in.hi + i, a.in.cap}, ord);
                 v = r.verdict;
                 handles += r.handles;
             }
@@ -145,116 +259,8 @@ __device__ __forceinline__ void level_step(const LevelArgs& a, size_t j, LevelSm
     level_emit<FAM>(a, sm, v, clipped, fp32_decided, lo, hi, depth, given);
 }
 
-// The end of a level step, for every lane of a warp (all 32 must call it):
-// v = the lane's verdict (-1: no box evaluated), its box lo/hi and depth,
-// given = its split axis for SPLIT_GIVEN.
-// Counts the verdicts, folds the digest and writes the children of every box
-// that is neither proved nor empty (unresolved at the depth limit).
-template <int FAM, int WARPS>
-__device__ __forceinline__ void level_emit(const LevelArgs& a, LevelSmem<WARPS>& sm, int v, bool clipped,
-                                           bool fp32_decided, const double* lo, const double* hi, int depth,
-                                           int given) {
-    constexpr int D = family_dims(FAM);
-    unsigned nchild = 0;
-    int axis = 0;
-    bool unresolved = false;
-    unsigned long long h = 0;  // digest hash of (box, verdict)
-    if (v >= 0) {
-        if (a.digest) h = box_hash<D>(lo, hi, v);
-        if (v != V_PROVED && v != V_EMPTY) {
-            if (depth >= a.max_depth) {
-                unresolved = true;
-            } else {
-                nchild = fanout(a.policy, D);
-                if (a.policy == SPLIT_WIDEST)
-                    axis = widest_axis<D>(lo, hi);
-                else if (a.policy == SPLIT_HYBRID)
-                    axis = hybrid_axis<D>(lo, hi, a.lambda_scale);
-                else if (a.policy == SPLIT_GIVEN)
-                    axis = given;
-            }
-        }
-    }
-    // counts, once per warp (all 32 lanes are here): one shared-memory atomic
-    // per verdict, depth and flag present in the warp instead of one per box
-    {
-        const int lane = threadIdx.x & 31;
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            const unsigned b = __ballot_sync(0xffffffffu, v == k);
-            if (b && lane == 0) atomicAdd(&sm.hist[k], (unsigned long long)__popc(b));
-        }
-        const unsigned bc = __ballot_sync(0xffffffffu, clipped);
-        const unsigned bu = __ballot_sync(0xffffffffu, unresolved);
-        const unsigned bf = __ballot_sync(0xffffffffu, fp32_decided);
-        if (lane == 0) {
-            if (bc) atomicAdd(&sm.hist[C_CLIPPED], (unsigned long long)__popc(bc));
-            if (bu) atomicAdd(&sm.hist[C_UNRESOLVED], (unsigned long long)__popc(bu));
-            if (bf) atomicAdd(&sm.hist[C_FP32], (unsigned long long)__popc(bf));
-        }
-        const int dbin = v >= 0 ? (depth < kDepthBins ? depth : kDepthBins - 1) : -1;
-        const unsigned peers = __match_any_sync(0xffffffffu, dbin);
-        if (dbin >= 0 && lane == __ffs(peers) - 1) atomicAdd(&sm.depth[dbin], (unsigned long long)__popc(peers));
-        if (a.digest) {
-            unsigned long long hs = v >= 0 ? h : 0ull;
-            unsigned long long hx = v >= 0 ? mix64(h ^ 0x5851f42d4c957f2dull) : 0ull;
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                hs += __shfl_xor_sync(0xffffffffu, hs, off);
-                hx ^= __shfl_xor_sync(0xffffffffu, hx, off);
-            }
-            if (lane == 0) {
-                atomicAdd(&sm.dig_sum, hs);
-                atomicXor(&sm.dig_xor, hx);
-            }
-        }
-    }
-    // children: the warp reserves one contiguous range and writes it
-    // cooperatively, lane k of an iteration writing slot k, so every store
-    // of an axis array is one coalesced 256-byte segment per warp
-    unsigned excl, total;
-    const unsigned long long wbase = warp_reserve_range(&a.cnt[C_OUT], nchild, &excl, &total);
-    if (total) {
-        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        if (wbase + total > a.out.cap) {
-            if (lane == 0) atomicOr(&a.cnt[C_ERR], E_OVERFLOW);
-        } else {
-            // slot -> owning lane; the parent box itself comes from the owner by shuffles
-            for (unsigned c = 0; c < nchild; ++c) sm.own[w][excl + c] = (uint8_t)lane;
-            __syncwarp();
-            for (unsigned base = 0; base < total; base += 32) {
-                const unsigned k = base + lane;
-                const bool valid = k < total;
-                const int own = valid ? sm.own[w][k] : 0;
-                double plo[4], phi[4], clo[4], chi[4];
-#pragma unroll
-                for (int d = 0; d < D; ++d) {
-                    plo[d] = __shfl_sync(0xffffffffu, lo[d], own);
-                    phi[d] = __shfl_sync(0xffffffffu, hi[d], own);
-                }
-                const int c = (int)k - (int)__shfl_sync(0xffffffffu, excl, own);
-                const int pax = __shfl_sync(0xffffffffu, axis, own);
-                const int pdep = __shfl_sync(0xffffffffu, depth, own);
-                if (valid) {
-                    make_child<D>(plo, phi, a.policy, pax, c, clo, chi);
-                    const bool alive = clip_child<FAM>(clo, chi, a.tab);
-                    const size_t o = (size_t)(wbase + k);
-#pragma unroll
-                    for (int d = 0; d < D; ++d) {
-                        a.out.lo[d * a.out.cap + o] = clo[d];
-                        a.out.hi[d * a.out.cap + o] = chi[d];
-                    }
-                    a.out.depth[o] = alive ? (uint8_t)(pdep + 1) : (uint8_t)0xFF;
-                }
-            }
-            __syncwarp();
-        }
-    }
-}
-
 // Adds the block's counts to the global counters (after the last step).
-template <int WARPS>
-__device__ __forceinline__ void level_flush(const LevelArgs& a, LevelSmem<WARPS>& sm, unsigned handles) {
+__device__ __forceinline__ void level_flush(const LevelArgs& a, LevelCounts& sm, unsigned handles) {
     for (int off = 16; off > 0; off >>= 1) handles += __shfl_xor_sync(0xffffffffu, handles, off);
     if ((threadIdx.x & 31) == 0 && handles) atomicAdd(&sm.handles, (unsigned long long)handles);
     __syncthreads();

@@ -1065,7 +1065,7 @@ __global__ void __launch_bounds__(128) k_label(LabelArgs a) {
             lo[d] = a.in.lo[d * a.in.cap + i];
             hi[d] = a.in.hi[d * a.in.cap + i];
         }
-        const Verdict v = judge_box<FAM, FULL, flt::NEED_FULL>(lo, hi, 0);
+        const Verdict v = judge_box<FAM, FULL, flt::NEED_FULL>(BoxRef<D>{a.in.lo + i, a.in.hi + i, a.in.cap}, 0);
         if (v.verdict == V_EMPTY) continue;
         int label = -1;
         if (v.verdict == V_CRITICAL) {
@@ -1382,7 +1382,7 @@ cp_status cp_model_net_params(cp_prover* p, int fam, const void** views, const f
 }
 
 cp_status cp_model_collect_chunk(cp_prover* p, int fam, const BoxList& in, size_t begin, size_t count,
-                                 const double* tab_t, const double* tab_v, int tab_n, double tab_h) {
+                                 const double* tab_v, int tab_n, double tab_h) {
     ModelState* m = state(p, false);
     if (!m || !m->collecting || m->rec_family != fam || count == 0) return CP_OK;
     LabelArgs a;
@@ -1392,7 +1392,7 @@ cp_status cp_model_collect_chunk(cp_prover* p, int fam, const BoxList& in, size_
     a.stride = m->rec_stride;
     a.phase = m->rec_phase % m->rec_stride;
     m->rec_phase += 7919;  // vary the sampled residue between chunks
-    a.tab = SingleTable{tab_t, tab_v, tab_n, tab_h};
+    a.tab = SingleTable{tab_v, tab_n, tab_h, 1.0 / tab_h};
     a.feats = m->rec_x;
     a.crit = m->rec_crit;
     a.axis = m->rec_axis;

@@ -30,7 +30,7 @@ namespace {
 constexpr size_t kStaticScratchBytes = size_t(32) << 20;
 constexpr int kTableN = 1 << 16;  // the same grid as the handle's table (cp_create)
 constexpr size_t kCounterBytes = 4096;
-constexpr size_t kTableBytes = 2 * sizeof(double) * kTableN;
+constexpr size_t kTableBytes = sizeof(double) * kTableN;
 constexpr int kMaxDevices = 64;
 
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
@@ -52,10 +52,9 @@ cp_status setup(int dev, cudaStream_t st, unsigned char** base) {
         cudaError_t e = cudaGetSymbolAddress(&p, g_static_scratch);
         if (e != cudaSuccess || !p) return cp_record_cuda_error(e, CP_ERR_CUDA);
         unsigned char* b = (unsigned char*)p;
-        double* t = (double*)(b + kCounterBytes);
-        double* v = t + kTableN;
+        double* v = (double*)(b + kCounterBytes);
         const double h = (cpb::kLambdaMax - cpb::kLambdaMin) / (kTableN - 1);
-        cp_status rc = cp_engine_launch_table(cpb::kLambdaMin, h, kTableN, t, v, st);
+        cp_status rc = cp_engine_launch_table(cpb::kLambdaMin, h, kTableN, v, st);
         if (rc != CP_OK) return rc;
         e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return cp_record_cuda_error(e, CP_ERR_CUDA);
@@ -99,8 +98,7 @@ extern "C" cp_status cp_refine_boxes_static(int family, int precision, int polic
 
     // layout: counters | table | (max_depth + 1) level buffers of equal capacity
     unsigned long long* cnt = (unsigned long long*)base;
-    const double* tab_t = (const double*)(base + kCounterBytes);
-    const double* tab_v = tab_t + kTableN;
+    const double* tab_v = (const double*)(base + kCounterBytes);
     const double tab_h = (cpb::kLambdaMax - cpb::kLambdaMin) / (kTableN - 1);
     const int D = cpb::family_dims(family);
     const int levels = max_depth + 1;
@@ -156,7 +154,7 @@ extern "C" cp_status cp_refine_boxes_static(int family, int precision, int polic
         if (c == 0) return CP_ERR_CAPACITY;
         const size_t begin = cnt_in[l] - c;
         rc = cp_engine_launch_level(family, precision, 0, lv[l], begin, c, last ? nullptr : &lv[l + 1],
-                                    last ? 0ull : (unsigned long long)cnt_in[l + 1], cnt, tab_t, tab_v, kTableN,
+                                    last ? 0ull : (unsigned long long)cnt_in[l + 1], cnt, tab_v, kTableN,
                                     tab_h, policy, max_depth, st);
         if (rc != CP_OK) return rc;
         if ((e = cudaMemcpyAsync(h_cnt, cnt, words * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st)) !=

@@ -27,18 +27,19 @@ enum SplitPolicy : int {
 // used to clip child boxes: the bound is non-increasing in lambda, so the value
 // at the largest grid point t_i <= lambda.lo is an upper bound for the box.
 struct SingleTable {
-    const double* t;  // grid points
     const double* v;  // single_placement(t_i)
     int n;
-    double h;
+    double h, inv_h;
 };
 
 __device__ __forceinline__ double single_upper(const SingleTable& tab, double la_lo) {
-    if (!(la_lo >= tab.t[0])) return 0.25;  // the bisection never exceeds 0.25
-    int i = (int)((la_lo - tab.t[0]) / tab.h);
+    const double t0 = kLambdaMin;
+    if (!(la_lo >= t0)) return 0.25;  // the bisection never exceeds 0.25
+    // the grid points are recomputed as k_single_table fills them, not loaded
+    int i = (int)((la_lo - t0) * tab.inv_h);
     if (i >= tab.n) i = tab.n - 1;
-    while (i > 0 && tab.t[i] > la_lo) --i;
-    while (i + 1 < tab.n && tab.t[i + 1] <= la_lo) ++i;
+    while (i > 0 && __fma_rn((double)i, tab.h, t0) > la_lo) --i;
+    while (i + 1 < tab.n && __fma_rn((double)(i + 1), tab.h, t0) <= la_lo) ++i;
     return tab.v[i];
 }
 
@@ -107,30 +108,19 @@ __device__ __forceinline__ int hybrid_axis(const double* lo, const double* hi, d
 __host__ __device__ constexpr int fanout(int policy, int dims) { return policy == SPLIT_UNIFORM ? (1 << dims) : 2; }
 
 // Writes child c (0 <= c < fanout) of box (lo, hi) split on `axis` (binary
-// policies) or on every axis (uniform).
+// policies) or on every axis (uniform).  No array is indexed by the axis: that
+// would put the boxes into local memory (long-scoreboard stalls of 2 to 5 per issued
+// instruction in the refinement kernels).
 template <int D>
 __device__ __forceinline__ void make_child(const double* lo, const double* hi, int policy, int axis, int c, double* clo,
                                            double* chi) {
+    const bool every = policy == SPLIT_UNIFORM;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-        clo[d] = lo[d];
-        chi[d] = hi[d];
-    }
-    if (policy == SPLIT_UNIFORM) {
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-            const double m = midpoint(lo[d], hi[d]);
-            if ((c >> d) & 1)
-                clo[d] = m;
-            else
-                chi[d] = m;
-        }
-    } else {
-        const double m = midpoint(lo[axis], hi[axis]);
-        if (c & 1)
-            clo[axis] = m;
-        else
-            chi[axis] = m;
+        const double m = midpoint(lo[d], hi[d]);
+        const bool cut = every || axis == d, upper = ((every ? c >> d : c) & 1) != 0;
+        clo[d] = cut && upper ? m : lo[d];
+        chi[d] = cut && !upper ? m : hi[d];
     }
 }
 

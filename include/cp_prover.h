@@ -197,7 +197,7 @@ typedef struct cp_refine_opts {
     int64_t level_capacity; /* boxes per level buffer; 0 = 1<<25 */
     int32_t block;          /* threads per block of the level kernel; 0 = 128 */
     int32_t learned_order;  /* 1 = learned criterion order (needs a trained or loaded model) */
-    int32_t engine;         /* cp_engine: host-driven level loop or one CUDA graph launch */
+    int32_t engine;         /* cp_engine: host-driven level loop, or one launch on the device */
     int32_t boxes_per_thread; /* graph engine: boxes a warp lane takes per claim (1..8); 0 = tuned */
     double lambda_scale;    /* CP_SPLIT_HYBRID: lambda target width scale; 0 = 4e-3 */
     int32_t digest;         /* 1 = compute report->digest (per-box verdict identity checks) */
@@ -211,11 +211,14 @@ typedef struct cp_refine_opts {
 
 /* Refinement engines.  CP_ENGINE_LEVELS: the host picks each chunk, launches
  * the level kernel and reads the counters back (one round trip per chunk).
- * CP_ENGINE_GRAPH: the same schedule runs on the device -- a scheduler kernel
- * and a persistent level kernel (warps claim boxes dynamically) inside a CUDA
- * graph WHILE loop -- so a whole refinement is one graph launch; `block`
- * (64, 128, 256, 512, 1024; 0 = tuned) and boxes_per_thread select the
- * kernel shape.  Both engines produce identical reports. */
+ * CP_ENGINE_GRAPH: the refinement runs
+ * on the device in one kernel launch: every warp refines its boxes depth first from a
+ * stack of its own and shares work with warps that run out (report->launches: kernel
+ * launches, more than 1 only when shared work was left over); `block` (64, 128, 256,
+ * 512, 1024; 0 = tuned) selects the kernel shape, boxes_per_thread the boxes per
+ * claim.  With a learned policy, a scheduler kernel and a persistent level kernel with
+ * the network inline run in a CUDA graph WHILE loop.  Both engines produce identical
+ * reports. */
 typedef enum cp_engine { CP_ENGINE_LEVELS = 0, CP_ENGINE_GRAPH = 1 } cp_engine;
 
 typedef struct cp_refine_report {

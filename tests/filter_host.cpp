@@ -18,7 +18,7 @@ void run(const double* lo, const double* hi, long n, int order, unsigned char* d
         if (b.l1 < b.l2) b.l1 = b.l2;
         FOut o{0, 0};
         const bool empty = b.ll > b.lh || b.l1 > b.h1 || b.l2 > b.h2 || (kThree && b.l3 > b.h3);
-        decided[i] = !empty && filter_box<FAM, NEED>(b, order, o);
+        decided[i] = !empty && filter_box<FAM, NEED>(ValRef{b}, order, o);
         mask[i] = o.mask;
     }
 }
