@@ -50,6 +50,7 @@ __global__ void __launch_bounds__(kEvalBlock, MINB) k_level(RefineArgs r) {
     const unsigned w = threadIdx.x >> 5;
     refine_warp<FAM, PREC, false>(r, sm, wb[w], gridDim.x * kWarps, blockIdx.x * kWarps + w, handles);
     level_flush(r.level, sm, handles);
+    level_end(r.level.cnt);
 }
 
 // The level kernel for refinements in which every box passes through a level:
@@ -64,6 +65,7 @@ __global__ void __launch_bounds__(kEvalBlock) k_level_each(LevelArgs a) {
     for (size_t base = (size_t)blockIdx.x * blockDim.x; base < a.count; base += step)
         level_step<FAM, PREC>(a, base + threadIdx.x, sm, handles);
     level_flush(a, sm, handles);
+    level_end(a.cnt);
 }
 
 // Seed: every box of a family lattice, depth 0.
@@ -102,19 +104,16 @@ __global__ void k_copy_seed(int dims, const double* __restrict__ lo, const doubl
     }
 }
 
-// A chunk of the host-driven loop starts: its children append at `base`, none of
-// its boxes is handed out yet.
-__global__ void k_begin_chunk(unsigned long long* cnt, unsigned long long base) {
-    cnt[C_OUT] = base;
-    cnt[C_CLAIM] = 0;
-}
+// Counters read from a checkpoint: ready for the next chunk (level_end).
+__global__ void k_ready_chunk(unsigned long long* cnt) { cnt[C_OUT] = cnt[C_CLAIM] = cnt[C_DONE] = 0; }
 // A depth-first refinement of `count` seed boxes starts.
-__global__ void k_begin_deep(DeepSched* s, unsigned long long count) {
-    if (threadIdx.x != 0) return;
+// The first ticket of each warp is its number.
+__global__ void k_begin_deep(DeepSched* s, unsigned long long count, unsigned warps) {
     const unsigned long long epoch = s->epoch + 2;  // no flag of an earlier refinement carries this or the one before
     *s = DeepSched{};
     s->epoch = epoch;
     s->count = count;
+    s->ticket = warps;
 }
 __global__ void k_zero_u64(unsigned long long* p, int n) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) p[i] = 0;
@@ -362,13 +361,13 @@ struct cp_prover {
     unsigned long long* deep_flags = nullptr;  // two arrays of kParcels
     MetaList deep_spill{};
     int deep_dims = 0;
-    int graph_variant[6][2] = {{3, 3}, {3, 3}, {3, 3}, {3, 3}, {3, 3}, {3, 3}};  // block-size variant
+    int graph_variant[6][2] = {{3, 4}, {3, 4}, {3, 4}, {3, 4}, {3, 4}, {3, 4}};  // block-size variant
     int graph_bpt[6][2] = {{1, 1}, {1, 1}, {1, 1}, {1, 1}, {1, 1}, {1, 1}};      // boxes per thread
     // an interrupted host-driven refinement: the level stack and counters hold
     // its remaining boxes and partial counts (cp_refine_resume, checkpoints)
     bool pending = false;
     cp_refine_opts pending_opts{};
-    int variant[6][2] = {{2, 1}, {2, 0}, {2, 1}, {2, 1}, {2, 0}, {2, 1}};  // level-kernel variant per family/precision
+    int variant[6][2] = {{2, 3}, {2, 3}, {2, 3}, {2, 3}, {2, 3}, {2, 3}};  // level-kernel variant per family/precision
     // called before every lattice launch of cp_prove_family_reference
     cp_step_callback step_cb = nullptr;
     void* step_user = nullptr;
@@ -498,9 +497,7 @@ LevelEachKernel level_each_kernel(int fam, int prec) {
 constexpr unsigned kClaim = 32;
 // Launches the level kernel over a chunk.  A warp per input box at most: the
 // boxes of a small chunk are spread over the device.
-cp_status launch_level(LevelKernel k, const LevelArgs& a, unsigned long long out_base, cudaStream_t st) {
-    k_begin_chunk<<<1, 1, 0, st>>>(a.cnt, out_base);
-    CP_TRY(cp_check_launch());
+cp_status launch_level(LevelKernel k, const LevelArgs& a, cudaStream_t st) {
     RefineArgs r{};
     r.level = a;
     r.claim = a.cnt + C_CLAIM;
@@ -538,7 +535,7 @@ cp_status cp_engine_launch_table(double lambda_lo, double h, int n, double* v, c
 }
 
 cp_status cp_engine_launch_level(int fam, int prec, int variant, const BoxList& in, size_t begin, size_t count,
-                                 const BoxList* out, unsigned long long out_base, unsigned long long* counters,
+                                 const BoxList* out, unsigned long long* counters,
                                  const double* tab_v, int tab_n, double tab_h, int policy,
                                  int max_depth, cudaStream_t st) {
     LevelArgs a;
@@ -555,11 +552,11 @@ cp_status cp_engine_launch_level(int fam, int prec, int variant, const BoxList& 
     a.axis_hint = nullptr;
     a.order_hint = nullptr;
     a.digest = 0;
-    return launch_level(level_kernel(fam, prec, variant), a, out_base, st);
+    return launch_level(level_kernel(fam, prec, variant), a, st);
 }
 
 bool cp_engine_overflowed(const unsigned long long* h) { return (h[C_ERR] & E_OVERFLOW) != 0; }
-unsigned long long cp_engine_children(const unsigned long long* h) { return h[C_OUT]; }
+unsigned long long cp_engine_children(const unsigned long long* h) { return h[C_CHILDREN]; }
 
 void cp_engine_fill_report(const unsigned long long* h, cp_refine_report* r) {
     for (int v = 0; v < 5; ++v) r->verdicts[v] = (int64_t)h[C_VERDICT + v];
@@ -596,20 +593,17 @@ cp_status cp_engine_eval_chunk(cp_prover* p, int fam, const cp_refine_opts& o, L
     a.axis_hint = axis_hint;
     a.order_hint = order_hint;
     a.digest = o.digest ? 1 : 0;
-    // children append after the boxes already in `out`
-    const unsigned long long base = out ? out->n : 0;
+    // (the deepest non-empty level is taken first, so `out` is empty)
     const int pr = o.precision ? 1 : 0;
     cudaEventRecord(p->ev0, p->stream);
     if (axis_hint || order_hint || cp_model_collecting(p)) {
-        k_begin_chunk<<<1, 1, 0, p->stream>>>(p->cnt, base);
-        CP_TRY(cp_check_launch());
         LevelEachKernel k = level_each_kernel(fam, pr);
         const size_t need = (count + kEvalBlock - 1) / kEvalBlock;
         const unsigned grid = (unsigned)std::min<size_t>(grid_of(k, kEvalBlock), std::max<size_t>(need, 1));
         k<<<grid, kEvalBlock, 0, p->stream>>>(a);
         CP_TRY(cp_check_launch());
     } else {
-        CP_TRY(launch_level(level_kernel(fam, pr, p->variant[fam][pr]), a, base, p->stream));
+        CP_TRY(launch_level(level_kernel(fam, pr, p->variant[fam][pr]), a, p->stream));
     }
     cudaEventRecord(p->ev1, p->stream);
     CP_TRY(read_counters(p));
@@ -617,7 +611,7 @@ cp_status cp_engine_eval_chunk(cp_prover* p, int fam, const cp_refine_opts& o, L
     cudaEventElapsedTime(&t, p->ev0, p->ev1);
     *ms += t;
     if (p->h_cnt[C_ERR] & E_OVERFLOW) return CP_ERR_CAPACITY;
-    if (out) out->n = (size_t)p->h_cnt[C_OUT];
+    if (out) out->n = (size_t)p->h_cnt[C_CHILDREN];
     return CP_OK;
 }
 
@@ -935,7 +929,7 @@ cp_status refine_graph(cp_prover* p, const cp_refine_opts& o, cp_refine_report* 
     a.flags[0] = p->deep_flags;
     a.flags[1] = p->deep_flags + kParcels;
     a.spill = p->deep_spill;
-    k_begin_deep<<<1, 1, 0, p->stream>>>(p->deep_sched, (unsigned long long)n);
+    k_begin_deep<<<1, 1, 0, p->stream>>>(p->deep_sched, (unsigned long long)n, (unsigned)warps);
     CP_TRY(cp_check_launch());
     CP_TRY(cuda_ok(cudaEventRecord(p->ev0, p->stream)));
     do {  // (hardly ever more than one round)
@@ -1553,6 +1547,8 @@ cp_status cp_checkpoint_load(cp_prover* p, const char* path, cp_refine_opts* opt
     CP_TRY(ensure_levels(p, (int)h.nlevels, (int)h.dims, (size_t)h.level_cap));
     std::vector<unsigned char> stage(sizeof(double) * kCkptStage);
     CP_TRY(load(fc.f, p->cnt, h.counter_words, stage, p->stream));
+    k_ready_chunk<<<1, 1, 0, p->stream>>>(p->cnt);
+    CP_TRY(cp_check_launch());
     for (auto& L : p->levels) L.n = 0;
     for (uint32_t l = 0; l < h.nlevels; ++l) {
         if (!n[l]) continue;

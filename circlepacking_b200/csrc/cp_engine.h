@@ -44,7 +44,7 @@ cp_status cp_model_net_params(cp_prover* p, int fam, const void** views, const f
 size_t cp_engine_counter_words();
 cp_status cp_engine_launch_table(double lambda_lo, double h, int n, double* v, cudaStream_t st);
 cp_status cp_engine_launch_level(int fam, int prec, int variant, const cpb::BoxList& in, size_t begin, size_t count,
-                                 const cpb::BoxList* out, unsigned long long out_base, unsigned long long* counters,
+                                 const cpb::BoxList* out, unsigned long long* counters,
                                  const double* tab_v, int tab_n, double tab_h, int policy,
                                  int max_depth, cudaStream_t st);
 // Reads the overflow flag and children count of a counter block copied to the host.

@@ -383,10 +383,18 @@ CPF_HD uint8_t middle_handle(const Ref& ref, bool& ok) {
     const FBox b = ref.load();
     uint8_t m = 0;
     if (fa) {
-        const double c13_lo = INNER ? inner_angle(b.lh, b.l1, b.l3) : outer_angle(b.l1, b.l3);
-        const double c23_hi =
-            INNER ? mixed_hi(b.ll, b.lh, b.h2, b.h3, ok) : mixed_hi(b.ll, b.lh, b.h3, b.h2, ok);
-        if (less_(c13_lo, c12_hi + c23_hi, kTau, ok)) m |= 1;
+        // g1: c13.lo <= (c12 + c23).hi, often by c13.lo <= c13.hi < c12.hi alone
+        bool g1 = c13_hi + kTau < c12_hi;
+        if (!g1) {
+            const double c13_lo = INNER ? inner_angle(b.lh, b.l1, b.l3) : outer_angle(b.l1, b.l3);
+            g1 = c13_lo + kTau < c12_hi;
+            if (!g1) {
+                const double c23_hi =
+                    INNER ? mixed_hi(b.ll, b.lh, b.h2, b.h3, ok) : mixed_hi(b.ll, b.lh, b.h3, b.h2, ok);
+                g1 = less_(c13_lo, c12_hi + c23_hi, kTau, ok);
+            }
+        }
+        if (g1) m |= 1;
         if (NEED != NEED_FULL && m) return m;
     }
     if (fb) {
@@ -427,13 +435,16 @@ CPF_HD bool end2d_fails(const Ref& ref, bool& ok) {
     return less_(lhs, kRatio * fma_(0.5 * rho, other - a_lo, used), tol, ok);
 }
 
-// end_configuration.cu:154-210
+// end_configuration.cu:154-210.  The area test comes first: a handle whose test holds
+// does not fail, whatever its early exit (a12 + a23 definitely at least a13) says.
+// alpha = (a13 + a3).lo - (a12 + a2).hi is at most (a13 + a3).hi - a2.hi, which often
+// shows the failure without a12.
 template <bool INNER, class Ref>
 CPF_HD bool end3d_fails(const Ref& ref, bool& ok) {
     double a13_hi;
     {
         const FBox b = ref.load();
-        double s_lo;
+        const Terms t(b);
         if (INNER) {
             ok = ok && clear_same(b.h1, b.h3, sides_inner(b.ll, b.h1, b.h3)) &&
                  clear_same_low(b.l1, b.l3, sides_inner(b.lh, b.l1, b.l3)) && clear_mixed_hi(b.ll, b.lh, b.h2, b.h1) &&
@@ -441,7 +452,6 @@ CPF_HD bool end3d_fails(const Ref& ref, bool& ok) {
                  clear_mixed_lo(b.ll, b.l2, b.l3);
             if (!ok) return false;
             a13_hi = inner_angle(b.ll, b.h1, b.h3);
-            s_lo = mixed_lo(b.ll, b.lh, b.l2, b.l1, ok) + mixed_lo(b.ll, b.lh, b.l2, b.l3, ok);
         } else {
             ok = ok && clear_same(b.h1, b.h3, sides_outer(b.h1, b.h3)) &&
                  clear_same_low(b.l1, b.l3, sides_outer(b.l1, b.l3)) && clear_mixed_hi(b.ll, b.lh, b.h1, b.h2) &&
@@ -449,26 +459,27 @@ CPF_HD bool end3d_fails(const Ref& ref, bool& ok) {
                  clear_mixed_lo(b.ll, b.l3, b.l2);
             if (!ok) return false;
             a13_hi = outer_angle(b.h1, b.h3);
-            s_lo = mixed_lo(b.ll, b.lh, b.l1, b.l2, ok) + mixed_lo(b.ll, b.lh, b.l3, b.l2, ok);
         }
-        if (less_(a13_hi, s_lo, kTau, ok)) return false;
+        const double a3_hi = INNER ? semi_inner(b.ll, b.h3) : semi_outer(b.h3);
+        const double a2_hi = INNER ? semi_outer(b.h2) : semi_inner(b.ll, b.h2);
+        const double q = INNER ? fma_(2.0, b.h3, b.lh) : 1.0 - 2.0 * b.h3;
+        double rho = INNER ? 1.0 - q * q : q * q - b.lh * b.lh;
+        if (rho < 0.0) rho = 0.0;
+        const double top = a13_hi + a3_hi, used = 0.5 * t.ratio * top;
+        const double lhs = fma_(0.5, disk_area(b.l1), disk_area(b.l2) + disk_area(b.l3));
+        if (lhs - kRatio * fma_(-0.5 * rho, top - a2_hi, used) >= -t.tol) {
+            const double a13_lo = INNER ? inner_angle(b.lh, b.l1, b.l3) : outer_angle(b.l1, b.l3);
+            const double a12_hi = INNER ? mixed_hi(b.ll, b.lh, b.h2, b.h1, ok) : mixed_hi(b.ll, b.lh, b.h1, b.h2, ok);
+            const double a3_lo = INNER ? semi_inner(b.lh, b.l3) : semi_outer(b.l3);
+            const double alpha = (a13_lo + a3_lo) - (a12_hi + a2_hi);
+            const double tol = b.l3 < kMinB ? fma_(0.5 * kLowSlack, rho, t.tol) : t.tol;
+            if (!less_(lhs, kRatio * fma_(-0.5 * rho, alpha, used), tol, ok) || !ok) return false;
+        }
     }
     const FBox b = ref.load();
-    const Terms t(b);
-    const double a13_lo = INNER ? inner_angle(b.lh, b.l1, b.l3) : outer_angle(b.l1, b.l3);
-    const double a12_hi = INNER ? mixed_hi(b.ll, b.lh, b.h2, b.h1, ok) : mixed_hi(b.ll, b.lh, b.h1, b.h2, ok);
-    const double a3_lo = INNER ? semi_inner(b.lh, b.l3) : semi_outer(b.l3);
-    const double a3_hi = INNER ? semi_inner(b.ll, b.h3) : semi_outer(b.h3);
-    const double a2_hi = INNER ? semi_outer(b.h2) : semi_inner(b.ll, b.h2);
-    const double q = INNER ? fma_(2.0, b.h3, b.lh) : 1.0 - 2.0 * b.h3;
-    double rho = INNER ? 1.0 - q * q : q * q - b.lh * b.lh;
-    if (rho < 0.0) rho = 0.0;
-    const double alpha = (a13_lo + a3_lo) - (a12_hi + a2_hi);
-    const double used = 0.5 * t.ratio * (a13_hi + a3_hi);
-    double tol = t.tol;
-    if (b.l3 < kMinB) tol = fma_(0.5 * kLowSlack, rho, tol);
-    const double lhs = fma_(0.5, disk_area(b.l1), disk_area(b.l2) + disk_area(b.l3));
-    return less_(lhs, kRatio * fma_(-0.5 * rho, alpha, used), tol, ok);
+    const double s_lo = INNER ? mixed_lo(b.ll, b.lh, b.l2, b.l1, ok) + mixed_lo(b.ll, b.lh, b.l2, b.l3, ok)
+                              : mixed_lo(b.ll, b.lh, b.l1, b.l2, ok) + mixed_lo(b.ll, b.lh, b.l3, b.l2, ok);
+    return !less_(a13_hi, s_lo, kTau, ok);
 }
 
 // start_configuration.cu:126-162.  Criterion 1 is evaluated when a12 + a23 > a13
@@ -498,18 +509,28 @@ CPF_HD bool start_box(const Ref& ref, FOut& o) {
         return true;
     }
     if (NEED != NEED_HANDLES && !f1 && !f2) return true;
+    // a13.lo <= a13.hi < a12.hi <= (a12 + a23).hi: "possibly" without a13.lo and a23
+    bool pos = a13_hi + kTau < a12_hi, def = false;
+    if (pos && f1 && !f2) {
+        o.mask = 1;
+        return true;
+    }
     const FBox b = ref.load();
-    bool pos = true, def = false;
-    if (f2 || NEED == NEED_HANDLES) {
+    if (f2 || (NEED == NEED_HANDLES && !f1)) {
         def = less_(a13_hi, mixed_lo(b.ll, b.lh, b.l1, b.l2, ok) + mixed_lo(b.ll, b.lh, b.l3, b.l2, ok), kTau, ok);
         if (!ok) return false;
+        if (def) pos = true;
     }
-    if ((f1 || NEED == NEED_HANDLES) && !def)
-        pos = less_(outer_angle(b.l1, b.l3), a12_hi + mixed_hi(b.ll, b.lh, b.h3, b.h2, ok), kTau, ok);
+    if ((f1 || NEED == NEED_HANDLES) && !pos) {
+        const double a13_lo = outer_angle(b.l1, b.l3);
+        pos = a13_lo + kTau < a12_hi;
+        if (!pos) pos = less_(a13_lo, a12_hi + mixed_hi(b.ll, b.lh, b.h3, b.h2, ok), kTau, ok);
+    }
     if (pos && f1) o.mask |= 1;
     if (NEED != NEED_FULL && o.mask) return ok;
     if (!def && f2) o.mask |= 2;
-    o.handles = (pos ? 1 : 0) + (def ? 0 : 1);
+    // (where only criterion 1 fails, one is evaluated: it, or criterion 2)
+    if (!f1) o.handles = (pos ? 1 : 0) + (def ? 0 : 1);
     return ok;
 }
 

@@ -49,7 +49,8 @@ __global__ void __launch_bounds__(deep_threads(BLOCK)) __maxnreg__(deep_regs(BLO
     s.left = left;
     s.epoch += 1;
     s.inputs = parcels < kParcels ? parcels : kParcels;
-    s.ticket = s.parcels = s.filled = s.taken = s.idle = s.done = 0;
+    s.ticket = gridDim.x * kWarps;
+    s.parcels = s.filled = s.taken = s.idle = s.done = 0;
 }
 
 struct PersistArgs {

@@ -21,11 +21,13 @@ enum : int {
     C_OUT = 8,      // children appended
     C_ERR = 9,      // error flags
     C_BEST_SLAB = 10,
-    C_CLAIM = C_BEST_SLAB,  // in a refinement: boxes of the chunk handed to warps
+    C_CLAIM = C_BEST_SLAB,  // in a host-driven refinement: boxes of the chunk handed to warps
     C_EVALUATED = 11,
     C_FIRST_BITS = 12,  // ordered encoding of the smallest failing lambda.lb
     C_ERRBOX_CLAIM = 13,
+    C_DONE = C_ERRBOX_CLAIM,  // in a host-driven refinement: blocks of the chunk finished
     C_ERRBOX = 14,      // 8 slots: lo/hi of the first erroneous box
+    C_CHILDREN = C_ERRBOX,    // in a host-driven refinement: children the last chunk appended
     C_COLLECT = 22,
     C_NOFIT_SLAB = 23,  // smallest lambda slab holding a box whose fit check fired (middle/end)
     C_TRAP_SLAB = 24,   // smallest lambda slab holding a box that reached a trap site
@@ -95,12 +97,15 @@ __device__ __forceinline__ void level_smem_init(LevelCounts& sm) {
     }
 }
 
+__device__ __forceinline__ unsigned long long digest_xor_word(unsigned long long h) {
+    return mix64(h ^ 0x5851f42d4c957f2dull);
+}
 // Folds a warp's evaluated boxes (v >= 0) into the block's digest words.
 template <int D>
 __device__ __forceinline__ void digest_step(LevelCounts& sm, int v, const double* lo, const double* hi) {
     const unsigned long long h = v >= 0 ? box_hash<D>(lo, hi, v) : 0ull;
     unsigned long long hs = h;
-    unsigned long long hx = v >= 0 ? mix64(h ^ 0x5851f42d4c957f2dull) : 0ull;
+    unsigned long long hx = v >= 0 ? digest_xor_word(h) : 0ull;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         hs += __shfl_xor_sync(0xffffffffu, hs, off);
@@ -273,6 +278,18 @@ __device__ __forceinline__ void level_flush(const LevelArgs& a, LevelCounts& sm,
     }
     for (int t = threadIdx.x; t < kDepthBins; t += blockDim.x)
         if (sm.depth[t]) atomicAdd(&a.per_depth[t], sm.depth[t]);
+}
+
+// Ends a chunk of the host-driven loop, after level_flush: the last block leaves the
+// number of children for the host and the counters ready for the next chunk, whose
+// launch then needs no preparation.
+__device__ __forceinline__ void level_end(unsigned long long* cnt) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x != 0 || atomicAdd(&cnt[C_DONE], 1ull) + 1ull != gridDim.x) return;
+    __threadfence();
+    cnt[C_CHILDREN] = *(volatile unsigned long long*)&cnt[C_OUT];
+    cnt[C_OUT] = cnt[C_CLAIM] = cnt[C_DONE] = 0;
 }
 
 }  // namespace cpb

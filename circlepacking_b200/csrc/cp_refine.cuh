@@ -43,6 +43,7 @@ template <int D>
 struct WarpBoxes {
     double plo[D][kParents], phi[D][kParents];
     double rlo[D][kReady], rhi[D][kReady];
+    unsigned long long dig_sum[32], dig_xor[32];  // digest words per lane
     uint32_t pmeta[kParents];  // depth | axis << 8
     uint32_t rdepth[kReady];
 };
@@ -161,34 +162,28 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
     const unsigned lane = threadIdx.x & 31, full = 0xffffffffu;
     const int flog = a.policy == SPLIT_UNIFORM ? D : 1;  // log2 of the children per parent
     const unsigned group = 32u >> flog;                  // parents that fill a warp
-    unsigned long long count = a.count, epoch = 0;
-    unsigned round = 0, inputs = 0, ticket = 0;
-    bool drawn = false;  // DEEP: `ticket` has been drawn and not used up
-    MetaList in{}, out{};
-    unsigned long long *in_flag = nullptr, *out_flag = nullptr;
-    if (DEEP) {
-        round = r.sched->rounds;
-        count = r.sched->count;
-        epoch = r.sched->epoch;
-        in = r.lists[(round + 1) & 1];
-        out = r.lists[round & 1];
-        in_flag = r.flags[(round + 1) & 1];
-        out_flag = r.flags[round & 1];
+    unsigned round = 0, inputs = 0, ticket = warp_id, per;
+    bool drawn = DEEP;  // DEEP: `ticket` has been drawn and not used up
+    {
+        // small inputs are spread over all warps
+        const unsigned long long count = DEEP ? r.sched->count : a.count, share = (count + nwarps - 1) / nwarps;
+        per = share < r.per ? (unsigned)(share ? share : 1) : r.per;
+        if (DEEP) {
+            round = r.sched->rounds;
+            inputs = round ? r.sched->inputs : (unsigned)((count + per - 1) / per);
+        }
     }
-    // small inputs are spread over all warps
-    const unsigned long long share = (count + nwarps - 1) / nwarps;
-    const unsigned per = share < r.per ? (unsigned)(share ? share : 1) : r.per;
-    if (DEEP) inputs = round ? r.sched->inputs : (unsigned)((count + per - 1) / per);
     unsigned long long cur = 0, end = 0;
     bool more = true;
+    if (!DEEP) {  // the first pieces are the warps' by number
+        cur = (unsigned long long)warp_id * per;
+        end = cur + per < a.count ? cur + per : a.count;
+        more = a.count > (unsigned long long)nwarps * per;
+    }
     unsigned np = 0, nr = 0, nspill = 0, nclip = 0;
     WarpTally t;
+    wb.dig_sum[lane] = wb.dig_xor[lane] = 0;
     for (;;) {
-        unsigned wanted = 0, given = 0;  // read here, used after the step
-        if (DEEP) {
-            wanted = *(volatile unsigned*)&r.sched->ticket;
-            given = *(volatile unsigned*)&r.sched->parcels;
-        }
         const bool strict = DEEP && nspill >= r.strict;  // evaluate the next children made, and nothing else
         unsigned made = 0;
         while (nr < 32 && !(strict && made)) {
@@ -244,9 +239,9 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
             } else if (!DEEP && more) {
                 unsigned long long start = 0;
                 if (lane == 0) start = atomicAdd(r.claim, (unsigned long long)per);
-                cur = __shfl_sync(full, start, 0);
-                more = cur < count;
-                end = !more ? cur : cur + per < count ? cur + per : count;
+                cur = __shfl_sync(full, start, 0) + (unsigned long long)nwarps * per;
+                more = cur < a.count;
+                end = !more ? cur : cur + per < a.count ? cur + per : a.count;
                 continue;
             } else if (DEEP && more) {
                 if (!drawn) {
@@ -262,6 +257,7 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
                     drawn = true;
                 }
                 if (ticket < inputs && round == 0) {
+                    const unsigned long long count = r.sched->count;
                     cur = (unsigned long long)ticket * per;
                     end = cur + per < count ? cur + per : count;
                     drawn = false;
@@ -272,17 +268,17 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
                 unsigned long long* flag;
                 if (!given_now) {  // a parcel left over from the last round
                     p = ticket;
-                    flag = in_flag + p;
+                    flag = r.flags[(round + 1) & 1] + p;
                     const unsigned long long f = *(volatile unsigned long long*)flag;
-                    n = f >> 40 == ((epoch - 1) & 0xFFFFFFull) && (f & 0xFF) != kParcelTaken ? (unsigned)(f & 0xFF) : 0u;
+                    n = f >> 40 == ((r.sched->epoch - 1) & 0xFFFFFFull) && (f & 0xFF) != kParcelTaken ? (unsigned)(f & 0xFF) : 0u;
                     n = __shfl_sync(full, n, 0);
                     drawn = false;
                     if (n == 0) continue;
                 } else {
                     if (nr > 0) break;  // (the last input went to another warp meanwhile)
-                    const unsigned long long tag = parcel_tag(epoch, ticket - inputs);
+                    const unsigned long long tag = parcel_tag(r.sched->epoch, ticket - inputs);
                     p = (ticket - inputs) % kParcels;
-                    flag = out_flag + p;
+                    flag = r.flags[round & 1] + p;
                     if (lane == 0) {
                         atomicAdd(&r.sched->idle, 1u);
                         for (int k = 0; k < kWaitPolls; ++k) {
@@ -302,7 +298,7 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
                     }
                     drawn = false;
                 }
-                const MetaList& from = given_now ? out : in;
+                const MetaList& from = r.lists[(given_now ? round : round + 1) & 1];
                 __threadfence();
                 if (lane < n) {
                     const size_t e = (size_t)p * 32 + lane;
@@ -381,7 +377,11 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
         if (a.digest) {
             double lo[4], hi[4];
             box_copy<D>(box, lo, hi);
-            digest_step<D>(sm, v, lo, hi);
+            if (v >= 0) {
+                const unsigned long long h = box_hash<D>(lo, hi, v);
+                wb.dig_sum[lane] += h;
+                wb.dig_xor[lane] ^= digest_xor_word(h);
+            }
         }
         if (!__any_sync(full, split)) {
             if (!DEEP) continue;
@@ -424,27 +424,30 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
             if constexpr (!DEEP)
                 emit_children<FAM>(a, sm, lo, hi, depth, axis, split && !local ? 1u << flog : 0u);
         }
-        if (DEEP && np + nspill >= kMinGive) {
+        if (DEEP && np + nspill >= kMinGive && (t.steps & 3u) == 0) {
             // more tickets than parcels: give parents away, the older ones.  About four
-            // warps per missing parcel do so at a time (a hash of warp and step picks them).
-            const unsigned missing = wanted - inputs - given;  // (wraps when tickets are input still)
+            // warps per missing parcel do so at a time (a hash of warp and step picks
+            // them), those with small stacks only when an eighth of the warps is waiting.
+            const unsigned wanted = *(volatile unsigned*)&r.sched->ticket, given = *(volatile unsigned*)&r.sched->parcels;
+            const unsigned missing = wanted > inputs + given ? wanted - inputs - given : 0u;
             const unsigned pick = (warp_id * 2654435761u + t.steps * 0x9E3779B9u) >> 16;
-            bool give = wanted > inputs + given &&
-                        (unsigned long long)pick * nwarps < (unsigned long long)missing * (4u << 16);
+            bool give = (unsigned long long)pick * nwarps < (unsigned long long)missing * (4u << 16) &&
+                        (np + nspill >= 48 || missing * 8u > nwarps);
             give = __shfl_sync(full, (int)give, 0) != 0;
             unsigned d = 0, n = 0;
             bool room = false;  // the slot's last parcel has been taken
             if (give) {
                 if (lane == 0) {
                     d = atomicAdd(&r.sched->parcels, 1u);
-                    const unsigned long long f = *(volatile unsigned long long*)(out_flag + d % kParcels);
-                    room = f >> 40 != (epoch & 0xFFFFFFull) || (f & 0xFF) == kParcelTaken;
+                    const unsigned long long f = *(volatile unsigned long long*)(r.flags[round & 1] + d % kParcels);
+                    room = f >> 40 != (r.sched->epoch & 0xFFFFFFull) || (f & 0xFF) == kParcelTaken;
                 }
                 d = __shfl_sync(full, d, 0);
                 room = __shfl_sync(full, (int)room, 0) != 0;
             }
             if (room) {
                 const unsigned p = d % kParcels;
+                const MetaList& out = r.lists[round & 1];
                 const size_t o = (size_t)p * 32 + lane;
                 if (nspill >= 32) {
                     n = 32;
@@ -508,7 +511,7 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
                 __threadfence();
                 __syncwarp();
                 if (lane == 0) {
-                    atomicExch(out_flag + p, parcel_tag(epoch, d) << 8 | n);
+                    atomicExch(r.flags[round & 1] + p, parcel_tag(r.sched->epoch, d) << 8 | n);
                     atomicAdd(&r.sched->filled, 1u);
                 }
             }
@@ -517,6 +520,10 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
     }
     tally_flush(t, sm);
     tally_run(t, sm);
+    if (a.digest) {
+        atomicAdd(&sm.dig_sum, wb.dig_sum[lane]);
+        atomicXor(&sm.dig_xor, wb.dig_xor[lane]);
+    }
     if (PREC == CP_FP32_PREFILTER) {
         const unsigned n = __reduce_add_sync(full, t.fp32);
         if (lane == 0 && n) atomicAdd(&sm.hist[C_FP32], (unsigned long long)n);
