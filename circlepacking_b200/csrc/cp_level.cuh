@@ -75,7 +75,7 @@ __device__ __forceinline__ unsigned long long box_hash(const double* lo, const d
 }
 
 // Per-block shared state of the level step: counts, and for kernels that append
-// children to a level (WARPS > 0) the lane owning each slot of a warp's children.
+// children to a level (WARPS > 0) the lanes whose boxes are split.
 struct LevelCounts {
     unsigned long long hist[8];
     unsigned long long depth[kDepthBins];
@@ -84,7 +84,7 @@ struct LevelCounts {
 };
 template <int WARPS>
 struct LevelSmem : LevelCounts {
-    uint8_t own[WARPS][32 * 16];
+    uint8_t own[WARPS][32];
 };
 
 __device__ __forceinline__ void level_smem_init(LevelCounts& sm) {
@@ -170,13 +170,16 @@ __device__ __forceinline__ void emit_children(const LevelArgs& a, LevelSmem<WARP
         if (lane == 0) atomicOr(&a.cnt[C_ERR], E_OVERFLOW);
         return;
     }
-    // slot -> owning lane; the parent box itself comes from the owner by shuffles
-    for (unsigned c = 0; c < nchild; ++c) sm.own[w][excl + c] = (uint8_t)lane;
+    // slot -> owning lane: all owners have 2^flog children; the parent box itself comes
+    // from the owner by shuffles.  (A byte per owner, not per slot: with 512 B a warp the
+    // level kernel's five blocks took the next larger shared-memory carveout from the L1.)
+    const int flog = a.policy == SPLIT_UNIFORM ? D : 1;
+    if (nchild) sm.own[w][excl >> flog] = (uint8_t)lane;
     __syncwarp();
     for (unsigned base = 0; base < total; base += 32) {
         const unsigned k = base + lane;
         const bool valid = k < total;
-        const int own = valid ? sm.own[w][k] : 0;
+        const int own = valid ? sm.own[w][k >> flog] : 0;
         double plo[4], phi[4], clo[4], chi[4];
 #pragma unroll
         for (int d = 0; d < D; ++d) {

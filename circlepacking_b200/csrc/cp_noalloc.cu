@@ -153,7 +153,7 @@ extern "C" cp_status cp_refine_boxes_static(int family, int precision, int polic
         if (!last) c = std::min(c, (cap - cnt_in[l + 1]) / (size_t)F);
         if (c == 0) return CP_ERR_CAPACITY;
         const size_t begin = cnt_in[l] - c;
-        rc = cp_engine_launch_level(family, precision, precision ? 3 : 2, lv[l], begin, c, last ? nullptr : &lv[l + 1],
+        rc = cp_engine_launch_level(family, precision, 0, lv[l], begin, c, last ? nullptr : &lv[l + 1],
                                     cnt, tab_v, kTableN,
                                     tab_h, policy, max_depth, st);
         if (rc != CP_OK) return rc;
