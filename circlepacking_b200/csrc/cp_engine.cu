@@ -361,13 +361,13 @@ struct cp_prover {
     unsigned long long* deep_flags = nullptr;  // two arrays of kParcels
     MetaList deep_spill{};
     int deep_dims = 0;
-    int graph_variant[6][2] = {{3, 4}, {3, 4}, {3, 4}, {3, 4}, {3, 4}, {3, 4}};  // block-size variant
+    int graph_variant[6][2] = {{3, 4}, {3, 3}, {3, 4}, {3, 0}, {3, 3}, {3, 3}};  // block-size variant
     int graph_bpt[6][2] = {{1, 1}, {1, 1}, {1, 1}, {1, 1}, {1, 1}, {1, 1}};      // boxes per thread
     // an interrupted host-driven refinement: the level stack and counters hold
     // its remaining boxes and partial counts (cp_refine_resume, checkpoints)
     bool pending = false;
     cp_refine_opts pending_opts{};
-    int variant[6][2] = {{2, 3}, {2, 3}, {2, 3}, {2, 3}, {2, 3}, {2, 3}};  // level-kernel variant per family/precision
+    int variant[6][2] = {{2, 3}, {2, 3}, {2, 3}, {2, 2}, {2, 3}, {2, 3}};  // level-kernel variant per family/precision
     // called before every lattice launch of cp_prove_family_reference
     cp_step_callback step_cb = nullptr;
     void* step_user = nullptr;

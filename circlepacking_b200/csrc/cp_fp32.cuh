@@ -354,6 +354,93 @@ __device__ __forceinline__ E collision(EI L, EI S, EI ab, bool& ok) {
     return r.v;
 }
 
+// The same chain where the longer side is a point P, the shorter an interval [Ql, Qh]
+// of positive bounds with Qh <= P (certified: Qh.u <= P.l; two disks on one border:
+// Ql = Qh and P >= Q in every bound), and the sum of the radii a point C.  Bit for bit
+// collision_body's result wherever that keeps `ok`:
+//   * the two clamps at its head change nothing, squares and quotients of positive
+//     bounds take one case each, P^2 - Q^2 > 0 (else the general chain runs);
+//   * definitely obtuse, or definitely not: every emptiness and domain test must come
+//     out false to keep `ok`, and RU(x / y) <= 1 is x <= y, so the quotients that only
+//     such tests read are not formed (4 of 6; of a point all coincide);
+//   * possibly, not definitely obtuse (an interval only): both angles and their join,
+//     where the obtuse part's quotients are at most 1 once it is not empty.
+// Most of the shadow's time goes into these chains, and most of theirs into the
+// directed quotients and arcsines, calls one and all.
+template <bool POINT>
+__device__ __forceinline__ E collision_fast_body(E P, E Ql, E Qh, E C, const int W, bool& ok, bool& general) {
+    const bool HI = (W == W_HI);
+    general = false;
+    if (!(Ql.l > 0.f && C.l > 0.f)) {
+        ok = false;
+        return ek(0.f);
+    }
+    const E zero = ek(0.f), half = ek(0.5f);
+    const E p2 = emul(P, P), c2 = emul(C, C), ql2 = emul(Ql, Ql), qh2 = POINT ? ql2 : emul(Qh, Qh);
+    const bool obt_def = clt(eadd(qh2, c2), p2, ok);
+    const bool obt_pos = POINT ? obt_def : clt(eadd(ql2, c2), p2, ok);
+    const E dl = esub(p2, qh2);
+    general = ok && !(dl.l > 0.f);
+    if (!ok || general) return zero;
+    const E al = ediv(dl, C, ok), ah = POINT ? al : ediv(esub(p2, ql2), C, ok);
+    const E lxl = emul(half, eadd(al, C)), lxh = POINT ? lxl : emul(half, eadd(ah, C));
+    if (obt_def) {
+        const E xl = esub(al, C), xh = POINT ? xl : esub(ah, C);
+        const E sxl{__fmul_rd(xl.l, 0.5f), __fmul_ru(xl.u, 0.5f)}, sxh{__fmul_rd(xh.l, 0.5f), __fmul_ru(xh.u, 0.5f)};
+        ok = sxh.l >= 0.f && Qh.l >= sxl.u && P.l >= lxl.u;
+        if (!ok || W == W_TRAP) return zero;
+        if (HI) return esub(easin(emin(ediv(emin(lxh, P), P, ok), ek(1.f)), ok), easin(ediv(emax(sxl, zero), Qh, ok), ok));
+        return emax(esub(easin(ediv(lxl, P, ok), ok), easin(emin(ediv(emin(sxh, Qh), Ql, ok), ek(1.f)), ok)), zero);
+    }
+    E ob = ek(HI ? -1.f : 0.f);
+    int nonempty = T_FALSE;
+    if (!POINT && obt_pos) {
+        const E xl = esub(al, C), xh = esub(ah, C);
+        const E sxl{__fmul_rd(xl.l, 0.5f), __fmul_ru(xl.u, 0.5f)}, sxh{__fmul_rd(xh.l, 0.5f), __fmul_ru(xh.u, 0.5f)};
+        const bool e = clt(sxh, zero, ok) || clt(Qh, sxl, ok) || clt(P, lxl, ok);
+        if (!ok) return zero;
+        if (!e && W != W_TRAP) {
+            const E lqh = emin(ediv(emin(lxh, P), P, ok), ek(1.f)), sql = ediv(emax(sxl, zero), Qh, ok);
+            if (HI) {
+                ob = esub(easin(lqh, ok), easin(sql, ok));
+                nonempty = tnot(tlt(ob, zero));
+            } else {
+                ob = emax(esub(easin(ediv(lxl, P, ok), ok), easin(emin(ediv(emin(sxh, Qh), Ql, ok), ek(1.f)), ok)), zero);
+                nonempty = tle(sql, lqh);
+                if (nonempty != T_TRUE)
+                    nonempty = tor(nonempty, tnot(tlt(esub(easin(lqh, ok), easin(sql, ok)), zero)));
+            }
+        }
+    }
+    const E xl = esub(C, ah), xh = POINT ? xl : esub(C, al);
+    const E sxl{__fmul_rd(xl.l, 0.5f), __fmul_ru(xl.u, 0.5f)}, sxh{__fmul_rd(xh.l, 0.5f), __fmul_ru(xh.u, 0.5f)};
+    const bool e5 = clt(sxh, zero, ok);
+    if (e5) {
+        if (!obt_pos) ok = false;
+        return ob;
+    }
+    ok = ok && lxh.u <= P.l && sxh.u <= Ql.l;
+    if (!ok || W == W_TRAP) return zero;
+    const E r = HI ? eadd(easin(ediv(lxh, P, ok), ok), easin(ediv(sxh, Ql, ok), ok))
+                   : eadd(easin(ediv(lxl, P, ok), ok), emax(easin(ediv(emax(sxl, zero), Qh, ok), ok), zero));
+    const E joined = HI ? emax(ob, r) : emin(ob, r);
+    return nonempty == T_TRUE ? joined : nonempty == T_FALSE ? r : hull(joined, r);
+}
+// one copy each of the two shapes, for all three Wants
+template <bool POINT>
+__device__ __noinline__ EOk collision_fast_call(E P, E Ql, E Qh, E C, int W) {
+    bool ok = true, general;
+    const E v = collision_fast_body<POINT>(P, Ql, Qh, C, W, ok, general);
+    if (general) return collision_call(ept(P), EI{Ql, Qh}, ept(C), W);
+    return {v, ok};
+}
+template <int W, bool POINT>
+__device__ __forceinline__ E collision_fast(E P, E Ql, E Qh, E C, bool& ok) {
+    const EOk r = collision_fast_call<POINT>(P, Ql, Qh, C, W);
+    ok = ok && r.ok;
+    return r.v;
+}
+
 // corner wrappers (shadows of cp_fp64.cuh); LOC = lower-bound corner, which
 // returns 0 when the radii sum is not positive (collision_angles.cu:131-137, 222-228)
 // ra, rb: the exact FP64 corner radii; ra >= rb makes the corner intervals
@@ -361,18 +448,18 @@ __device__ __forceinline__ E collision(EI L, EI S, EI ab, bool& ok) {
 template <int W, bool LOC>
 __device__ __forceinline__ E ca_ii_corner(double la, double ra, double rb, bool& ok) {
     const E eR = ec(ra), eS = ec(rb), eL = ec(la);
-    EI lc = ept(eadd(eR, eL)), sc = ept(eadd(eS, eL)), ab = ept(eadd(eR, eS));
-    if (LOC && cle(ab.lo, ek(0.f), ok)) return ek(0.f);
+    const E lc = eadd(eR, eL), sc = eadd(eS, eL), ab = eadd(eR, eS);
+    if (LOC && cle(ab, ek(0.f), ok)) return ek(0.f);
     if (!(ra >= rb)) ok = false;
-    return collision<W>(lc, sc, ab, ok);
+    return collision_fast<W, true>(lc, sc, sc, ab, ok);
 }
 template <int W, bool LOC>
 __device__ __forceinline__ E ca_oo_corner(double ra, double rb, bool& ok) {
     const E eR = ec(ra), eS = ec(rb);
-    EI lc = ept(esub(ek(1.f), eS)), sc = ept(esub(ek(1.f), eR)), ab = ept(eadd(eR, eS));
-    if (LOC && cle(ab.lo, ek(0.f), ok)) return ek(0.f);
+    const E lc = esub(ek(1.f), eS), sc = esub(ek(1.f), eR), ab = eadd(eR, eS);
+    if (LOC && cle(ab, ek(0.f), ok)) return ek(0.f);
     if (!(ra >= rb)) ok = false;
-    return collision<W>(lc, sc, ab, ok);
+    return collision_fast<W, true>(lc, sc, sc, ab, ok);
 }
 template <int W, bool OUTER_FIRST>
 __device__ __forceinline__ E ca_mixed_corner(EI la, E a, E b, bool& ok) {
@@ -387,6 +474,11 @@ __device__ __forceinline__ E ca_mixed_corner(EI la, E a, E b, bool& ok) {
     EI ab = ept(eadd(a, b));
     const bool def_ca_longer = cle(cb.hi, ca.lo, ok);
     const bool pos_ca_longer = cle(cb.lo, ca.hi, ok);
+    if (OUTER_FIRST ? def_ca_longer : !def_ca_longer && !pos_ca_longer) {
+        // the outer disk's point is the longer side, nearly always
+        return OUTER_FIRST ? collision_fast<W, false>(ca.lo, cb.lo, cb.hi, ab.lo, ok)
+                           : collision_fast<W, false>(cb.lo, ca.lo, ca.hi, ab.lo, ok);
+    }
     if (def_ca_longer) return collision<W>(ca, cb, ab, ok);
     if (!pos_ca_longer) return collision<W>(cb, ca, ab, ok);
     const E r1 = collision<W>(ca, cb, ab, ok);

@@ -88,7 +88,10 @@ constexpr unsigned kParcelTaken = 0xFF;
 __device__ __forceinline__ unsigned long long parcel_tag(unsigned long long epoch, unsigned d) {
     return (epoch & 0xFFFFFFull) << 32 | d;
 }
-constexpr unsigned kMinGive = 8;                 // a warp with fewer parents keeps them
+// A warp with fewer parents keeps them.  FP32: its steps take ten times as long, so
+// that warps give from small stacks too and look after every step.
+template <int PREC>
+constexpr unsigned kMinGive = PREC == CP_FP32_PREFILTER ? 4 : 8;
 constexpr int kWaitPolls = 1 << 17, kWaitNs = 200;  // a wait ends after some 30 ms
 
 struct RefineArgs {
@@ -424,7 +427,8 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
             if constexpr (!DEEP)
                 emit_children<FAM>(a, sm, lo, hi, depth, axis, split && !local ? 1u << flog : 0u);
         }
-        if (DEEP && np + nspill >= kMinGive && (t.steps & 3u) == 0) {
+        constexpr bool eager = PREC == CP_FP32_PREFILTER;
+        if (DEEP && np + nspill >= kMinGive<PREC> && (eager || (t.steps & 3u) == 0)) {
             // more tickets than parcels: give parents away, the older ones.  About four
             // warps per missing parcel do so at a time (a hash of warp and step picks
             // them), those with small stacks only when an eighth of the warps is waiting.
@@ -432,7 +436,7 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
             const unsigned missing = wanted > inputs + given ? wanted - inputs - given : 0u;
             const unsigned pick = (warp_id * 2654435761u + t.steps * 0x9E3779B9u) >> 16;
             bool give = (unsigned long long)pick * nwarps < (unsigned long long)missing * (4u << 16) &&
-                        (np + nspill >= 48 || missing * 8u > nwarps);
+                        (eager || np + nspill >= 48 || missing * 8u > nwarps);
             give = __shfl_sync(full, (int)give, 0) != 0;
             unsigned d = 0, n = 0;
             bool room = false;  // the slot's last parcel has been taken
