@@ -83,7 +83,7 @@ struct DeepSched {
 // Parcel d lies in slot d % kParcels, whose flag says epoch << 40 | d << 8 | parents
 // held, or kParcelTaken.  Only warps with nothing left draw tickets, so there are
 // fewer parcels under way than warps.
-constexpr unsigned kParcels = 1u << 13;
+constexpr unsigned kParcels = 1u << 12;
 constexpr unsigned kParcelTaken = 0xFF;
 __device__ __forceinline__ unsigned long long parcel_tag(unsigned long long epoch, unsigned d) {
     return (epoch & 0xFFFFFFull) << 32 | d;
