@@ -257,11 +257,10 @@ def train_models(prover, cp, depth):
 
 
 # DRAM traffic of the graph refinement per evaluated box, from one ncu capture
-# (middle family, 32^4 seed, one level: 11.95M boxes evaluated, 10.9M children
-# written, 1.118 GB read + 1.208 GB written); algorithmic: 65 B read per 4-D box
-# and 65 B written per child.  FP64 pipe activity of the same capture.
-TRAFFIC_PER_BOX, ALGORITHMIC_BYTES_PER_BOX = 2.326e9 / 11.95e6, 124.0
-FP64_PIPE_ACTIVE_NCU = 0.239
+# (middle family, 32^4 seed, two levels: 138.4M boxes evaluated, 73.7 MB read + 6.1 MB
+# written); algorithmic: the 65 B of a 4-D seed.  FP64 pipe activity of the same capture.
+TRAFFIC_PER_BOX, ALGORITHMIC_BYTES_PER_BOX = 79.8e6 / 138.4e6, 65.0 * 32**4 / 138.4e6
+FP64_PIPE_ACTIVE_NCU = 0.441
 
 PROOF_FAMILIES = (0, 1, 2, 3, 4, 5)
 
@@ -274,7 +273,7 @@ def proof_leg(prover, cp, forms, families, world=1):
     each seeded with the reference's own radius lattice -- not-proved boxes
     bisected in lambda only (the reference's own refinement rule,
     run_kernel.cuh:110-127).  A family is proved when no box is left
-    unresolved.  The best form runs every slab as one graph launch, the plain
+    unresolved.  The best form runs every slab as one kernel launch, the plain
     form as the FP64 host-driven level loop; both evaluate the same tree, which
     the per-box verdict digests confirm."""
     out = []
@@ -355,10 +354,10 @@ def roofline_of(cp, device, reps, counts) -> dict:
     return {"bound": "fp64", "achieved": achieved / 1e12, "peak": peak / 1e12, "unit": "TFLOP/s",
             "frac": achieved / peak,
             "traffic": TRAFFIC_PER_BOX * boxes,
-            "traffic_note": f"DRAM bytes per step: {TRAFFIC_PER_BOX:.0f} B per evaluated box from one ncu capture of "
-                            f"the graph refinement (algorithmic {ALGORITHMIC_BYTES_PER_BOX:.0f} B), scaled by the "
+            "traffic_note": f"DRAM bytes per step: {TRAFFIC_PER_BOX:.2f} B per evaluated box from one ncu capture of "
+                            f"the graph refinement (algorithmic {ALGORITHMIC_BYTES_PER_BOX:.2f} B), scaled by the "
                             f"step's {boxes} evaluated boxes",
-            "kernel": "k_level_persist<family, precision, block> (per-box criteria + split), graph engine",
+            "kernel": "k_refine_deep<family, precision, block> (per-box criteria + split), graph engine",
             "work_model": "per evaluated box: the reference kernel's own add/sub, mul, div and asin count (it stops "
                           "at the first failing sub-check and handle), counted by the CPU restatement while it refines "
                           "sampled seeds of the same workload, per family and depth, weighted by the step's boxes per "
@@ -615,9 +614,9 @@ def main():
     boxes_step = sum(r["evaluated"] for r in reps_best)
     value = sum_over_ranks(world, boxes_step) / (ms_best / 1e3)
     plain_value = sum_over_ranks(world, sum(r["evaluated"] for r in reps_plain)) / (ms_plain / 1e3)
-    # kernels per step: the graph engine's chunk launches (+ scheduler, + inference
-    # with a learned order), the seed and slab-bound kernels
-    launches_step = sum(r["launches"] * ((3 if forms[f].get("learned_order") else 2)
+    # kernels per step: the graph engine's launches (with a learned order its chunks',
+    # scheduler and inference included), the seed and slab-bound kernels
+    launches_step = sum(r["launches"] * ((3 if forms[f].get("learned_order") else 1)
                                          if forms[f]["engine"] == cp.ENGINE_GRAPH else
                                          (2 if forms[f].get("learned_order") else 1)) + 2
                         for f, r in zip(FAMILIES, reps_best))

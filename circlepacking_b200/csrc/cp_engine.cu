@@ -132,7 +132,7 @@ __global__ void k_graph_upload(GraphUpload u, BoxList* levels, DevSched* sched) 
 }
 
 // Seeded random boxes on the family's domain (the uneven-depth workload of the
-// persistent engine).  Box i draws its numbers from a counter-based generator:
+// graph engine).  Box i draws its numbers from a counter-based generator:
 // u(i, k) = top 53 bits of mix64(seed ^ mix64(8 i + k)) / 2^53.  Lambda has its
 // centre uniform in [0.5, 0.99]; each radius has its centre uniform in the
 // dependent range of the axes before it (the ranges the lattice enumerates,
@@ -347,7 +347,7 @@ struct cp_prover {
     int levels_dims = 0;
     size_t level_cap = 0;
     void* model = nullptr;  // learned model state (cp_model.cu)
-    // device-driven loop (CUDA graph with a conditional WHILE node)
+    // device-driven loop of a learned policy (CUDA graph with a conditional WHILE node)
     BoxList* d_levels = nullptr;
     DevSched* d_sched = nullptr;
     DevSched* h_sched = nullptr;  // pinned mirror

@@ -543,7 +543,10 @@ CPF_HD bool start_end_2d_box(const Ref& ref, FOut& o) {
         const FBox b = ref.load();
         const Terms t(b);
         tol = t.tol;
-        ok = clear_mixed_lo(b.ll, b.l1, b.l2);
+        // (the order of the mixed corner, before any angle: slabs near lambda = 0.99 that are
+        // wide against their disks fail it throughout)
+        ok = clear_mixed_lo(b.ll, b.l1, b.l2) && b.lh + b.h2 <= 1.0 - b.h1;
+        if (!ok) return false;
         a1 = semi_outer(b.h1);
         const double a2_hi = semi_inner(b.ll, b.h2), a12_hi = mixed_hi(b.ll, b.lh, b.h1, b.h2, ok);
         const double q = fma_(2.0, b.h2, b.lh);

@@ -79,8 +79,7 @@ struct NetArgs {
 constexpr int kNetBlock = tc::kTcRows;  // one box per thread of a 128-thread CTA
 constexpr int kNetMaxCtasPerSm = 512 / (int)tc::kNetCols;  // tensor memory: 512 columns per SM
 
-// (__launch_bounds__ with 5 resident CTAs caps the registers near the 96 of the
-// plain persistent kernel's 128-thread shape)
+// (__launch_bounds__ with 5 resident CTAs caps the registers near 96)
 template <int FAM, int PREC>
 __global__ void __launch_bounds__(kNetBlock, 5) k_level_persist_net(PersistArgs pa, NetArgs na) {
     constexpr int D = family_dims(FAM);

@@ -1,6 +1,7 @@
-// The level step of the box refinement, shared by the level-synchronous
-// kernel (cp_engine.cu) and the persistent graph-driven kernel (cp_graph.cu):
-// evaluate one box per lane (DECIDE mode, optional FP32 pre-pass and per-box
+// The level step of the box refinement, for kernels whose children all go through a
+// level (per-box hints and trace records, cp_engine.cu; the network inline,
+// cp_graph_kernels.cuh), and what they share with the warp-local refinement
+// (cp_refine.cuh): evaluate one box per lane (DECIDE mode, optional FP32 pre-pass and per-box
 // criterion order), count verdicts, and append the children of every box that
 // is not proved to the next worklist level.
 #pragma once

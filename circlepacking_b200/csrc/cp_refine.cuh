@@ -8,7 +8,7 @@
 // Why: with the filter a box costs about 700 warp instructions, less than writing
 // its children to a level (65 B each, a division and two dependent table loads per
 // child) and reading them back cost.  A refinement's last level holds most of its
-// boxes.  B200, middle, 64^4 lattice and two uniform levels, graph engine: 188 -> 85 ms
+// boxes.  B200, middle, 64^4 lattice and two uniform levels, graph engine: 188 -> 75 ms
 // (of which the level's kernels and the filter read their boxes from shared memory
 // instead of holding them in registers: no spills at 20 warps per SM).
 //
