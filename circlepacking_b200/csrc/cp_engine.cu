@@ -266,8 +266,8 @@ __global__ void __launch_bounds__(kEvalBlock) k_ref_step(RefArgs a) {
         double lo[4], hi[4];
         if (!lattice_box(a.s, ix, a.slab_single[slab], lo, hi)) continue;
         ++evaluated;
-        const Verdict v = COLLECT ? judge_box<FAM, FULL, flt::NEED_FULL>(val_ref<D>(lo, hi), 0)
-                                  : judge_box<FAM, DECIDE, flt::NEED_VERDICT>(val_ref<D>(lo, hi), 0);
+        const Verdict v = COLLECT ? verdict_box<FAM, FULL, flt::NEED_FULL>(val_ref<D>(lo, hi), 0)
+                                  : verdict_box<FAM, DECIDE, flt::NEED_VERDICT>(val_ref<D>(lo, hi), 0);
         if (v.verdict == V_EMPTY) continue;
         const bool nofit = (v.mask & M_FIT) && FAM != F_START && FAM != F_START_END_2D && FAM != F_START_END_3D;
         const bool trap = (v.mask & M_TRAP) != 0;

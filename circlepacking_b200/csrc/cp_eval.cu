@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kEvalBlock) k_eval_fp64(const double* __restri
             }
         }
         const Verdict v = TRACE ? eval_box<FAM, MODE>(l, h, ord, trace + 16 * i)
-                                : judge_box<FAM, MODE, need_of(MODE)>(BoxRef<D>{lo + i, hi + i, stride}, ord);
+                                : verdict_box<FAM, MODE, need_of(MODE)>(BoxRef<D>{lo + i, hi + i, stride}, ord);
         verdict[i] = v.verdict;
         mask[i] = v.mask;
     }
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kEvalBlock) k_eval_prefilter(const double* __r
         const int pre = prefilter_box<FAM>(l, h, ord, MODE == FULL, &pmask);
         Verdict v;
         if (pre == PF_UNDECIDED)
-            v = TRACE ? eval_box<FAM, MODE>(l, h, ord, trace + 16 * i) : judge_box<FAM, MODE, need_of(MODE)>(BoxRef<D>{lo + i, hi + i, stride}, ord);
+            v = TRACE ? eval_box<FAM, MODE>(l, h, ord, trace + 16 * i) : verdict_box<FAM, MODE, need_of(MODE)>(BoxRef<D>{lo + i, hi + i, stride}, ord);
         else
             v = {pre == PF_PROVED ? V_PROVED : pre == PF_EMPTY ? V_EMPTY : pre == PF_NOFIT ? V_NOFIT : V_CRITICAL,
                  pmask};

@@ -414,10 +414,10 @@ struct BoxRef {
 
 // eval_box without a trace, through the FP64 filter: the same verdict, with the
 // part of mask and handles that NEED asks for (flt::Need).  In two steps, so that a
-// warp can come together in between: judge_fast returns false for the boxes the
-// filter leaves, judge_slow evaluates those.
+// warp can come together in between: verdict_fast returns false for the boxes the
+// filter leaves, verdict_slow evaluates those.
 template <int FAM, int MODE, int NEED, class Ref>
-__device__ __forceinline__ bool judge_fast(const Ref& ref, int order, Verdict& v) {
+__device__ __forceinline__ bool verdict_fast(const Ref& ref, int order, Verdict& v) {
     constexpr int D = family_dims(FAM);
     constexpr bool kFitStops = FAM != F_START && FAM != F_START_END_2D && FAM != F_START_END_3D;
     uint8_t fit = 0;
@@ -441,19 +441,19 @@ __device__ __forceinline__ bool judge_fast(const Ref& ref, int order, Verdict& v
     return decided;
 }
 template <int FAM, int MODE, class Ref>
-__device__ __forceinline__ Verdict judge_slow(const Ref& ref, int order) {
+__device__ __forceinline__ Verdict verdict_slow(const Ref& ref, int order) {
     const flt::FBox b = ref.load();  // (tightened: eval_box's own tightening changes nothing)
     const uint32_t r = eval_box_call<FAM, MODE>(b.ll, b.lh, b.l1, b.h1, b.l2, b.h2, b.l3, b.h3, order);
     return {(uint8_t)r, (uint8_t)(r >> 8), (uint8_t)(r >> 16)};
 }
 template <int FAM, int MODE, int NEED, class Ref>
-__device__ __forceinline__ Verdict judge_box(const Ref& ref, int order) {
+__device__ __forceinline__ Verdict verdict_box(const Ref& ref, int order) {
     Verdict v;
-    if (!judge_fast<FAM, MODE, NEED>(ref, order, v)) v = judge_slow<FAM, MODE>(ref, order);
+    if (!verdict_fast<FAM, MODE, NEED>(ref, order, v)) v = verdict_slow<FAM, MODE>(ref, order);
     return v;
 }
 
-// A box in registers, for judge_box.
+// A box in registers, for verdict_box.
 template <int D>
 __device__ __forceinline__ flt::ValRef val_ref(const double* lo, const double* hi) {
     flt::FBox b{lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], D == 4 ? lo[3] : 0.0, D == 4 ? hi[3] : 0.0};

@@ -250,7 +250,7 @@ __device__ __forceinline__ void level_step(const LevelArgs& a, size_t j, LevelSm
                 uint8_t pmask;
                 const int pre = prefilter_box<FAM>(lo, hi, ord, false, &pmask);
                 if (pre == PF_UNDECIDED) {
-                    const Verdict r = judge_box<FAM, DECIDE, flt::NEED_HANDLES>(BoxRef<D>{a.in.lo + i, a.in.hi + i, a.in.cap}, ord);
+                    const Verdict r = verdict_box<FAM, DECIDE, flt::NEED_HANDLES>(BoxRef<D>{a.in.lo + i, a.in.hi + i, a.in.cap}, ord);
                     v = r.verdict;
                     handles += r.handles;
                 } else {
@@ -258,7 +258,7 @@ __device__ __forceinline__ void level_step(const LevelArgs& a, size_t j, LevelSm
                     fp32_decided = pre != PF_EMPTY;
                 }
             } else {
-                const Verdict r = judge_box<FAM, DECIDE, flt::NEED_HANDLES>(BoxRef<D>{a.in.lo + i, a.in.hi + i, a.in.cap}, ord);
+                const Verdict r = verdict_box<FAM, DECIDE, flt::NEED_HANDLES>(BoxRef<D>{a.in.lo + i, a.in.hi + i, a.in.cap}, ord);
                 v = r.verdict;
                 handles += r.handles;
             }

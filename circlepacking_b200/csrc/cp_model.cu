@@ -1100,7 +1100,7 @@ __global__ void __launch_bounds__(128) k_label(LabelArgs a) {
             lo[d] = a.in.lo[d * a.in.cap + i];
             hi[d] = a.in.hi[d * a.in.cap + i];
         }
-        const Verdict v = judge_box<FAM, FULL, flt::NEED_FULL>(BoxRef<D>{a.in.lo + i, a.in.hi + i, a.in.cap}, 0);
+        const Verdict v = verdict_box<FAM, FULL, flt::NEED_FULL>(BoxRef<D>{a.in.lo + i, a.in.hi + i, a.in.cap}, 0);
         if (v.verdict == V_EMPTY) continue;
         int label = -1;
         if (v.verdict == V_CRITICAL) {

@@ -359,14 +359,14 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
             }
             if (v < 0) {
                 Verdict q;
-                left = !judge_fast<FAM, DECIDE, flt::NEED_HANDLES>(box, 0, q);
+                left = !verdict_fast<FAM, DECIDE, flt::NEED_HANDLES>(box, 0, q);
                 v = q.verdict;
                 if (!left) handles += q.handles;
             }
         }
         if (__any_sync(full, left)) {  // boxes the filter leaves to the directed evaluation
             if (left) {
-                const Verdict q = judge_slow<FAM, DECIDE>(box, 0);
+                const Verdict q = verdict_slow<FAM, DECIDE>(box, 0);
                 v = q.verdict;
                 handles += q.handles;
             }
