@@ -1,0 +1,54 @@
+// Parcels: how a warp of the depth-first refinement (cp_refine.cuh) hands parents to a
+// warp that has run out.  Parcel d lies in slot d % slots, whose flag says which
+// parcel it holds and how far that has come:
+//
+//     epoch (24 bits) | d (32 bits) | state (8 bits)
+//
+// state 0: claimed, its giver is writing the parents; 1 to 32: that many parents, ready;
+// kParcelTaken: read, the slot is free.  The epoch is the launch's; a flag of another
+// launch leaves its slot free.
+//
+// A giver claims its slot by compare-and-swap before it writes.  Givers run ahead of
+// takers (about four warps give per missing parcel), so two of them can want one slot at
+// a time: parcels d and d + slots.  The second finds the slot claimed or ready and keeps
+// its parents.
+//
+// Host code too, so that the protocol is tested without a GPU.
+#pragma once
+#include <cstdint>
+
+#ifdef __CUDACC__
+#define CPP_HD __host__ __device__ __forceinline__
+#else
+#define CPP_HD inline
+#endif
+
+namespace cpb {
+
+typedef unsigned long long ParcelFlag;
+
+constexpr unsigned kParcels = 1u << 12;  // slots
+constexpr unsigned kParcelTaken = 0xFF;
+
+CPP_HD ParcelFlag parcel_tag(unsigned long long epoch, unsigned d) { return (epoch & 0xFFFFFFull) << 32 | d; }
+
+CPP_HD ParcelFlag flag_read(const ParcelFlag* flag) { return *(const volatile ParcelFlag*)flag; }
+CPP_HD bool flag_swap(ParcelFlag* flag, ParcelFlag from, ParcelFlag to) {
+#ifdef __CUDA_ARCH__
+    return atomicCAS(flag, from, to) == from;
+#else
+    return __atomic_compare_exchange_n(flag, &from, to, false, __ATOMIC_SEQ_CST, __ATOMIC_SEQ_CST);
+#endif
+}
+
+// No parcel of this launch lies in the slot.
+CPP_HD bool parcel_free(ParcelFlag f, unsigned long long epoch) {
+    return f >> 40 != (epoch & 0xFFFFFFull) || (f & 0xFF) == kParcelTaken;
+}
+// The giver's: true when slot d % slots is the caller's to write.
+CPP_HD bool parcel_claim(ParcelFlag* flag, unsigned long long epoch, unsigned d) {
+    const ParcelFlag f = flag_read(flag);
+    return parcel_free(f, epoch) && flag_swap(flag, f, parcel_tag(epoch, d) << 8);
+}
+
+}  // namespace cpb

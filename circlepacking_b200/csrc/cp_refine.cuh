@@ -33,6 +33,7 @@
 // besides 31 ready ones: 63 parents.
 #pragma once
 #include "cp_level.cuh"
+#include "cp_parcel.cuh"
 
 namespace cpb {
 
@@ -80,14 +81,6 @@ struct DeepSched {
     unsigned int left;         // parcels left over: another round is needed
     int status;                // 0 ok, 1 spill overflow
 };
-// Parcel d lies in slot d % kParcels, whose flag says epoch << 40 | d << 8 | parents
-// held, or kParcelTaken.  Only warps with nothing left draw tickets, so there are
-// fewer parcels under way than warps.
-constexpr unsigned kParcels = 1u << 12;
-constexpr unsigned kParcelTaken = 0xFF;
-__device__ __forceinline__ unsigned long long parcel_tag(unsigned long long epoch, unsigned d) {
-    return (epoch & 0xFFFFFFull) << 32 | d;
-}
 // A warp with fewer parents keeps them.  FP32: its steps take ten times as long, so
 // that warps give from small stacks too and look after every step.
 template <int PREC>
@@ -439,12 +432,11 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
                         (eager || np + nspill >= 48 || missing * 8u > nwarps);
             give = __shfl_sync(full, (int)give, 0) != 0;
             unsigned d = 0, n = 0;
-            bool room = false;  // the slot's last parcel has been taken
+            bool room = false;  // the slot is this warp's
             if (give) {
                 if (lane == 0) {
                     d = atomicAdd(&r.sched->parcels, 1u);
-                    const unsigned long long f = *(volatile unsigned long long*)(r.flags[round & 1] + d % kParcels);
-                    room = f >> 40 != (r.sched->epoch & 0xFFFFFFull) || (f & 0xFF) == kParcelTaken;
+                    room = parcel_claim(r.flags[round & 1] + d % kParcels, r.sched->epoch, d);
                 }
                 d = __shfl_sync(full, d, 0);
                 room = __shfl_sync(full, (int)room, 0) != 0;

@@ -1,0 +1,41 @@
+"""The depth-first kernel's parcel protocol (csrc/cp_parcel.cuh), built for the host."""
+import ctypes
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "circlepacking_b200", "csrc")
+SLOTS, TAKEN = 1 << 12, 0xFF
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("parcel") / "libparcel.so")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-pthread", "-shared", "-fPIC", "-I" + CSRC,
+                    os.path.join(HERE, "parcel_host.cpp"), "-o", so], check=True)
+    L = ctypes.CDLL(so)
+    L.p_claim.argtypes = [ctypes.c_void_p, ctypes.c_ulonglong, ctypes.c_uint]
+    L.p_stress.restype = ctypes.c_long
+    return L
+
+
+@pytest.mark.parametrize("epoch", [1, 5, (1 << 24) - 1])
+def test_one_giver_per_slot(host, epoch):
+    """Parcels d and d + slots want one slot: the second giver is refused from the first one's claim on,
+    before anything is published, until the parcel has been taken."""
+    flag = ctypes.c_ulonglong(0)
+    p = ctypes.byref(flag)
+    assert host.p_claim(p, epoch, 3)
+    assert not host.p_claim(p, epoch, 3 + SLOTS)  # claimed, not yet published
+    flag.value |= 32
+    assert not host.p_claim(p, epoch, 3 + SLOTS)  # ready
+    flag.value |= TAKEN
+    assert host.p_claim(p, epoch, 3 + SLOTS)
+    assert flag.value == epoch << 40 | (3 + SLOTS) << 8
+    assert host.p_claim(p, epoch + 1, 3)  # another launch's flag
+
+
+def test_claims_exclude_each_other(host):
+    assert host.p_stress(8, 3, 20000) == 0
