@@ -13,6 +13,11 @@
 // a time: parcels d and d + slots.  The second finds the slot claimed or ready and keeps
 // its parents.
 //
+// A warp reads and writes a slot with all of its lanes, but one lane works its flag.  So
+// the lanes' copies stand between an acquire() and a release() of the warp: no lane
+// touches the slot before the lane at the flag has seen it in the warp's hands, and the
+// flag passes the slot on when every lane is done with it.
+//
 // Host code too, so that the protocol is tested without a GPU.
 #pragma once
 #include <cstdint>
@@ -49,6 +54,48 @@ CPP_HD bool parcel_free(ParcelFlag f, unsigned long long epoch) {
 CPP_HD bool parcel_claim(ParcelFlag* flag, unsigned long long epoch, unsigned d) {
     const ParcelFlag f = flag_read(flag);
     return parcel_free(f, epoch) && flag_swap(flag, f, parcel_tag(epoch, d) << 8);
+}
+
+#ifdef __CUDACC__
+// The warp that handles a slot; all of its lanes make each call.
+struct SlotWarp {
+    __device__ __forceinline__ bool first() const { return (threadIdx.x & 31) == 0; }
+    __device__ __forceinline__ void acquire() const {
+        __threadfence();
+        __syncwarp();
+    }
+    __device__ __forceinline__ void release() const {
+        __syncwarp();
+        __threadfence();
+    }
+};
+#endif
+CPP_HD void flag_set(ParcelFlag* flag, ParcelFlag to) {
+#ifdef __CUDA_ARCH__
+    atomicExch(flag, to);
+#else
+    __atomic_store_n(flag, to, __ATOMIC_SEQ_CST);
+#endif
+}
+
+// Writes the n parents of parcel d into its slot, which the warp has claimed: write() is a
+// lane's part.
+template <class Warp, class Write>
+CPP_HD void parcel_give(const Warp& w, ParcelFlag* flag, unsigned long long epoch, unsigned d, unsigned n,
+                        const Write& write) {
+    w.acquire();
+    write();
+    w.release();
+    if (w.first()) flag_set(flag, parcel_tag(epoch, d) << 8 | n);
+}
+// Reads the parents of a slot whose flag, as the warp's first lane saw it, holds a parcel:
+// read() is a lane's part.  The slot is free afterwards.
+template <class Warp, class Read>
+CPP_HD void parcel_take(const Warp& w, ParcelFlag* flag, const Read& read) {
+    w.acquire();
+    read();
+    w.release();
+    if (w.first()) flag_set(flag, flag_read(flag) | kParcelTaken);
 }
 
 }  // namespace cpb

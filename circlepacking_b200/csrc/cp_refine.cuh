@@ -295,8 +295,8 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
                     drawn = false;
                 }
                 const MetaList& from = r.lists[(given_now ? round : round + 1) & 1];
-                __threadfence();
-                if (lane < n) {
+                parcel_take(SlotWarp{}, flag, [&] {
+                    if (lane >= n) return;
                     const size_t e = (size_t)p * 32 + lane;
 #pragma unroll
                     for (int d = 0; d < D; ++d) {
@@ -304,13 +304,9 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
                         wb.phi[d][lane] = __ldcg(from.hi + d * from.cap + e);
                     }
                     wb.pmeta[lane] = __ldcg(from.meta + e);
-                }
+                });
                 np = n;
-                if (lane == 0) {
-                    atomicOr(flag, (unsigned long long)kParcelTaken);
-                    if (given_now) atomicAdd(&r.sched->taken, 1u);
-                }
-                __syncwarp();
+                if (lane == 0 && given_now) atomicAdd(&r.sched->taken, 1u);
                 continue;
             } else {
                 break;
@@ -444,32 +440,21 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
             if (room) {
                 const unsigned p = d % kParcels;
                 const MetaList& out = r.lists[round & 1];
-                const size_t o = (size_t)p * 32 + lane;
-                if (nspill >= 32) {
-                    n = 32;
-                    nspill -= 32;
-                    const size_t e = (size_t)warp_id * r.seg + nspill + lane;
-#pragma unroll
-                    for (int d = 0; d < D; ++d) {
-                        out.lo[d * out.cap + o] = r.spill.lo[d * r.spill.cap + e];
-                        out.hi[d * out.cap + o] = r.spill.hi[d * r.spill.cap + e];
-                    }
-                    out.meta[o] = r.spill.meta[e];
-                } else if (nspill > 0) {
-                    n = nspill;
-                    nspill = 0;
-                    const size_t e = (size_t)warp_id * r.seg + lane;
-                    if (lane < n) {
+                const bool spilled = nspill > 0;  // the youngest spilled parents, else half of those on chip
+                n = spilled ? (nspill < 32 ? nspill : 32) : np / 2;
+                if (spilled) nspill -= n;
+                parcel_give(SlotWarp{}, r.flags[round & 1] + p, r.sched->epoch, d, n, [&] {
+                    if (lane >= n) return;
+                    const size_t o = (size_t)p * 32 + lane;
+                    if (spilled) {
+                        const size_t e = (size_t)warp_id * r.seg + nspill + lane;
 #pragma unroll
                         for (int d = 0; d < D; ++d) {
                             out.lo[d * out.cap + o] = r.spill.lo[d * r.spill.cap + e];
                             out.hi[d * out.cap + o] = r.spill.hi[d * r.spill.cap + e];
                         }
                         out.meta[o] = r.spill.meta[e];
-                    }
-                } else {
-                    n = np / 2;  // at most 32; entries n .. np move down to 0 (two rounds of 32 lanes)
-                    if (lane < n) {
+                    } else {
 #pragma unroll
                         for (int d = 0; d < D; ++d) {
                             out.lo[d * out.cap + o] = wb.plo[d][lane];
@@ -477,7 +462,9 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
                         }
                         out.meta[o] = wb.pmeta[lane];
                     }
-                    __syncwarp();
+                });
+                if (lane == 0) atomicAdd(&r.sched->filled, 1u);
+                if (!spilled) {  // entries n .. np move down to 0 (two rounds of 32 lanes)
                     for (unsigned b = 0; b < np - n; b += 32) {
                         const unsigned to = b + lane, q = n + to;
                         const bool move = q < np;
@@ -503,12 +490,6 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
                         __syncwarp();
                     }
                     np -= n;
-                }
-                __threadfence();
-                __syncwarp();
-                if (lane == 0) {
-                    atomicExch(r.flags[round & 1] + p, parcel_tag(r.sched->epoch, d) << 8 | n);
-                    atomicAdd(&r.sched->filled, 1u);
                 }
             }
             __syncwarp();

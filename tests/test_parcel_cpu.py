@@ -17,7 +17,7 @@ def host(tmp_path_factory):
                     os.path.join(HERE, "parcel_host.cpp"), "-o", so], check=True)
     L = ctypes.CDLL(so)
     L.p_claim.argtypes = [ctypes.c_void_p, ctypes.c_ulonglong, ctypes.c_uint]
-    L.p_stress.restype = ctypes.c_long
+    L.p_stress.restype = L.p_hand_over.restype = ctypes.c_long
     return L
 
 
@@ -39,3 +39,8 @@ def test_one_giver_per_slot(host, epoch):
 
 def test_claims_exclude_each_other(host):
     assert host.p_stress(8, 3, 20000) == 0
+
+
+def test_slot_is_passed_on_by_the_whole_warp(host):
+    """The flag moves when every lane has read or written, not when the first one has."""
+    assert host.p_hand_over(200) == 0
