@@ -106,10 +106,15 @@ __global__ void k_copy_seed(int dims, const double* __restrict__ lo, const doubl
 
 // Counters read from a checkpoint: ready for the next chunk (level_end).
 __global__ void k_ready_chunk(unsigned long long* cnt) { cnt[C_OUT] = cnt[C_CLAIM] = cnt[C_DONE] = 0; }
-// A depth-first refinement of `count` seed boxes starts.
+// A depth-first refinement of `count` seed boxes starts (one block).
 // The first ticket of each warp is its number.
-__global__ void k_begin_deep(DeepSched* s, unsigned long long count, unsigned warps) {
-    const unsigned long long epoch = s->epoch + 2;  // no flag of an earlier refinement carries this or the one before
+__global__ void k_begin_deep(DeepSched* s, ParcelFlag* flags, unsigned long long count, unsigned warps) {
+    bool clear;
+    const unsigned long long epoch = parcel_epoch(s->epoch, clear);
+    if (clear)
+        for (unsigned i = threadIdx.x; i < 2 * kParcels; i += blockDim.x) flags[i] = 0;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
     *s = DeepSched{};
     s->epoch = epoch;
     s->count = count;
@@ -937,7 +942,7 @@ cp_status refine_graph(cp_prover* p, const cp_refine_opts& o, cp_refine_report* 
     a.flags[0] = p->deep_flags;
     a.flags[1] = p->deep_flags + kParcels;
     a.spill = p->deep_spill;
-    k_begin_deep<<<1, 1, 0, p->stream>>>(p->deep_sched, (unsigned long long)n, (unsigned)warps);
+    k_begin_deep<<<1, 256, 0, p->stream>>>(p->deep_sched, p->deep_flags, (unsigned long long)n, (unsigned)warps);
     CP_TRY(cp_check_launch());
     CP_TRY(cuda_ok(cudaEventRecord(p->ev0, p->stream)));
     do {  // (hardly ever more than one round)

@@ -6,7 +6,8 @@
 //
 // state 0: claimed, its giver is writing the parents; 1 to 32: that many parents, ready;
 // kParcelTaken: read, the slot is free.  The epoch is the launch's; a flag of another
-// launch leaves its slot free.
+// launch leaves its slot free.  Epochs come back after 2^24 launches, so the flags are
+// cleared ahead of that (parcel_epoch).
 //
 // A giver claims its slot by compare-and-swap before it writes.  Givers run ahead of
 // takers (about four warps give per missing parcel), so two of them can want one slot at
@@ -49,6 +50,23 @@ CPP_HD bool flag_swap(ParcelFlag* flag, ParcelFlag from, ParcelFlag to) {
 // No parcel of this launch lies in the slot.
 CPP_HD bool parcel_free(ParcelFlag f, unsigned long long epoch) {
     return f >> 40 != (epoch & 0xFFFFFFull) || (f & 0xFF) == kParcelTaken;
+}
+// Parents ready in the slot for the ticket of parcel d; 0: not yet.
+CPP_HD unsigned parcel_ready(ParcelFlag f, unsigned long long epoch, unsigned d) {
+    const unsigned n = (unsigned)(f & 0xFF);
+    return f >> 8 == parcel_tag(epoch, d) && n != kParcelTaken ? n : 0u;
+}
+// Parents that the launch of this epoch left over in the slot.
+CPP_HD unsigned parcel_left(ParcelFlag f, unsigned long long epoch) {
+    return parcel_free(f, epoch) ? 0u : (unsigned)(f & 0xFF);
+}
+// The epoch of a refinement's first launch, `last` being the epoch after the handle's
+// latest launch.  No flag carries it or the one before: the next one but one, or, when
+// half of the epochs are used up, epoch 1 over cleared flags (clear).  The other half is
+// left to the further launches of a refinement.
+CPP_HD unsigned long long parcel_epoch(unsigned long long last, bool& clear) {
+    clear = last + 2 >= 1ull << 23;
+    return clear ? 1 : last + 2;
 }
 // The giver's: true when slot d % slots is the caller's to write.
 CPP_HD bool parcel_claim(ParcelFlag* flag, unsigned long long epoch, unsigned d) {

@@ -265,14 +265,12 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
                 if (!given_now) {  // a parcel left over from the last round
                     p = ticket;
                     flag = r.flags[(round + 1) & 1] + p;
-                    const unsigned long long f = *(volatile unsigned long long*)flag;
-                    n = f >> 40 == ((r.sched->epoch - 1) & 0xFFFFFFull) && (f & 0xFF) != kParcelTaken ? (unsigned)(f & 0xFF) : 0u;
+                    n = parcel_left(flag_read(flag), r.sched->epoch - 1);
                     n = __shfl_sync(full, n, 0);
                     drawn = false;
                     if (n == 0) continue;
                 } else {
                     if (nr > 0) break;  // (the last input went to another warp meanwhile)
-                    const unsigned long long tag = parcel_tag(r.sched->epoch, ticket - inputs);
                     p = (ticket - inputs) % kParcels;
                     flag = r.flags[round & 1] + p;
                     if (lane == 0) {
@@ -280,8 +278,7 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
                         for (int k = 0; k < kWaitPolls; ++k) {
                             const bool over = *(volatile unsigned*)&r.sched->idle >= nwarps;
                             __threadfence();
-                            const unsigned long long f = *(volatile unsigned long long*)flag;
-                            n = f >> 8 == tag ? (unsigned)(f & 0xFF) : 0u;
+                            n = parcel_ready(flag_read(flag), r.sched->epoch, ticket - inputs);
                             if (n || over) break;
                             __nanosleep(kWaitNs);
                         }

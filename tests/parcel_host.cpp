@@ -34,6 +34,25 @@ void warp(pthread_barrier_t* bar, F f) {
 
 extern "C" {
 int p_claim(ParcelFlag* flag, unsigned long long epoch, unsigned d) { return parcel_claim(flag, epoch, d); }
+unsigned p_ready(unsigned long long f, unsigned long long epoch, unsigned d) { return parcel_ready(f, epoch, d); }
+unsigned p_left(unsigned long long f, unsigned long long epoch) { return parcel_left(f, epoch); }
+// Refinements of `launches` launches each on one handle; returns how many launches had
+// an epoch (24 bits) at or below one that an uncleared flag may carry.
+long p_epochs(long refinements, int launches) {
+    long again = 0;
+    unsigned long long last = 0, highest = 0;  // highest: of the flags since they were cleared
+    for (long k = 0; k < refinements; ++k) {
+        bool clear;
+        last = parcel_epoch(last, clear);
+        if (clear) highest = 0;
+        if (((last - 1) & 0xFFFFFF) < highest) ++again;  // (a first launch looks back by one)
+        for (int l = 0; l < launches; ++l, ++last) {
+            if ((last & 0xFFFFFF) <= highest) ++again;
+            highest = last & 0xFFFFFF;
+        }
+    }
+    return again;
+}
 // Threads claim, mark and leave `slots` slots `each` times; returns how often a slot had two owners.
 long p_stress(int threads, unsigned slots, int each) {
     std::vector<ParcelFlag> flag(slots, 0);

@@ -17,6 +17,10 @@ def host(tmp_path_factory):
                     os.path.join(HERE, "parcel_host.cpp"), "-o", so], check=True)
     L = ctypes.CDLL(so)
     L.p_claim.argtypes = [ctypes.c_void_p, ctypes.c_ulonglong, ctypes.c_uint]
+    L.p_ready.argtypes = [ctypes.c_ulonglong, ctypes.c_ulonglong, ctypes.c_uint]
+    L.p_left.argtypes = [ctypes.c_ulonglong, ctypes.c_ulonglong]
+    L.p_epochs.argtypes = [ctypes.c_long, ctypes.c_int]
+    L.p_epochs.restype = ctypes.c_long
     L.p_stress.restype = L.p_hand_over.restype = ctypes.c_long
     return L
 
@@ -44,3 +48,20 @@ def test_claims_exclude_each_other(host):
 def test_slot_is_passed_on_by_the_whole_warp(host):
     """The flag moves when every lane has read or written, not when the first one has."""
     assert host.p_hand_over(200) == 0
+
+
+@pytest.mark.parametrize("n", [0, 1, 32, TAKEN])
+def test_only_parents_that_are_there_are_read(host, n):
+    """A taken parcel is none, neither for the ticket that once waited for it (epochs come back) nor as a left-over."""
+    e, d = 9, 70000
+    there = n if n != TAKEN else 0
+    for epoch in (e, e + (1 << 24)):
+        assert host.p_ready(e << 40 | d << 8 | n, epoch, d) == there
+        assert host.p_left(e << 40 | d << 8 | n, epoch) == there
+    assert host.p_ready(e << 40 | d << 8 | n, e, d + SLOTS) == host.p_ready(e << 40 | d << 8 | n, e + 1, d) == 0
+    assert host.p_left(e << 40 | d << 8 | n, e + 1) == 0
+
+
+@pytest.mark.parametrize("launches", [1, 3, 1 << 20])
+def test_epochs_do_not_come_back_over_uncleared_flags(host, launches):
+    assert host.p_epochs((1 << 25) // launches + 3, launches) == 0
