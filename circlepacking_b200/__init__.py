@@ -272,6 +272,8 @@ def _declare_handle(L):
     L.cp_autotune.argtypes = [P, ctypes.POINTER(RefineOpts), ctypes.POINTER(ctypes.c_int), P]
     L.cp_refine_boxes_static.argtypes = [I, I, I, I, P, P, P, SZ, ctypes.POINTER(RefineReport), P]
     L.cp_set_level_variant.argtypes = [P, I, I, I]
+    L.cp_set_deep_limits.argtypes = [P, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int64]
+    L.cp_deep_stats.argtypes = [P, P]
     L.cp_refine_resume.argtypes = [P, ctypes.POINTER(RefineReport)]
     L.cp_checkpoint_save.argtypes = [P, ctypes.c_char_p]
     L.cp_checkpoint_load.argtypes = [P, ctypes.c_char_p, ctypes.POINTER(RefineOpts)]
@@ -409,6 +411,16 @@ class Prover:
 
     def set_level_variant(self, family, precision, variant):
         _check(self._L.cp_set_level_variant(self._h, family, precision, variant), "cp_set_level_variant")
+
+    def set_deep_limits(self, polls=-1, slots=-1, strict=-1, epoch=-1):
+        """Diagnostic limits of the graph engine's work sharing (-1: default, or left alone)."""
+        _check(self._L.cp_set_deep_limits(self._h, polls, slots, strict, epoch), "cp_set_deep_limits")
+
+    def deep_stats(self) -> dict:
+        """Launches, parcels, spilled boxes and launch number of the last graph-engine refinement."""
+        v = np.zeros(4, np.int64)
+        _check(self._L.cp_deep_stats(self._h, v.ctypes.data_as(ctypes.c_void_p)), "cp_deep_stats")
+        return dict(zip(("launches", "parcels", "spilled", "epoch"), v.tolist()))
 
     def refine(self, family, **kw) -> dict:
         o = self.opts(family, **kw)

@@ -367,6 +367,8 @@ struct cp_prover {
     MetaList deep_spill{};
     unsigned char* deep_buf = nullptr;         // holds the lists and flags
     int deep_dims = 0;
+    int deep_polls = kWaitPolls;  // cp_set_deep_limits
+    unsigned deep_slots = kParcels, deep_strict = kStrict;
     int graph_variant[6][2] = {{3, 4}, {3, 3}, {3, 4}, {3, 0}, {3, 3}, {3, 3}};  // block-size variant
     int graph_bpt[6][2] = {{1, 1}, {1, 1}, {1, 1}, {1, 1}, {1, 1}, {1, 1}};      // boxes per thread
     // an interrupted host-driven refinement: the level stack and counters hold
@@ -922,9 +924,10 @@ cp_status refine_graph(cp_prover* p, const cp_refine_opts& o, cp_refine_report* 
     const unsigned grid = (unsigned)(sm_count(p->device) * per_sm);
     const size_t warps = (size_t)grid * (k.threads / 32);
     RefineArgs a{};
-    // a warp works strictly from 128 spilled parents on (512 was no faster); then the stack's bound, and what
-    // the buffers on chip add (cp_refine.cuh)
-    a.strict = 128;
+    // spilled before a warp works strictly, then the stack's bound, and what the buffers on chip add (cp_refine.cuh)
+    a.strict = p->deep_strict;
+    a.slots = p->deep_slots;
+    a.polls = p->deep_polls;
     a.seg = a.strict + 32 * (size_t)(o.max_depth + 1) + 2 * (kParents + kReady);
     a.per = 32u * (unsigned)bpt;
     CP_TRY(ensure_deep(p, D, warps * a.seg));
@@ -1268,6 +1271,28 @@ cp_status cp_set_level_variant(cp_prover* p, int family, int precision, int vari
     if (!p || family < 0 || family > 5 || precision < 0 || precision > 1 || variant < 0 || variant >= kVariants)
         return CP_ERR_INVALID;
     p->variant[family][precision] = variant;
+    return CP_OK;
+}
+
+cp_status cp_set_deep_limits(cp_prover* p, int32_t polls, int32_t slots, int32_t strict, int64_t epoch) {
+    if (!p || polls > kWaitPolls || slots == 0 || slots > (int32_t)kParcels || strict > 4096) return CP_ERR_INVALID;
+    CP_TRY(cuda_ok(cudaSetDevice(p->device)));
+    p->deep_polls = polls < 0 ? kWaitPolls : polls;
+    p->deep_slots = slots < 0 ? kParcels : (unsigned)slots;
+    p->deep_strict = strict < 0 ? kStrict : (unsigned)strict;
+    if (epoch < 0) return CP_OK;
+    CP_TRY(ensure_deep(p, 3, 0));
+    const unsigned long long e = (unsigned long long)epoch;
+    CP_TRY(cuda_ok(cudaMemcpyAsync(&p->deep_sched->epoch, &e, sizeof(e), cudaMemcpyHostToDevice, p->stream)));
+    return cuda_ok(cudaStreamSynchronize(p->stream));
+}
+
+cp_status cp_deep_stats(cp_prover* p, int64_t* out) {
+    if (!p || !out || !p->h_deep) return CP_ERR_INVALID;
+    out[0] = p->h_deep->rounds;
+    out[1] = (int64_t)p->h_deep->given;
+    out[2] = (int64_t)p->h_deep->spilled;
+    out[3] = (int64_t)p->h_deep->epoch;
     return CP_OK;
 }
 

@@ -48,7 +48,8 @@ __global__ void __launch_bounds__(deep_threads(BLOCK)) __maxnreg__(deep_regs(BLO
     s.rounds += 1;
     s.left = left;
     s.epoch += 1;
-    s.inputs = parcels < kParcels ? parcels : kParcels;
+    s.inputs = parcels < r.slots ? parcels : r.slots;
+    s.given += *(volatile unsigned*)&s.filled;
     s.ticket = gridDim.x * kWarps;
     s.parcels = s.filled = s.taken = s.idle = s.done = 0;
 }

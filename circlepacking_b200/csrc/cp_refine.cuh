@@ -80,12 +80,15 @@ struct DeepSched {
     unsigned int rounds;
     unsigned int left;         // parcels left over: another round is needed
     int status;                // 0 ok, 1 spill overflow
+    unsigned long long given;  // over all rounds: parcels given, parents spilled
+    unsigned long long spilled;
 };
 // A warp with fewer parents keeps them.  FP32: its steps take ten times as long, so
 // that warps give from small stacks too and look after every step.
 template <int PREC>
 constexpr unsigned kMinGive = PREC == CP_FP32_PREFILTER ? 4 : 8;
-constexpr int kWaitPolls = 1 << 17, kWaitNs = 200;  // a wait ends after some 30 ms
+constexpr int kWaitPolls = 1 << 17, kWaitNs = 200;  // polls of a wait (it ends after some 30 ms), pause between them
+constexpr unsigned kStrict = 128;                   // RefineArgs::strict (512 was no faster)
 
 struct RefineArgs {
     LevelArgs level;            // policy, limits, counters, input list
@@ -98,6 +101,8 @@ struct RefineArgs {
     MetaList spill;             // warp w: entries [w * seg, (w + 1) * seg)
     size_t seg;
     unsigned strict;            // spilled parents from which a warp works strictly
+    unsigned slots;             // parcel slots in use, at most kParcels
+    int polls;                  // of a wait for a parcel
 };
 
 // A warp's counts, in registers: per lane 10-bit fields for the five verdicts and the
@@ -271,11 +276,11 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
                     if (n == 0) continue;
                 } else {
                     if (nr > 0) break;  // (the last input went to another warp meanwhile)
-                    p = (ticket - inputs) % kParcels;
+                    p = (ticket - inputs) % r.slots;
                     flag = r.flags[round & 1] + p;
                     if (lane == 0) {
                         atomicAdd(&r.sched->idle, 1u);
-                        for (int k = 0; k < kWaitPolls; ++k) {
+                        for (int k = 0; k < r.polls; ++k) {
                             const bool over = *(volatile unsigned*)&r.sched->idle >= nwarps;
                             __threadfence();
                             n = parcel_ready(flag_read(flag), r.sched->epoch, ticket - inputs);
@@ -393,6 +398,7 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
                         r.spill.meta[e] = wb.pmeta[k];
                     }
                     nspill += np;
+                    if (lane == 0) atomicAdd(&r.sched->spilled, (unsigned long long)np);
                 } else if (lane == 0) {
                     r.sched->status = 1;  // (beyond the bound)
                 }
@@ -429,13 +435,13 @@ __device__ __forceinline__ void refine_warp(const RefineArgs& r, Smem& sm, WarpB
             if (give) {
                 if (lane == 0) {
                     d = atomicAdd(&r.sched->parcels, 1u);
-                    room = parcel_claim(r.flags[round & 1] + d % kParcels, r.sched->epoch, d);
+                    room = parcel_claim(r.flags[round & 1] + d % r.slots, r.sched->epoch, d);
                 }
                 d = __shfl_sync(full, d, 0);
                 room = __shfl_sync(full, (int)room, 0) != 0;
             }
             if (room) {
-                const unsigned p = d % kParcels;
+                const unsigned p = d % r.slots;
                 const MetaList& out = r.lists[round & 1];
                 const bool spilled = nspill > 0;  // the youngest spilled parents, else half of those on chip
                 n = spilled ? (nspill < 32 ? nspill : 32) : np / 2;

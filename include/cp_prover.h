@@ -448,6 +448,19 @@ cp_status cp_autotune_graph(cp_prover* p, const cp_refine_opts* opts, int* block
 /* Selects a level-kernel variant explicitly (0 .. CP_LEVEL_VARIANTS-1). */
 cp_status cp_set_level_variant(cp_prover* p, int family, int precision, int variant);
 
+/* Diagnostics: limits of the graph engine's work sharing, so that a test reaches what
+ * hardly any refinement does.  polls: of a wait for shared work (0: every wait ends at
+ * once, and what was given away is left for another launch); slots: places for shared
+ * work (1 to 4096); strict: spilled boxes from which a warp keeps its stack from growing
+ * (at most 4096); epoch: the launch number that the handle goes on from.  Negative:
+ * default, or the number left alone. */
+cp_status cp_set_deep_limits(cp_prover* p, int32_t polls, int32_t slots, int32_t strict, int64_t epoch);
+
+/* Diagnostics: of the handle's last graph-engine refinement, its launches, parcels of
+ * boxes that one warp gave to another, boxes spilled to memory, and the launch number
+ * after it (4 values). */
+cp_status cp_deep_stats(cp_prover* p, int64_t* out);
+
 /* ---------------------------------------------------------------- learned proposal model
  * The reference has no learned component: these entry points serve the
  * CP_SPLIT_LEARNED policy and cp_refine_opts.learned_order, which replace the
