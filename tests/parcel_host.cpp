@@ -33,7 +33,9 @@ void warp(pthread_barrier_t* bar, F f) {
 }  // namespace
 
 extern "C" {
-int p_claim(ParcelFlag* flag, unsigned long long epoch, unsigned d) { return parcel_claim(flag, epoch, d); }
+int p_claim(ParcelFlag* flag, unsigned long long epoch, unsigned d, unsigned slots) {
+    return parcel_claim(flag, epoch, d, slots);
+}
 unsigned p_ready(unsigned long long f, unsigned long long epoch, unsigned d) { return parcel_ready(f, epoch, d); }
 unsigned p_left(unsigned long long f, unsigned long long epoch) { return parcel_left(f, epoch); }
 // Refinements of `launches` launches each on one handle; returns how many launches had
@@ -65,11 +67,11 @@ long p_stress(int threads, unsigned slots, int each) {
         ts.emplace_back([&] {
             for (int k = 0; k < each; ++k) {
                 const unsigned d = next++, s = d % slots;
-                if (!parcel_claim(&flag[s], 7, d)) continue;
+                if (!parcel_claim(&flag[s], 7, d, slots)) continue;
                 if (owners[s].fetch_add(1) != 0) ++clashes;
                 std::this_thread::yield();
                 owners[s].fetch_sub(1);
-                __atomic_fetch_or(&flag[s], (ParcelFlag)kParcelTaken, __ATOMIC_SEQ_CST);
+                flag_set(&flag[s], parcel_tag(7, d) << 8 | kParcelTaken);
             }
         });
     for (auto& t : ts) t.join();
@@ -88,8 +90,8 @@ long p_hand_over(int parcels) {
     std::thread giver([&] {
         warp(&give, [&](HostWarp w) {
             for (int d = 0; d < parcels; ++d) {
-                while (w.first() && !parcel_claim(&flag, 1, d)) std::this_thread::yield();
-                parcel_give(w, &flag, 1, d, kLanes, [&] {
+                while (w.first() && !parcel_claim(&flag, 1, d, 1)) std::this_thread::yield();
+                parcel_give(w, &flag, 1, d, kLanes, d > 0, [&] {
                     w.late();
                     slot[w.lane] = kLanes * d + w.lane;
                 });

@@ -16,7 +16,7 @@ def host(tmp_path_factory):
     subprocess.run(["g++", "-O2", "-std=c++17", "-pthread", "-shared", "-fPIC", "-I" + CSRC,
                     os.path.join(HERE, "parcel_host.cpp"), "-o", so], check=True)
     L = ctypes.CDLL(so)
-    L.p_claim.argtypes = [ctypes.c_void_p, ctypes.c_ulonglong, ctypes.c_uint]
+    L.p_claim.argtypes = [ctypes.c_void_p, ctypes.c_ulonglong, ctypes.c_uint, ctypes.c_uint]
     L.p_ready.argtypes = [ctypes.c_ulonglong, ctypes.c_ulonglong, ctypes.c_uint]
     L.p_left.argtypes = [ctypes.c_ulonglong, ctypes.c_ulonglong]
     L.p_epochs.argtypes = [ctypes.c_long, ctypes.c_int]
@@ -27,18 +27,21 @@ def host(tmp_path_factory):
 
 @pytest.mark.parametrize("epoch", [1, 5, (1 << 24) - 1])
 def test_one_giver_per_slot(host, epoch):
-    """Parcels d and d + slots want one slot: the second giver is refused from the first one's claim on,
-    before anything is published, until the parcel has been taken."""
-    flag = ctypes.c_ulonglong(0)
-    p = ctypes.byref(flag)
-    assert host.p_claim(p, epoch, 3)
-    assert not host.p_claim(p, epoch, 3 + SLOTS)  # claimed, not yet published
-    flag.value |= 32
-    assert not host.p_claim(p, epoch, 3 + SLOTS)  # ready
+    """Parcels d, d + slots and d + 2 slots want one slot: a giver is refused from the moment another one
+    may write, before anything is published, until the parcel has been taken."""
+    old = (epoch - 1) << 40 | 3 << 8 | TAKEN  # another launch's flag
+    flag = ctypes.c_ulonglong(old)
+    claim = lambda d: bool(host.p_claim(ctypes.byref(flag), epoch, d, SLOTS))
+    assert claim(3)
+    assert not claim(3 + SLOTS)  # the first one has published nothing yet
+    flag.value = epoch << 40 | 3 << 8 | 32
+    assert not claim(3 + SLOTS)  # ready
     flag.value |= TAKEN
-    assert host.p_claim(p, epoch, 3 + SLOTS)
-    assert flag.value == epoch << 40 | (3 + SLOTS) << 8
-    assert host.p_claim(p, epoch + 1, 3)  # another launch's flag
+    assert claim(3 + 2 * SLOTS)
+    assert flag.value == epoch << 40 | (3 + 2 * SLOTS) << 8
+    assert not claim(3 + SLOTS)  # claimed
+    flag.value |= TAKEN
+    assert claim(3 + SLOTS)
 
 
 def test_claims_exclude_each_other(host):
