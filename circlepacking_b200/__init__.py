@@ -272,6 +272,7 @@ def _declare_handle(L):
     L.cp_autotune.argtypes = [P, ctypes.POINTER(RefineOpts), ctypes.POINTER(ctypes.c_int), P]
     L.cp_refine_boxes_static.argtypes = [I, I, I, I, P, P, P, SZ, ctypes.POINTER(RefineReport), P]
     L.cp_set_level_variant.argtypes = [P, I, I, I]
+    L.cp_get_level_variant.argtypes = [P, I, I, SZ, ctypes.POINTER(I)]
     L.cp_set_deep_limits.argtypes = [P, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int64]
     L.cp_deep_stats.argtypes = [P, P]
     L.cp_refine_resume.argtypes = [P, ctypes.POINTER(RefineReport)]
@@ -411,6 +412,12 @@ class Prover:
 
     def set_level_variant(self, family, precision, variant):
         _check(self._L.cp_set_level_variant(self._h, family, precision, variant), "cp_set_level_variant")
+
+    def get_level_variant(self, family, precision, count) -> int:
+        """The level-kernel variant that a chunk of `count` boxes runs."""
+        v = ctypes.c_int(-1)
+        _check(self._L.cp_get_level_variant(self._h, family, precision, count, ctypes.byref(v)), "cp_get_level_variant")
+        return v.value
 
     def set_deep_limits(self, polls=-1, slots=-1, strict=-1, epoch=-1):
         """Diagnostic limits of the graph engine's work sharing (-1: default, or left alone)."""

@@ -376,6 +376,7 @@ struct cp_prover {
     bool pending = false;
     cp_refine_opts pending_opts{};
     int variant[6][2] = {{2, 3}, {2, 3}, {2, 3}, {2, 2}, {2, 3}, {2, 3}};  // level-kernel variant per family/precision
+    bool variant_chosen[6][2] = {};  // by cp_set_level_variant or cp_autotune
     // called before every lattice launch of cp_prove_family_reference
     cp_step_callback step_cb = nullptr;
     void* step_user = nullptr;
@@ -583,6 +584,18 @@ void cp_engine_fill_report(const unsigned long long* h, cp_refine_report* r) {
     }
 }
 
+// The level-kernel variant of a chunk: the one that the caller or the autotuner chose for
+// the family and precision, else the default.  A small chunk waits for single evaluations:
+// of the defaults, the 128-register variant, which hardly spills, is the faster one there,
+// also where a large chunk wants more blocks per SM (B200: 34^3 start_end_2d boxes 94.6 ->
+// 90.9 us, FP32 116 -> 111 us; 10^4 start boxes FP32 173 -> 166 us; from some 1e5 boxes on
+// the default wins).
+static int variant_of(const cp_prover* p, int fam, int pr, size_t count) {
+    constexpr size_t kSmallChunk = (size_t)1 << 16;
+    const int v = p->variant[fam][pr];
+    return !p->variant_chosen[fam][pr] && count < kSmallChunk && v > 1 ? 1 : v;
+}
+
 // ------------------------------------------------------------------ internal API
 cp_status cp_engine_eval_chunk(cp_prover* p, int fam, const cp_refine_opts& o, LevelBuf& in, size_t begin,
                                size_t count, LevelBuf* out, const uint8_t* axis_hint, const uint8_t* order_hint,
@@ -611,13 +624,7 @@ cp_status cp_engine_eval_chunk(cp_prover* p, int fam, const cp_refine_opts& o, L
         k<<<grid, kEvalBlock, 0, p->stream>>>(a);
         CP_TRY(cp_check_launch());
     } else {
-        // A small chunk waits for single evaluations: the 128-register variant, which hardly
-        // spills, is the faster one there, also where a large chunk wants more blocks per
-        // SM (B200: 34^3 start_end_2d boxes 94.6 -> 90.9 us, FP32 116 -> 111 us; 10^4 start
-        // boxes FP32 173 -> 166 us; from some 1e5 boxes on the tuned variant wins).
-        constexpr size_t kSmallChunk = (size_t)1 << 16;
-        const int variant = count < kSmallChunk && p->variant[fam][pr] > 1 ? 1 : p->variant[fam][pr];
-        CP_TRY(launch_level(level_kernel(fam, pr, variant), a, p->stream));
+        CP_TRY(launch_level(level_kernel(fam, pr, variant_of(p, fam, pr, count)), a, p->stream));
     }
     cudaEventRecord(p->ev1, p->stream);
     CP_TRY(read_counters(p));
@@ -1271,6 +1278,13 @@ cp_status cp_set_level_variant(cp_prover* p, int family, int precision, int vari
     if (!p || family < 0 || family > 5 || precision < 0 || precision > 1 || variant < 0 || variant >= kVariants)
         return CP_ERR_INVALID;
     p->variant[family][precision] = variant;
+    p->variant_chosen[family][precision] = true;
+    return CP_OK;
+}
+
+cp_status cp_get_level_variant(cp_prover* p, int family, int precision, size_t count, int* variant) {
+    if (!p || !variant || family < 0 || family > 5 || precision < 0 || precision > 1) return CP_ERR_INVALID;
+    *variant = variant_of(p, family, precision, count);
     return CP_OK;
 }
 
@@ -1302,6 +1316,7 @@ cp_status cp_autotune(cp_prover* p, const cp_refine_opts* o, int* best, double* 
     const int pr = o->precision ? 1 : 0;
     double best_ms = 1e300;
     int best_v = 0;
+    p->variant_chosen[o->family][pr] = true;
     for (int v = 0; v < kVariants; ++v) {
         p->variant[o->family][pr] = v;
         cp_refine_report r;

@@ -445,8 +445,14 @@ cp_status cp_autotune(cp_prover* p, const cp_refine_opts* opts, int* best, doubl
  * (row = block size, column = boxes per thread). */
 cp_status cp_autotune_graph(cp_prover* p, const cp_refine_opts* opts, int* block, int* boxes_per_thread, double* ms);
 
-/* Selects a level-kernel variant explicitly (0 .. CP_LEVEL_VARIANTS-1). */
+/* Selects a level-kernel variant explicitly (0 .. CP_LEVEL_VARIANTS-1).  It holds for
+ * chunks of every size, as cp_autotune's choice does; a handle that neither was called on
+ * takes a default per family, precision and size of the chunk.  (Chunks with per-box hints
+ * of the learned model, or whose records are collected, run a kernel of one variant.) */
 cp_status cp_set_level_variant(cp_prover* p, int family, int precision, int variant);
+
+/* The variant that a chunk of `count` boxes runs. */
+cp_status cp_get_level_variant(cp_prover* p, int family, int precision, size_t count, int* variant);
 
 /* Diagnostics: limits of the graph engine's work sharing, so that a test reaches what
  * hardly any refinement does.  polls: of a wait for shared work (0: every wait ends at
