@@ -928,8 +928,7 @@ cp_status refine_graph(cp_prover* p, const cp_refine_opts& o, cp_refine_report* 
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.kernel, k.threads, k.smem) != cudaSuccess || per_sm < 1)
         per_sm = 1;
-    const unsigned grid = (unsigned)(sm_count(p->device) * per_sm);
-    const size_t warps = (size_t)grid * (k.threads / 32);
+    unsigned grid = (unsigned)(sm_count(p->device) * per_sm);
     RefineArgs a{};
     // spilled before a warp works strictly, then the stack's bound, and what the buffers on chip add (cp_refine.cuh)
     a.strict = p->deep_strict;
@@ -937,7 +936,17 @@ cp_status refine_graph(cp_prover* p, const cp_refine_opts& o, cp_refine_report* 
     a.polls = p->deep_polls;
     a.seg = a.strict + 32 * (size_t)(o.max_depth + 1) + 2 * (kParents + kReady);
     a.per = 32u * (unsigned)bpt;
-    CP_TRY(ensure_deep(p, D, warps * a.seg));
+    // The stacks need room for every warp, whatever the input (cp_refine_opts.level_capacity).
+    // Where the device has none left, fewer blocks do the same work.
+    cp_status room;
+    size_t warps;
+    for (;; grid = (grid + 1) / 2) {
+        warps = (size_t)grid * (k.threads / 32);
+        room = ensure_deep(p, D, warps * a.seg);
+        if (room != CP_ERR_NOMEM || grid == 1) break;
+        cudaGetLastError();  // the failed allocation is dealt with
+    }
+    CP_TRY(room);
     a.level.in = p->levels[0].b;
     a.level.cnt = p->cnt;
     a.level.per_depth = p->per_depth;

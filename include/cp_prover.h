@@ -194,8 +194,13 @@ typedef struct cp_refine_opts {
     int32_t max_depth;      /* a box not proved at this depth is unresolved (<= 250) */
     int32_t seed_sizes[4];  /* lattice seed: subdivisions per axis */
     double seed_lambda[2];  /* outer lambda interval of the lattice seed */
-    int64_t level_capacity; /* boxes per level buffer; 0 = 1<<25 */
-    int32_t block;          /* threads per block of the level kernel; 0 = 128 */
+    int64_t level_capacity; /* boxes per level buffer; 0 = 1<<25.  CP_ENGINE_LEVELS keeps max_depth + 1 of
+                               them.  CP_ENGINE_GRAPH keeps one for the seeds, and besides, whatever the
+                               capacity, 18 MB and its warps' stacks (100 MB at max_depth 2, 280 MB at 30,
+                               580 MB at 62 and block 1024), which the handle holds until it is destroyed;
+                               where the device has less left, it runs fewer warps */
+    int32_t block;          /* CP_ENGINE_GRAPH: 64, 128, 256, 512 or 1024 names a kernel shape (64, 128 and 256
+                               threads of 128 registers, 320 of 96, 384 of 80); 0 = tuned */
     int32_t learned_order;  /* 1 = learned criterion order (needs a trained or loaded model) */
     int32_t engine;         /* cp_engine: host-driven level loop, or one launch on the device */
     int32_t boxes_per_thread; /* graph engine: boxes a warp lane takes per claim (1..8); 0 = tuned */
