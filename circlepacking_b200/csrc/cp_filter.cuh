@@ -11,7 +11,8 @@
 //
 // Error bound.  "Directed" is eval_box's value, "filter" the value here, both
 // against the same formula in exact arithmetic.  The box guard (box_ok) bounds
-// the inputs: lambda in [0.49, 0.996], radii at most 1/3, 0.25 <= L, S < 1.4.
+// the inputs: lambda in [kLambdaLow, kLambdaHigh], radii at most kMaxRadius, so that
+// 0.25 <= L, S < 1.4.
 //   * Directed: L^2 - S^2 and (a + b)^2 are off by at most 2^-49.4 (a few ulps of
 //     values below 2), the quotient q = (L^2 - S^2 +- c^2) / (2 c L) of a
 //     collision angle by 2^-49.4 / c <= 2^-41.4 (c = a + b >= 2^-8), and asin(q) by
@@ -68,6 +69,7 @@ constexpr double kGap = 9.313225746154785e-10;   // 2^-30, least excess of 2 (a 
 constexpr double kMinB = 0.000244140625;             // 2^-12
 constexpr double kLowSlack = 3.814697265625e-06;     // 2^-18
 constexpr double kMinC = 0.00390625;                // 2^-8, least a + b
+constexpr double kLambdaLow = 0.49, kLambdaHigh = 0.992, kMaxRadius = 0.3333;
 constexpr double kHalfPi = 1.5707963267948966;
 constexpr double kRatio = 0.5642, kPi = 3.141592653589793;  // lane_packing/values.hpp:28-32
 
@@ -80,12 +82,15 @@ CPF_HD double fma_(double a, double b, double c) {
 #endif
 }
 CPF_HD double abs_(double x) { return fabs(x); }
-// seeds of 1/d and 1/sqrt(d): the FP64 approximations, within 2^-19 (host: rounded to float)
+// seeds of 1/d and 1/sqrt(d): the FP64 approximations, within 2^-19 (host: rounded to
+// float, or off by the relative error CPF_SEED_ERROR)
 CPF_HD double rcp_seed_(double d) {
 #ifdef __CUDA_ARCH__
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
     return y;
+#elif defined(CPF_SEED_ERROR)
+    return (1.0 + (CPF_SEED_ERROR)) / d;
 #else
     return (double)(1.0f / (float)d);
 #endif
@@ -95,6 +100,8 @@ CPF_HD double rsqrt_seed_(double d) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
     return y;
+#elif defined(CPF_SEED_ERROR)
+    return (1.0 + (CPF_SEED_ERROR)) / std::sqrt(d);
 #else
     return (double)(1.0f / std::sqrt((float)d));
 #endif
@@ -313,13 +320,13 @@ template <bool THREE>
 CPF_HD bool box_ok(const FBox& b) {
     const double w = b.lh - b.ll;
     double m = b.h1 > b.h2 ? b.h1 : b.h2;
-    bool ok = b.ll >= 0.49 && b.lh <= 0.992 && w >= 9.094947017729282e-13;
+    bool ok = b.ll >= kLambdaLow && b.lh <= kLambdaHigh && w >= 9.094947017729282e-13;
     ok = ok && b.l1 > 0.0 && b.l2 >= 0.0 && b.l1 <= b.h1 && b.l2 <= b.h2 && b.h1 + b.h2 >= kMinC;
     if (THREE) {
         ok = ok && b.l3 >= 0.0 && b.l3 <= b.h3 && b.h2 + b.h3 >= kMinC && b.l1 + b.l3 >= 0.5 * kMinC;
         if (b.h3 > m) m = b.h3;
     }
-    ok = ok && m <= 0.3333;
+    ok = ok && m <= kMaxRadius;
     return ok && (1.0 - b.lh) * (1.0 + b.lh - 2.0 * m) >= fma_(4.0 * m, w, kGap);
 }
 
