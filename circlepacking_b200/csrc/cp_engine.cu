@@ -53,10 +53,11 @@ __global__ void __launch_bounds__(kEvalBlock, MINB) k_level(RefineArgs r) {
     level_end(r.level.cnt);
 }
 
-// The level kernel for refinements in which every box passes through a level:
-// per-box proposals of the learned model, and the collection of its records.
-template <int FAM, int PREC>
-__global__ void __launch_bounds__(kEvalBlock) k_level_each(LevelArgs a) {
+// The level kernel for chunks whose children all go through a level: per-box proposals of
+// the learned model, the collection of its records, and some chunks with the FP32 pre-pass
+// (each_variant).
+template <int FAM, int PREC, int MINB>
+__global__ void __launch_bounds__(kEvalBlock, MINB) k_level_each(LevelArgs a) {
     __shared__ LevelSmem<kEvalBlock / 32> sm;
     level_smem_init(sm);
     __syncthreads();
@@ -487,18 +488,19 @@ LevelKernel level_kernel(int fam, int prec, int v) {
     }
 }
 
+// dense (FP32 only): 6 blocks per SM, else 4.
 template <int FAM>
-LevelEachKernel level_each_p(int prec) {
-    return prec ? k_level_each<FAM, 1> : k_level_each<FAM, 0>;
+LevelEachKernel level_each_p(int prec, bool dense) {
+    return !prec ? k_level_each<FAM, 0, 1> : dense ? k_level_each<FAM, 1, 6> : k_level_each<FAM, 1, 4>;
 }
-LevelEachKernel level_each_kernel(int fam, int prec) {
+LevelEachKernel level_each_kernel(int fam, int prec, bool dense) {
     switch (fam) {
-    case 0: return level_each_p<0>(prec);
-    case 1: return level_each_p<1>(prec);
-    case 2: return level_each_p<2>(prec);
-    case 3: return level_each_p<3>(prec);
-    case 4: return level_each_p<4>(prec);
-    default: return level_each_p<5>(prec);
+    case 0: return level_each_p<0>(prec, dense);
+    case 1: return level_each_p<1>(prec, dense);
+    case 2: return level_each_p<2>(prec, dense);
+    case 3: return level_each_p<3>(prec, dense);
+    case 4: return level_each_p<4>(prec, dense);
+    default: return level_each_p<5>(prec, dense);
     }
 }
 
@@ -514,6 +516,13 @@ cp_status launch_level(LevelKernel k, const LevelArgs& a, cudaStream_t st) {
     const size_t warps = kEvalBlock / 32, need = (a.count + warps - 1) / warps;
     const unsigned grid = (unsigned)std::min<size_t>(grid_of(k, kEvalBlock), std::max<size_t>(need, 1));
     k<<<grid, kEvalBlock, 0, st>>>(r);
+    return cp_check_launch();
+}
+
+cp_status launch_level_each(LevelEachKernel k, const LevelArgs& a, cudaStream_t st) {
+    const size_t need = (a.count + kEvalBlock - 1) / kEvalBlock;
+    const unsigned grid = (unsigned)std::min<size_t>(grid_of(k, kEvalBlock), std::max<size_t>(need, 1));
+    k<<<grid, kEvalBlock, 0, st>>>(a);
     return cp_check_launch();
 }
 
@@ -561,6 +570,13 @@ cp_status cp_engine_launch_level(int fam, int prec, int variant, const BoxList& 
     a.axis_hint = nullptr;
     a.order_hint = nullptr;
     a.digest = 0;
+    // Small, uneven seeds and many levels.  Children kept on chip make long chains of
+    // evaluations on a few warps: with the FP32 pre-pass, and in the start families, whose
+    // undecided boxes pay for two evaluations, also in FP64 (B200, random boxes, microseconds
+    // on chip and through levels: 20000 start_end_3d to depth 6 489, 424, FP32 1158, 780; 4096
+    // end_2d to depth 6 251, 268, FP32 382, 346; one level of 20000 start 156, 191).
+    if (max_depth > 1 && (prec || (fam <= F_START_END_3D && count >= 4096)))
+        return launch_level_each(level_each_kernel(fam, prec, false), a, st);
     return launch_level(level_kernel(fam, prec, variant), a, st);
 }
 
@@ -596,6 +612,33 @@ static int variant_of(const cp_prover* p, int fam, int pr, size_t count) {
     return !p->variant_chosen[fam][pr] && count < kSmallChunk && v > 1 ? 1 : v;
 }
 
+// Blocks per SM with which a chunk with the FP32 pre-pass, under the default variant, goes
+// through k_level_each; 0: it goes through k_level.  The shadow's evaluations are long
+// (some 25 us) and live on spilled registers, for which k_level's boxes leave little L1.
+// Best of both on a B200, microseconds for k_level and k_level_each, lattices:
+//   * boxes without children.  k_level spreads a few thousand over more warps than the SMs
+//     issue for at a time: 10^4 start_end_3d 174, 166; 16^4 213, 180.  Fewer or more are
+//     its own: 6^4 start 152, 170; 20^4 224, 235.  Below the seeds, where most boxes are
+//     decided in FP32, k_level_each goes on: 12^4 start and two levels 1697, 1236;
+//   * boxes with children.  On chip, a warp that starts with a few boxes evaluates all of
+//     their children by itself, and between one and two pieces a warp half of the warps wait
+//     for the others: 12^4 start and one level 522, 369; 12^4 start_end_3d 625, 456; 10^4
+//     end_3d and two levels 814, 589; 20^3 start_end_2d 310, 288.  Below 8192 the second
+//     launch costs more (8^4 start and one level 252, 293), from 2^19 on, dropped children
+//     counted, the pieces even out (16^4 start_end_3d and two levels 5030, 5678; 50^3
+//     start_end_2d, from 2^16 on, 838, 954).  Middle and end_2d, whose evaluations are
+//     shorter, are faster on chip throughout.
+static int each_blocks(const cp_prover* p, int fam, int pr, size_t count, bool seeds, bool children) {
+    if (!pr || p->variant_chosen[fam][pr]) return 0;
+    const bool long_chain = fam == F_START || fam == F_START_END_3D || fam == F_END_3D;
+    if (!children) {
+        if (count < (size_t)1 << 12) return 0;
+        return count < (size_t)1 << 17 ? 4 : long_chain && !seeds ? 6 : 0;
+    }
+    const size_t end = long_chain ? (size_t)1 << 19 : fam == F_START_END_2D ? (size_t)1 << 16 : 0;
+    return count >= (size_t)1 << 13 && count < end ? 6 : 0;
+}
+
 // ------------------------------------------------------------------ internal API
 cp_status cp_engine_eval_chunk(cp_prover* p, int fam, const cp_refine_opts& o, LevelBuf& in, size_t begin,
                                size_t count, LevelBuf* out, const uint8_t* axis_hint, const uint8_t* order_hint,
@@ -617,12 +660,10 @@ cp_status cp_engine_eval_chunk(cp_prover* p, int fam, const cp_refine_opts& o, L
     // (the deepest non-empty level is taken first, so `out` is empty)
     const int pr = o.precision ? 1 : 0;
     cudaEventRecord(p->ev0, p->stream);
-    if (axis_hint || order_hint || cp_model_collecting(p)) {
-        LevelEachKernel k = level_each_kernel(fam, pr);
-        const size_t need = (count + kEvalBlock - 1) / kEvalBlock;
-        const unsigned grid = (unsigned)std::min<size_t>(grid_of(k, kEvalBlock), std::max<size_t>(need, 1));
-        k<<<grid, kEvalBlock, 0, p->stream>>>(a);
-        CP_TRY(cp_check_launch());
+    const bool records = axis_hint || order_hint || cp_model_collecting(p);
+    const int each = records ? 4 : each_blocks(p, fam, pr, count, &in == &p->levels[0], out != nullptr);
+    if (each) {
+        CP_TRY(launch_level_each(level_each_kernel(fam, pr, each > 4), a, p->stream));
     } else {
         CP_TRY(launch_level(level_kernel(fam, pr, variant_of(p, fam, pr, count)), a, p->stream));
     }
