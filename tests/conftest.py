@@ -33,6 +33,12 @@ def ref():
     from oracle import refcheck
 
     if not refcheck.available():
+        # built from the reference's sources: without them there is nothing to build it from (the
+        # golden vectors it left stand in, tests/test_golden.py); with them it is missing by mistake
+        from __graft_entry__ import reference_dir
+
+        if not os.path.isdir(reference_dir()):
+            pytest.skip(f"no reference sources to build the reference checker {refcheck.SO} from")
         pytest.fail(f"reference checker {refcheck.SO} is missing (build: make -C oracle ref)")
     refcheck.lib()
     return refcheck
