@@ -204,16 +204,17 @@ def same_boxes_and_verdicts(a, b):
             and a["unresolved"] == b["unresolved"] and a["per_depth"] == b["per_depth"])
 
 
-def autotune(prover, cp, learned: bool):
+def autotune(prover, cp, learned: bool, depth: int):
     """Per family, outside the timed region: the fastest form on a calibration
-    refinement (32^dims seed, one level) among the device-driven graph engine
+    refinement (32^dims seed, the step's depth: the share of the last level, where
+    the engines differ, is the step's) among the device-driven graph engine
     (block size x boxes per thread) and the host-driven level loop (register
     variants), each in FP64 and with the FP32 pre-pass, then (with `learned`)
     whether the trained network's criterion order is faster still.  Every
     candidate gives identical verdicts, so the choice is speed only."""
     forms, table = {}, {}
     for f in FAMILIES:
-        calib = dict(policy=cp.SPLIT_UNIFORM, max_depth=1, seed_sizes=[32] * DIMS[f])
+        calib = dict(policy=cp.SPLIT_UNIFORM, max_depth=depth, seed_sizes=[32] * DIMS[f])
         cands = []
         for prec in (cp.FP64, cp.FP32_PREFILTER):
             blk, bpt, ms = prover.autotune_graph(f, precision=prec, **calib)
@@ -256,11 +257,17 @@ def train_models(prover, cp, depth):
     return out
 
 
-# DRAM traffic of the graph refinement per evaluated box, from one ncu capture
-# (middle family, 32^4 seed, two levels: 138.4M boxes evaluated, 73.7 MB read + 6.1 MB
-# written); algorithmic: the 65 B of a 4-D seed.  FP64 pipe activity of the same capture.
-TRAFFIC_PER_BOX, ALGORITHMIC_BYTES_PER_BOX = 79.8e6 / 138.4e6, 65.0 * 32**4 / 138.4e6
-FP64_PIPE_ACTIVE_NCU = 0.441
+# Per engine, from one ncu capture each (middle family, 24^4 seed, two levels, FP64: 41.80M
+# boxes evaluated): DRAM bytes per evaluated box (levels: 372.6 MB read + 309.1 MB written in
+# 12 launches, the first level's children through memory; graph: 25.6 + 0.6 MB), the bytes it
+# cannot do without (the 65 B of a 4-D seed, and of the children that go through a level,
+# written and read), and the FP64 pipe's activity.
+KERNELS = {
+    "levels": {"kernel": "k_level", "traffic": 681.7e6 / 41.80e6, "algorithmic": 65.0 * (24**4 + 2 * 3.233e6) / 41.80e6,
+               "fp64_pipe_active": 0.367},
+    "graph": {"kernel": "k_refine_deep", "traffic": 26.1e6 / 41.80e6, "algorithmic": 65.0 * 24**4 / 41.80e6,
+              "fp64_pipe_active": 0.389},
+}
 
 PROOF_FAMILIES = (0, 1, 2, 3, 4, 5)
 
@@ -283,8 +290,10 @@ def proof_leg(prover, cp, forms, families, world=1):
         best_kw = dict(engine=cp.ENGINE_GRAPH, precision=forms[f]["precision"], digest=1, seed_parts=PARTS,
                        seed_part=PART)
         plain_kw = dict(best_kw, engine=cp.ENGINE_LEVELS, precision=cp.FP64, reuse=0)
-        # warm-up (graph build): one slab of a 4^dims seed as given, no per-slab scaling
-        prover.prove_family(f, **dict(best_kw, slabs=1, seed_sizes=[4, 4, 4, 4], slab_radii=[]))
+        # warm-up of both forms (their worklists are allocated): one slab of a 4^dims seed as
+        # given, no per-slab scaling
+        for kw in (plain_kw, best_kw):
+            prover.prove_family(f, **dict(kw, slabs=1, seed_sizes=[4, 4, 4, 4], slab_radii=[]))
         b = prover.prove_family(f, **best_kw)
         p = prover.prove_family(f, **plain_kw)
         same = (b["digest"] == p["digest"] and b["verdicts"] == p["verdicts"] and b["per_depth"] == p["per_depth"]
@@ -321,7 +330,7 @@ def seed_boxes_host(family):
     return hlo, hhi, hdp
 
 
-def roofline_of(cp, device, reps, counts) -> dict:
+def roofline_of(cp, device, reps, counts, forms) -> dict:
     """Roofline of the FP64 criterion evaluation (the level kernel): the
     reference kernel's own primitive operations per evaluated box (add/sub,
     mul, div, asin, each counting one), weighted by the step's boxes per depth,
@@ -331,8 +340,11 @@ def roofline_of(cp, device, reps, counts) -> dict:
     reference's __ddiv_rd and once with this library's division."""
     rates = cp.measure_primitives(device)
     ops = {"add": 0.0, "mul": 0.0, "div": 0.0, "asin": 0.0}
-    boxes = 0
+    boxes, ms_of, boxes_of = 0, {}, {}
     for f, r in zip(FAMILIES, reps):
+        engine = "graph" if forms[f]["engine"] == cp.ENGINE_GRAPH else "levels"
+        ms_of[engine] = ms_of.get(engine, 0.0) + r["device_ms"]
+        boxes_of[engine] = boxes_of.get(engine, 0) + r["evaluated"]
         per = counts[f]
         depths = sorted(per)
         for d, n in enumerate(r["per_depth"]):
@@ -353,11 +365,13 @@ def roofline_of(cp, device, reps, counts) -> dict:
     achieved = unweighted / kernel_s
     return {"bound": "fp64", "achieved": achieved / 1e12, "peak": peak / 1e12, "unit": "TFLOP/s",
             "frac": achieved / peak,
-            "traffic": TRAFFIC_PER_BOX * boxes,
-            "traffic_note": f"DRAM bytes per step: {TRAFFIC_PER_BOX:.2f} B per evaluated box from one ncu capture of "
-                            f"the graph refinement (algorithmic {ALGORITHMIC_BYTES_PER_BOX:.2f} B), scaled by the "
-                            f"step's {boxes} evaluated boxes",
-            "kernel": "k_refine_deep<family, precision, block> (per-box criteria + split), graph engine",
+            "traffic": sum(KERNELS[e]["traffic"] * n for e, n in boxes_of.items()),
+            "traffic_note": "DRAM bytes per step: per engine the bytes per evaluated box of one ncu capture, scaled by "
+                            "the boxes that the step evaluates with it; " + "; ".join(
+                                f"{e}: {KERNELS[e]['traffic']:.2f} B (algorithmic {KERNELS[e]['algorithmic']:.2f} B) x "
+                                f"{n} boxes" for e, n in boxes_of.items()),
+            "kernel": "; ".join(f"{KERNELS[e]['kernel']}<family, precision, shape> ({e} engine), "
+                                f"{t:.1f} ms of the step" for e, t in ms_of.items()),
             "work_model": "per evaluated box: the reference kernel's own add/sub, mul, div and asin count (it stops "
                           "at the first failing sub-check and handle), counted by the CPU restatement while it refines "
                           "sampled seeds of the same workload, per family and depth, weighted by the step's boxes per "
@@ -365,7 +379,7 @@ def roofline_of(cp, device, reps, counts) -> dict:
             "ops_per_second": {k: v / kernel_s / 1e12 for k, v in ops.items()} | {"unit": "T/s"},
             "frac_weighted_ddiv_rd": weighted(rates["ddiv_rd"]) / kernel_s / peak,
             "frac_weighted_library_div": weighted(rates["div_rd_lib"]) / kernel_s / peak,
-            "fp64_pipe_active_ncu": FP64_PIPE_ACTIVE_NCU,
+            "fp64_pipe_active_ncu": sum(KERNELS[e]["fp64_pipe_active"] * t for e, t in ms_of.items()) / sum(ms_of.values()),
             "peaks_measured_tops": {k: v / 1e12 for k, v in rates.items()},
             "peak_source": "measured in-process (MEASURED_PEAKS.json has no FP64 figure): DFMA instruction rate",
             "ops_per_box": {cp.FAMILIES[f]: {str(d): v for d, v in counts[f].items()} for f in FAMILIES}}
@@ -569,7 +583,7 @@ def main():
     else:
         if not args.no_learned:
             models = train_models(prover, cp, args.depth)
-        forms, tuning = autotune(prover, cp, learned=not args.no_learned)
+        forms, tuning = autotune(prover, cp, learned=not args.no_learned, depth=args.depth)
 
     tuned_variant = {f: tuning[cp.FAMILIES[f]].get("variant", 1) for f in FAMILIES}
 
@@ -700,7 +714,7 @@ def main():
     cpu, counts = None, None
     if rank == 0 and not args.no_cpu:
         cpu, counts = cpu_baseline(args.cpu_seconds, args.depth)
-    roofline = roofline_of(cp, local, reps_best, counts) if (counts and not args.no_roofline) else None
+    roofline = roofline_of(cp, local, reps_best, counts, forms) if (counts and not args.no_roofline) else None
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": ms_best, "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "dtype": "f64",
