@@ -37,9 +37,10 @@
 // about 24 certified divisions and 12 padded arcsines per box, each a call.  Here
 // a collision angle costs one approximate reciprocal and two short polynomials,
 // inlined, and most boxes are decided from a few of their angles.  About 1 in 5000
-// lattice boxes is left to eval_box.  On B200: middle, 64^4 lattice and two uniform
-// levels, 494 -> 188 ms; 1e6 complete masks (middle) 390 -> 86 us; half of the start
-// proof 74.6 -> 33.8 ms.
+// lattice boxes is left to eval_box.  On B200: 1e6 complete masks (middle) 388 -> 93 us.
+// What it gave refinements by itself, while every box still passed through a level: 64^4
+// middle lattice and two uniform levels 494 -> 188 ms, half of the start proof 74.6 ->
+// 33.8 ms (they take 76 and 26 ms now, cp_refine.cuh).
 #pragma once
 #include <cstdint>
 

@@ -806,7 +806,7 @@ __device__ __forceinline__ void tt_gemm(uint32_t tmem, uint32_t dcol, const bf16
 // Sums of 32 columns over a warp's rows: r[c] is column c of the lane's row; returns
 // column `lane`.  Each step folds half of the columns into the other lanes: 31 shuffles,
 // where an atomic per element of a shared column serialised all 128 rows.  k_train_tc
-// on a B200, 65536 rows: about 2.7 ms -> 0.227 ms (512 tiles, one CTA per SM).
+// on a B200, 65536 rows: 2.7 ms -> 0.23 ms (512 tiles, one CTA per SM).
 __device__ __forceinline__ float warp_colsum32(float (&v)[32], int lane) {
 #pragma unroll
     for (int w = 16; w > 0; w >>= 1) {

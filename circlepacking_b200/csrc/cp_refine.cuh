@@ -8,9 +8,9 @@
 // Why: with the filter a box costs about 700 warp instructions, less than writing
 // its children to a level (65 B each, a division and two dependent table loads per
 // child) and reading them back cost.  A refinement's last level holds most of its
-// boxes.  B200, middle, 64^4 lattice and two uniform levels, graph engine: 188 -> 75 ms
-// (of which the level's kernels and the filter read their boxes from shared memory
-// instead of holding them in registers: no spills at 20 warps per SM).
+// boxes.  B200, middle, 64^4 lattice and two uniform levels, graph engine: 188 -> 76 ms,
+// the filter reading its boxes from shared memory included; half of the start proof 34 ->
+// 26 ms; 31^4 start_end_3d lattice with the FP32 pre-pass 74 -> 50 ms.
 //
 // A warp holds, in shared memory:
 //   * a stack of parents: boxes evaluated, not proved and above the depth limit,
@@ -57,8 +57,8 @@ struct MetaList {
 };
 
 // Work sharing of a depth-first refinement.  Warps draw tickets: the first ones are
-// pieces of the input, ticket `inputs` + d is the d-th parcel of 32 parents that some
-// warp gives away.  A warp whose ticket's parcel does not exist yet waits for it (a
+// pieces of the input, ticket `inputs` + d is the d-th parcel of up to 32 parents that
+// some warp gives away (cp_parcel.cuh).  A warp whose ticket's parcel does not exist yet waits for it (a
 // bounded wait); warps with enough parents give a parcel away per step while there
 // are more tickets than parcels.  Parcels that nobody waited for to the end are the
 // input of the next kernel launch ("round"); there are hardly ever any.
@@ -66,8 +66,8 @@ struct MetaList {
 // Without sharing the trees below the seeds are too uneven: on the last slab of the
 // start_end_3d proof (2.9e7 boxes, 26010 seeds) warps that stopped as soon as a
 // quarter of them were idle, for a new round to spread the rest, needed 13 rounds and
-// 4.2 ms; with parcels it is one round of 3.5 ms, and the smallest slabs of the start
-// and start_end_3d proofs take 0.10 to 0.2 ms instead of 0.2 to 0.4 (a level each).
+// 4.2 ms, where parcels needed one round of 3.5 ms; the smallest slabs of the start
+// and start_end_3d proofs took 0.10 to 0.2 ms instead of 0.2 to 0.4 (a level each).
 struct DeepSched {
     unsigned long long count;  // seed boxes
     unsigned long long epoch;  // of this round; a parcel's flag carries it

@@ -79,7 +79,8 @@ typedef enum cp_precision {
     CP_FP64 = 0,           /* FP64: verdicts of the reference's directed rounding, decided by a round-to-nearest
                               FP64 evaluation where every comparison clears its error bound, else by directed
                               rounding, bit-identical to the reference */
-    CP_FP32_PREFILTER = 1  /* FP32 enclosure pass issues PROVED; every other box is re-evaluated in FP64 */
+    CP_FP32_PREFILTER = 1  /* an FP32 enclosure pass decides the boxes it can, the others are evaluated in FP64;
+                              same verdicts.  It costs time: on a B200 about six times CP_FP64's */
 } cp_precision;
 
 typedef enum cp_eval_mode {
@@ -216,9 +217,8 @@ typedef struct cp_refine_opts {
 
 /* Refinement engines.  CP_ENGINE_LEVELS: the host picks each chunk, launches
  * the level kernel and reads the counters back (one round trip per chunk).
- * CP_ENGINE_GRAPH: the refinement runs
- * on the device in one kernel launch: every warp refines its boxes depth first from a
- * stack of its own and shares work with warps that run out (report->launches: kernel
+ * CP_ENGINE_GRAPH: the refinement runs on the device in one kernel launch: every warp
+ * refines its boxes depth first from a stack of its own and shares work with warps that run out (report->launches: kernel
  * launches, more than 1 only when shared work was left over); `block` (64, 128, 256,
  * 512, 1024; 0 = tuned) selects the kernel shape, boxes_per_thread the boxes per
  * claim.  With a learned policy, a scheduler kernel and a persistent level kernel with
@@ -231,7 +231,7 @@ typedef struct cp_refine_report {
     int64_t verdicts[5];     /* evaluated boxes per cp_verdict */
     int64_t unresolved;      /* boxes not proved at max_depth */
     int64_t clipped;         /* children outside the domain, dropped unevaluated */
-    int64_t fp32_decided;    /* boxes proved by the FP32 pass */
+    int64_t fp32_decided;    /* boxes decided by the FP32 pass */
     int64_t per_depth[64];   /* boxes evaluated per depth (depth >= 63 in the last) */
     int32_t max_depth_seen;
     int32_t launches;
