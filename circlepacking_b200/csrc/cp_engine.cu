@@ -378,6 +378,7 @@ struct cp_prover {
     cp_refine_opts pending_opts{};
     int variant[6][2] = {{2, 3}, {2, 3}, {2, 3}, {2, 2}, {2, 3}, {2, 3}};  // level-kernel variant per family/precision
     bool variant_chosen[6][2] = {};  // by cp_set_level_variant or cp_autotune
+    bool graph_chosen[6][2] = {};    // graph_variant, by cp_autotune_graph
     // called before every lattice launch of cp_prove_family_reference
     cp_step_callback step_cb = nullptr;
     void* step_user = nullptr;
@@ -948,6 +949,19 @@ cp_status ensure_deep(cp_prover* p, int dims, size_t spill_cap) {
     return CP_OK;
 }
 
+// The shape of the depth-first kernel: the autotuner's for the family and precision, else
+// the default.  With the FP32 pre-pass, small inputs of the families whose default has 80
+// registers wait for single evaluations, and 64 threads of 128 registers are faster: 9^4
+// start_end_3d, no level, 237 -> 175 us; 16^4 and one level 1194 -> 1106 us; 11^4 start and
+// two levels 1394 -> 1294 us.  Not so 20^4 and one level (1661, 1773 us) and, of
+// start_end_3d, 10^4 and two (1445, 1498).
+int deep_variant(const cp_prover* p, int fam, int prec, size_t seeds, int max_depth) {
+    const int v = p->graph_variant[fam][prec];
+    if (!prec || p->graph_chosen[fam][prec] || (fam != F_START && fam != F_START_END_3D)) return v;
+    const bool small = max_depth <= 1 ? seeds <= (size_t)1 << 16 : fam == F_START && seeds <= (size_t)1 << 14;
+    return small ? 0 : v;
+}
+
 // The whole refinement as one launch of the depth-first kernel.
 cp_status refine_graph(cp_prover* p, const cp_refine_opts& o, cp_refine_report* r, double t_wall0) {
     const int fam = o.family;
@@ -955,7 +969,8 @@ cp_status refine_graph(cp_prover* p, const cp_refine_opts& o, cp_refine_report* 
     const int prec = o.precision ? 1 : 0;
     if (o.max_depth + 1 > kMaxLevels)
         return cp_fail(CP_ERR_INVALID, "graph engine: max_depth must be < %d", kMaxLevels);
-    const int variant = o.block > 0 ? graph_variant_of_block(o.block) : p->graph_variant[fam][prec];
+    const int variant = o.block > 0 ? graph_variant_of_block(o.block)
+                                    : deep_variant(p, fam, prec, p->levels[0].n, o.max_depth);
     if (variant < 0) return cp_fail(CP_ERR_INVALID, "graph engine: block must be 64, 128, 256, 512 or 1024");
     const int bpt = o.boxes_per_thread > 0 ? o.boxes_per_thread : p->graph_bpt[fam][prec];
     if (bpt > 8) return cp_fail(CP_ERR_INVALID, "graph engine: boxes_per_thread must be 1..8");
@@ -1407,6 +1422,7 @@ cp_status cp_autotune_graph(cp_prover* p, const cp_refine_opts* o, int* block, i
         }
     const int pr = o->precision ? 1 : 0;
     p->graph_variant[o->family][pr] = best_v;
+    p->graph_chosen[o->family][pr] = true;
     p->graph_bpt[o->family][pr] = best_b;
     *block = kGraphBlock[best_v];
     *boxes_per_thread = best_b;

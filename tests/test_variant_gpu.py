@@ -56,3 +56,16 @@ def test_static_call_agrees_with_the_level_loop(cp, family, n, depth, precision)
     for k in ("evaluated", "unresolved", "clipped", "fp32_decided", "handles_evaluated", "verdicts", "per_depth"):
         assert a[k] == b[k], k
     p.close()
+
+
+@pytest.mark.parametrize("n,depth", [(1 << 16, 1), ((1 << 16) + 1, 1), (1 << 14, 2), ((1 << 14) + 1, 2), (100, 0)])
+@pytest.mark.parametrize("family", [0, 2])
+def test_fp32_graph_agrees_whatever_its_shape(cp, family, n, depth):
+    p = cp.Prover()
+    lo, hi, dp = p.random_boxes(family, n, seed=n, max_label=2)
+    kw = dict(max_depth=depth, policy=cp.SPLIT_UNIFORM, precision=cp.FP32_PREFILTER, digest=1, level_capacity=1 << 20,
+              engine=cp.ENGINE_GRAPH)
+    a, b = p.refine_boxes(family, lo, hi, dp, **kw), p.refine_boxes(family, lo, hi, dp, block=1024, **kw)
+    for k in ("evaluated", "unresolved", "clipped", "fp32_decided", "handles_evaluated", "verdicts", "per_depth", "digest"):
+        assert a[k] == b[k], k
+    p.close()
